@@ -55,7 +55,10 @@ __device__ __forceinline__ void sl_axis(double C, int c, int cs, int ce, int &c0
         c1 = c0 - 1;
         r = frac1(C);
     } else if (C < -eps) {
-        const int t = c - (int) C;
+        // a flow that runs away: the conversion saturates at INT_MIN, and c - INT_MIN
+        // would wrap to an index far below the array; -2^30 is past every axis' end
+        // (levels hold fewer than 2^31 cells, three per axis at least)
+        const int t = c - max((int) C, -(1 << 30));
         c0 = t < ce ? t : ce;
         c1 = c0 + 1;
         r = frac1(-C);
