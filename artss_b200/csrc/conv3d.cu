@@ -7,323 +7,330 @@
 //     y[z,y,x,co] = bias[co] + sum_{t, ci} w[t][co][ci] * x[z+dz, y+dy, x+dx, ci]
 // with tap t = 9 (dz+1) + 3 (dy+1) + (dx+1).
 //
-// GEMM view: M = 128 output voxels (a run of x, several y rows and z planes
-// when W or W*H is below 128),
-// N = C_out, K = 27 taps x C_in.  Per tap one TMA load brings the 128 shifted
-// input rows (out-of-range voxels arrive as zeros, which is the padding) in
-// the K-major core-matrix layout [C_in/8][128][8] (the tensor map orders the
-// dimensions channel-in-group, x, y, z, channel group), and one bulk copy brings
-// the tap's weights, pre-packed as [C_in/8][C_out][8]; one thread issues the
-// C_in/16 MMAs of the tap and commits them to the stage's "empty" barrier.
-// After the 27th tap the accumulator (128 lanes x C_out FP32 columns) is read
-// by warps 0-3 with tcgen05.ld: bias, optional ReLU, BF16, store.  Warp 4
-// loads and issues: two accumulators in tensor memory alternate between tiles,
-// so the MMAs of tile n+1 run while tile n is read out.  Blocks are persistent
-// over output tiles; loads run as many taps ahead as shared memory holds
-// stages (ConvShape::stages, at most kConvMaxStages), across tile boundaries.
+// GEMM view of the forward pass: M = 128 output voxels (8 in x, 16 in y), a
+// block owns `zb` such planes above one another and `nt` output channels, K = 27
+// taps x C_in.  Per 16 input channels the block's input planes with their halo
+// (10 x 18 x (zb + 2) voxels) and the weights are brought into shared memory
+// ONCE, as 16-byte pieces [z][channel / 8][y][x][8 channels] by cp.async (zero
+// filled outside the grid, which is the padding).  In that no-swizzle layout the
+// 8 rows of a core matrix are 8 neighbours in x and the 16 groups lie one y row
+// apart, so every tap is the same tile at another start address: the tap needs no
+// copy of its own.  The three taps of a (dy, dx) pair that differ in dz read the
+// same input plane and write three neighbouring output planes, whose accumulators
+// lie side by side in tensor memory: one MMA with N = 3 nt does all three, so the
+// A tile, whose reading bounds these narrow layers (4 KB per MMA, 32 cycles, more
+// than the arithmetic for N < 128), is read 9 instead of 27 times per plane.
+//
+// The accumulators start from zero (tcgen05.st); the epilogue adds the bias,
+// clamps and stores.  Several blocks share a multiprocessor, so that one block's
+// loads and epilogue run under another's MMAs; zb, nt and the number of stages
+// follow from a cost model of the two (conv_plan).  Measured at 64 x 64 x 128, 16 ->
+// 16 channels: 25 us (293 TFLOP/s), 48 -> 16: 56 us (390); with one TMA copy of the
+// tile per tap, 256 rows of 16 bytes at some four cycles each, the ten layers of the
+// network took 3008 us, now 260.
+//
 // Every wait is bounded and raises an error flag.
 #include "internal.cuh"
 #include "tc.cuh"
 
 #include <cuda_bf16.h>
-#include <cudaTypedefs.h>
-#include <mutex>
-#include <tuple>
 
 namespace artss {
 
 namespace {
 
-constexpr int kConvThreads = 128;
-constexpr int kConvFwdThreads = 160;  // warps 0-3: epilogue (tensor-memory lanes 0..127); warp 4: loads and MMAs
-constexpr int kConvMaxStages = 16;
 constexpr int kConvPolls = 1 << 20;
-constexpr size_t kConvGuard = 64 * 1024;           // shared memory past the last stage, never addressed by a correct descriptor
-constexpr size_t kConvSmemMax = 227 * 1024 - 2048;  // dynamic limit minus the kernels' static shared memory
+constexpr int kConvThreads = 256;
+constexpr size_t kConvSmemMax = 227 * 1024 - 1024;  // dynamic limit minus the kernels' static shared memory
+constexpr int kTx = 8, kTy = 16;                    // output voxels of one MMA (M = 128)
+constexpr int kHx = kTx + 2, kHy = kTy + 2;         // with halo
+constexpr unsigned kRowB = kHx * 16;                // bytes between y rows of a channel group
+constexpr unsigned kGroupB = kHy * kRowB;           // bytes between channel groups (8 channels) of a plane
 
 struct ConvShape {
     int D, H, W, cin, cout;
-    int tw, th, tz;           // tile: tw x th x tz voxels, tw * th * tz = 128 (x fastest)
-    int tiles_x, tiles_y, tiles_z, tiles;
-    unsigned a_bytes, b_bytes, stage_bytes;
-    int stages;               // ring depth (taps in flight)
+    int tiles_x, tiles_y;
 };
 
-__global__ void __launch_bounds__(kConvFwdThreads, 1)
-k_conv3d_fwd(const __grid_constant__ CUtensorMap tm_x, const __nv_bfloat16 *__restrict__ wp,
-             const float *__restrict__ bias, __nv_bfloat16 *__restrict__ y, ConvShape s, int relu,
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool valid) {
+    const int n = valid ? 16 : 0;  // 0: the 16 bytes are zero-filled, nothing is read
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async_done() {
+    asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;\n" ::: "memory");
+}
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+    const uint32_t z = 0;
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+        "%1};\n" ::"r"(taddr),
+        "r"(z)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
+
+// the tile at (x0, y0) with its halo, planes z0 - 1 .. z0 - 2 + planes, `groups`
+// channel groups from c8 on, to [plane][group][y][x][16 bytes] at dst
+__device__ __forceinline__ void load_halo(uint32_t dst, const __nv_bfloat16 *__restrict__ x, const ConvShape &s,
+                                          int x0, int y0, int z0, int planes, int c8, int groups, int tid) {
+    const int n = planes * groups * kHx * kHy;
+    for (int e = tid; e < n; e += kConvThreads) {
+        const int g = e % groups, v = e / groups;  // groups of a voxel are neighbours in memory
+        const int xx = v % kHx, yy = (v / kHx) % kHy, zz = v / (kHx * kHy);
+        const int gx = x0 - 1 + xx, gy = y0 - 1 + yy, gz = z0 - 1 + zz;
+        const bool in = gx >= 0 && gx < s.W && gy >= 0 && gy < s.H && gz >= 0 && gz < s.D;
+        const __nv_bfloat16 *src = in ? x + (((size_t) gz * s.H + gy) * s.W + gx) * s.cin + (c8 + g) * 8 : x;
+        cp_async16(dst + (uint32_t) (zz * groups + g) * kGroupB + (uint32_t) yy * kRowB + (uint32_t) xx * 16, src, in);
+    }
+}
+
+struct ConvPlan {
+    int zb, nt, stages, tiles_z, cols;
+    unsigned a_bytes, b_bytes;
+    size_t smem;
+};
+
+__global__ void __launch_bounds__(kConvThreads)
+k_conv3d_fwd(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ wp,
+             const float *__restrict__ bias, __nv_bfloat16 *__restrict__ y, ConvShape s, ConvPlan p, int relu,
              int *__restrict__ err) {
-    extern __shared__ __align__(1024) uint8_t cv_sm[];
-    // full / empty: the stage ring; accf[a]: accumulator a holds a finished tile;
-    // acce[a]: the four epilogue warps have read accumulator a out
-    __shared__ __align__(8) uint64_t full[kConvMaxStages], empty[kConvMaxStages], accf[2], acce[2];
+    extern __shared__ __align__(128) uint8_t cv_sm[];
+    __shared__ __align__(8) uint64_t done[2];  // the MMAs of the stage's last use have completed
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int S = s.stages;
-    const unsigned tcols = s.cout <= 32 ? 32u : (s.cout <= 64 ? 64u : (s.cout <= 128 ? 128u : 256u));
+    const int tile = (int) blockIdx.x;
+    const int x0 = (tile % s.tiles_x) * kTx, y0 = ((tile / s.tiles_x) % s.tiles_y) * kTy,
+              z0 = (tile / (s.tiles_x * s.tiles_y)) * p.zb;
+    const int n0 = (int) blockIdx.y * p.nt;
+    const int zb = min(p.zb, s.D - z0);  // output planes of this block
+    const int nt = p.nt, chunks = s.cin / 16;
+    const uint32_t base = tc::smem_addr(cv_sm);
+    const unsigned stage_bytes = p.a_bytes + p.b_bytes;
+
+    // input planes z0 - 1 .. z0 + zb and the weights of input channels 16 c ..: the
+    // weights as [dy dx][channel / 8][dz][nt][8], dz descending, so that any run of
+    // dz is one operand of neighbouring rows
+    auto load = [&](int c) {
+        const uint32_t a = base + (uint32_t) (c % p.stages) * stage_bytes, b = a + p.a_bytes;
+        load_halo(a, x, s, x0, y0, z0, zb + 2, 2 * c, 2, tid);
+        for (int e = tid; e < 54 * nt; e += kConvThreads) {
+            const int n = e % nt, kc = (e / nt) & 1, tap = e / (2 * nt);
+            const int dz = tap / 9, t9 = tap % 9;
+            cp_async16(b + (uint32_t) ((t9 * 2 + kc) * 3 * nt + (2 - dz) * nt + n) * 16,
+                       wp + (((size_t) tap * (s.cin / 8) + 2 * c + kc) * s.cout + n0 + n) * 8, true);
+        }
+    };
+    load(0);
     if (tid == 0) {
-        for (int i = 0; i < S; i++) {
-            tc::mbar_init(&full[i], 1);
-            tc::mbar_init(&empty[i], 1);
-        }
-        for (int i = 0; i < 2; i++) {
-            tc::mbar_init(&accf[i], 1);
-            tc::mbar_init(&acce[i], 4);
-        }
+        tc::mbar_init(&done[0], 1);
+        tc::mbar_init(&done[1], 1);
         tc::fence_barrier_init();
     }
     if (warp == 0) {
-        tc::tmem_alloc(&tmem_base, 2 * tcols);
+        tc::tmem_alloc(&tmem_base, (unsigned) p.cols);
         tc::tmem_relinquish();
     }
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = tmem_base;
-    const int my_tiles = (s.tiles - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x;
-    const int nsteps = my_tiles * 27;
+    const uint32_t lanes = (uint32_t) (32 * (warp & 3)) << 16;
+    for (int c0 = 16 * (warp >> 2); c0 < zb * nt; c0 += 32) tmem_zero16(tmem + lanes + (uint32_t) c0);
+    tmem_store_wait();
+    tc::tc_fence_before();
 
-    if (warp == 4) {
-        if (lane == 0) {
-            const int kk_n = s.cin / 16;
-            const uint32_t idesc = tc::idesc_bf16(128, s.cout, 0, 0);
-            const unsigned lbo_a = 128 * 16, lbo_b = (unsigned) s.cout * 16;
-            // the loads of step p (tile p / 27, tap p % 27)
-            auto produce = [&](int p) {
-                const int st = p % S;
-                if (p >= S && !tc::mbar_wait(&empty[st], (unsigned) ((p / S - 1) & 1), kConvPolls)) return false;
-                const int tile = (int) blockIdx.x + (p / 27) * (int) gridDim.x, tap = p % 27;
-                const int tx = tile % s.tiles_x, ty = (tile / s.tiles_x) % s.tiles_y, tzi = tile / (s.tiles_x * s.tiles_y);
-                const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-                uint8_t *a = cv_sm + (size_t) st * s.stage_bytes;
-                tc::mbar_expect_tx(&full[st], s.a_bytes + s.b_bytes);
-                tc::tma_load_5d(a, &tm_x, 0, tx * s.tw + dx, ty * s.th + dy, tzi * s.tz + dz, 0, &full[st]);
-                tc::bulk_load(a + s.a_bytes, wp + (size_t) tap * s.cout * s.cin, s.b_bytes, &full[st]);
-                return true;
-            };
-            bool ok = true;
-            int issued = 0;  // steps whose loads were issued
-            for (int p = 0; p < S - 1 && p < nsteps && ok; p++)
-                if ((ok = produce(p))) issued = p + 1;
-            int step = 0;
-            for (int it = 0; it < my_tiles && ok; it++) {
-                const int acc = it & 1;
-                const uint32_t d = tmem + (uint32_t) acc * tcols;
-                // accumulator acc last held tile it - 2: wait until it was read out
-                if (it >= 2) ok = tc::mbar_wait(&acce[acc], (unsigned) (((it >> 1) - 1) & 1), kConvPolls);
-                tc::tc_fence_after();
-                for (int tap = 0; tap < 27 && ok; tap++, step++) {
-                    if (step + S - 1 < nsteps && (ok = produce(step + S - 1))) issued = step + S;
-                    const int st = step % S;
-                    if (ok) ok = tc::mbar_wait(&full[st], (unsigned) ((step / S) & 1), kConvPolls);
-                    if (!ok) break;
-                    tc::tc_fence_after();
-                    const uint8_t *a = cv_sm + (size_t) st * s.stage_bytes;
-                    const uint8_t *b = a + s.a_bytes;
-                    for (int kk = 0; kk < kk_n; kk++) {
-                        const uint64_t da = tc::smem_desc(a + 2 * kk * lbo_a, lbo_a, 128);
-                        const uint64_t db = tc::smem_desc(b + 2 * kk * lbo_b, lbo_b, 128);
-                        tc::mma_bf16(d, da, db, idesc, (tap | kk) != 0);
-                    }
-                    tc::mma_commit(&empty[st]);
-                }
-                if (ok) tc::mma_commit(&accf[acc]);
-            }
-            if (!ok) {
-                if (err) atomicExch(err, 1);
-                // let this block's loads and MMAs in flight finish before it leaves
-                for (int p = step; p < issued; p++)
-                    (void) tc::mbar_wait(&full[p % S], (unsigned) ((p / S) & 1), kConvPolls);
-                if (step > 0)
-                    (void) tc::mbar_wait(&empty[(step - 1) % S], (unsigned) (((step - 1) / S) & 1), kConvPolls);
-            }
-        }
-    } else {
-        // epilogue: lane = voxel of the tile, columns = output channels
-        for (int it = 0; it < my_tiles; it++) {
-            const int acc = it & 1;
-            if (!tc::mbar_wait(&accf[acc], (unsigned) ((it >> 1) & 1), kConvPolls)) {
-                if (lane == 0 && err) atomicExch(err, 1);
-                break;
-            }
+    bool ok = true;
+    for (int c = 0; c < chunks && ok; c++) {
+        cp_async_done();
+        tc::fence_proxy_async();  // this thread's pieces, before the tensor core reads them
+        __syncthreads();
+        if (tid == 0) {
             tc::tc_fence_after();
-            const int tile = (int) blockIdx.x + it * (int) gridDim.x;
-            const int tx = tile % s.tiles_x, ty = (tile / s.tiles_x) % s.tiles_y, tzi = tile / (s.tiles_x * s.tiles_y);
-            const int vx = tx * s.tw + tid % s.tw, vy = ty * s.th + (tid / s.tw) % s.th,
-                      vz = tzi * s.tz + tid / (s.tw * s.th);
-            __nv_bfloat16 *yo = y + (((size_t) vz * s.H + vy) * s.W + vx) * s.cout;
-            const uint32_t src = tmem + (uint32_t) acc * tcols + ((uint32_t) (32 * warp) << 16);
-            for (int c0 = 0; c0 < s.cout; c0 += 16) {
+            const uint8_t *a = cv_sm + (size_t) (c % p.stages) * stage_bytes, *b = a + p.a_bytes;
+            for (int q = 0; q < zb + 2; q++) {
+                // input plane q feeds output planes q - 2 (dz = +1), q - 1, q (dz = -1)
+                const int lo = max(0, q - 2), hi = min(zb - 1, q), nz = hi - lo + 1;
+                const int gz = z0 - 1 + q;
+                if (gz < 0 || gz >= s.D) continue;  // padding adds nothing
+                const uint32_t idesc = tc::idesc_bf16(128, nz * nt, 0, 0);
+                const uint8_t *aq = a + (size_t) q * 2 * kGroupB, *bq = b + (size_t) (lo - q + 2) * nt * 16;
+#pragma unroll
+                for (int t = 0; t < 9; t++)
+                    tc::mma_bf16(tmem + (uint32_t) (lo * nt),
+                                 tc::smem_desc(aq + (t / 3) * kRowB + (t % 3) * 16, kGroupB, kRowB),
+                                 tc::smem_desc(bq + (size_t) t * 6 * nt * 16, (unsigned) (3 * nt * 16), 128), idesc, 1);
+            }
+            tc::mma_commit(&done[c % p.stages]);
+        }
+        const int n = c + 1;
+        if (n < chunks) {
+            // the stage of chunk n was last read by the MMAs of chunk n - stages
+            const int u = n - p.stages;
+            if (u >= 0) ok = tc::mbar_wait(&done[u % p.stages], (unsigned) ((u / p.stages) & 1), kConvPolls);
+            if (ok) load(n);
+            // no thread leaves the loop before the others have seen the same
+            ok = !__syncthreads_or(!ok);
+        }
+    }
+    if (ok) ok = tc::mbar_wait(&done[(chunks - 1) % p.stages], (unsigned) (((chunks - 1) / p.stages) & 1), kConvPolls);
+    if (__syncthreads_or(!ok)) {
+        if (tid == 0 && err) atomicExch(err, 1);
+        cp_async_done();
+    } else {
+        tc::tc_fence_after();
+        // lane = voxel of the tile, columns = planes x output channels
+        const int row = 32 * (warp & 3) + lane, vx = x0 + row % kTx, vy = y0 + row / kTx;
+        const bool in = vx < s.W && vy < s.H;
+        for (int z = warp >> 2; z < zb; z += 2) {
+            __nv_bfloat16 *yo = y + (((size_t) (z0 + z) * s.H + vy) * s.W + vx) * s.cout + n0;
+            for (int c0 = 0; c0 < nt; c0 += 16) {
                 float v[16];
-                tc::tmem_ld16(src + (uint32_t) c0, v);
+                tc::tmem_ld16(tmem + lanes + (uint32_t) (z * nt + c0), v);
                 __align__(16) __nv_bfloat16 o[16];
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
-                    float r = v[i] + (bias ? bias[c0 + i] : 0.f);
+                    float r = v[i] + (bias ? __ldg(bias + n0 + c0 + i) : 0.f);
                     if (relu) r = fmaxf(r, 0.f);
                     o[i] = __float2bfloat16_rn(r);
                 }
-                uint4 *dst = reinterpret_cast<uint4 *>(yo + c0);
-                dst[0] = reinterpret_cast<const uint4 *>(o)[0];
-                dst[1] = reinterpret_cast<const uint4 *>(o)[1];
+                if (in) {
+                    uint4 *dst = reinterpret_cast<uint4 *>(yo + c0);
+                    dst[0] = reinterpret_cast<const uint4 *>(o)[0];
+                    dst[1] = reinterpret_cast<const uint4 *>(o)[1];
+                }
             }
-            tc::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&acce[acc]);
         }
+        tc::tc_fence_before();
     }
-    tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
-    if (warp == 0) tc::tmem_dealloc(tmem, 2 * tcols);
+    if (warp == 0) tc::tmem_dealloc(tmem, (unsigned) p.cols);
 }
 
 // Weight gradient dW[t][co][ci] += sum_v dY[v][co] x[v + off_t][ci] as a GEMM
-// with M = C_out (padded to 128 by TMA's zero fill), N = C_in, K = voxels.
-// The activation tiles keep the forward's shared-memory layout
-// [channel/8][128 voxels][8], which read as MN-major operands is exactly the
-// canonical layout: 8 voxels (K) x 8 channels (M or N) per core matrix, the
-// core matrices of one channel group 128 bytes apart (LBO), channel groups
-// 2048 bytes apart (SBO).  A block accumulates one tap over its range of
-// voxel tiles in tensor memory, then adds the C_out x C_in block to dW with
-// FP32 atomics (dW must be zeroed by the caller), and moves to the next tap.
-constexpr int kWgradMRows = 128;
+// with M = C_out (128 rows, those past C_out ignored), N = (dz, C_in), K = voxels.
+// The activation tiles keep the forward's shared-memory layout, which read as
+// MN-major operands is 8 voxels (K) x 8 channels (M or N) per core matrix, the
+// next 8 voxels one y row on (LBO) and the next 8 channels one channel group on
+// (SBO); the channel groups of planes z - 1, z, z + 1 follow one another at the
+// same distance, so the three dz taps are one operand of N = 3 ct columns and an
+// x tile is loaded once for all its taps (before: one 256-row copy per tap).
+// A block accumulates `tg` (dy, dx) pairs for `ct` input channels over all its
+// voxel tiles in tensor memory and adds them to dW once, with FP32 atomics (dW
+// must be zeroed by the caller).
+struct WgradPlan {
+    int ct, tg, groups, tiles_z, cols;  // groups of (dy, dx) pairs
+    unsigned a_bytes, b_bytes;
+    size_t smem;
+};
 
-__global__ void __launch_bounds__(kConvThreads, 1)
-k_conv3d_wgrad(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_dy,
-               float *__restrict__ dw, ConvShape s, int tiles_per_block, int *__restrict__ err) {
-    extern __shared__ __align__(1024) uint8_t cv_sm[];
-    __shared__ __align__(8) uint64_t full[kConvMaxStages], empty[kConvMaxStages], accb;
+__global__ void __launch_bounds__(kConvThreads)
+k_conv3d_wgrad(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ dy, float *__restrict__ dw,
+               ConvShape s, WgradPlan p, int *__restrict__ err) {
+    extern __shared__ __align__(128) uint8_t cv_sm[];
+    __shared__ __align__(8) uint64_t done[2];
     __shared__ uint32_t tmem_base;
-    __shared__ int s_fail;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int S = s.stages;
-    const unsigned tcols = s.cin <= 32 ? 32u : (s.cin <= 64 ? 64u : (s.cin <= 128 ? 128u : 256u));
-    const int t_begin = (int) blockIdx.x * tiles_per_block;
-    const int t_end = min(s.tiles, t_begin + tiles_per_block);
-    const int ntile = t_end - t_begin;
-    if (ntile <= 0) return;
-    if (tid == 0) {
-        for (int i = 0; i < S; i++) {
-            tc::mbar_init(&full[i], 1);
-            tc::mbar_init(&empty[i], 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tiles = s.tiles_x * s.tiles_y * s.D;
+    const int t0 = (int) blockIdx.y % p.groups * p.tg, nt = min(p.tg, 9 - t0);  // this block's (dy, dx) pairs
+    const int ci0 = (int) blockIdx.y / p.groups * p.ct;
+    const int g_in = p.ct / 8, g_out = s.cout / 8;
+    const uint32_t base = tc::smem_addr(cv_sm);
+    const unsigned stage_bytes = p.a_bytes + p.b_bytes;
+    auto load = [&](int it) {
+        const int tile = (int) blockIdx.x + it * (int) gridDim.x;
+        const int x0 = (tile % s.tiles_x) * kTx, y0 = ((tile / s.tiles_x) % s.tiles_y) * kTy,
+                  z = tile / (s.tiles_x * s.tiles_y);
+        const uint32_t a = base + (uint32_t) (it & 1) * stage_bytes, b = a + p.a_bytes;
+        // dY tile [channel / 8][y][x][8]
+        for (int e = tid; e < g_out * kTx * kTy; e += kConvThreads) {
+            const int g = e % g_out, v = e / g_out, gx = x0 + v % kTx, gy = y0 + v / kTx;
+            const bool in = gx < s.W && gy < s.H;
+            cp_async16(a + (uint32_t) g * (kTx * kTy * 16) + (uint32_t) v * 16,
+                       in ? dy + (((size_t) z * s.H + gy) * s.W + gx) * s.cout + g * 8 : dy, in);
         }
-        tc::mbar_init(&accb, 1);
+        load_halo(b, x, s, x0, y0, z, 3, ci0 / 8, g_in, tid);
+    };
+    const int my_tiles = (tiles - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x;  // >= 1
+    load(0);
+    if (tid == 0) {
+        tc::mbar_init(&done[0], 1);
+        tc::mbar_init(&done[1], 1);
         tc::fence_barrier_init();
-        s_fail = 0;
     }
     if (warp == 0) {
-        tc::tmem_alloc(&tmem_base, tcols);
+        tc::tmem_alloc(&tmem_base, (unsigned) p.cols);
         tc::tmem_relinquish();
     }
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = tmem_base;
-    const int nsteps = 27 * ntile;
-    const uint32_t idesc = tc::idesc_bf16(kWgradMRows, s.cin, 1, 1);
-    const unsigned a_bytes = (unsigned) kWgradMRows * 128u * 2u;  // dY tile, 16 channel groups
-    const unsigned b_bytes = s.a_bytes;                            // x tile, C_in/8 channel groups
-
-    auto produce = [&](int p) {
-        const int st = p % S;
-        if (p >= S && !tc::mbar_wait(&empty[st], (unsigned) ((p / S - 1) & 1), kConvPolls)) return false;
-        const int tap = p / ntile, tile = t_begin + p % ntile;
-        const int tx = tile % s.tiles_x, ty = (tile / s.tiles_x) % s.tiles_y, tzi = tile / (s.tiles_x * s.tiles_y);
-        const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-        uint8_t *a = cv_sm + (size_t) st * s.stage_bytes;
-        tc::mbar_expect_tx(&full[st], a_bytes + b_bytes);
-        tc::tma_load_5d(a, &tm_dy, 0, tx * s.tw, ty * s.th, tzi * s.tz, 0, &full[st]);
-        tc::tma_load_5d(a + a_bytes, &tm_x, 0, tx * s.tw + dx, ty * s.th + dy, tzi * s.tz + dz, 0, &full[st]);
-        return true;
-    };
-
+    const uint32_t idesc = tc::idesc_bf16(128, 3 * p.ct, 1, 1);
     bool ok = true;
-    int step = 0;
-    if (tid == 0)
-        for (int p = 0; p < S - 1 && p < nsteps && ok; p++) ok = produce(p);
-    for (int tap = 0; tap < 27; tap++) {
-        if (tid == 0 && ok) {
-            for (int i = 0; i < ntile && ok; i++, step++) {
-                if (step + S - 1 < nsteps) ok = produce(step + S - 1);
-                const int st = step % S;
-                if (ok) ok = tc::mbar_wait(&full[st], (unsigned) ((step / S) & 1), kConvPolls);
-                if (!ok) break;
-                tc::tc_fence_after();
-                const uint8_t *a = cv_sm + (size_t) st * s.stage_bytes;
-                const uint8_t *b = a + a_bytes;
-#pragma unroll
-                for (int kk = 0; kk < 8; kk++) {  // 16 voxels per MMA
-                    const uint64_t da = tc::smem_desc(a + kk * 256, 128, 2048);
-                    const uint64_t db = tc::smem_desc(b + kk * 256, 128, 2048);
-                    tc::mma_bf16(tmem, da, db, idesc, (i | kk) != 0);
-                }
-                tc::mma_commit(&empty[st]);
-                if (i == ntile - 1) tc::mma_commit(&accb);
-            }
-            if (!ok) s_fail = 1;
-        }
-        bool acc_ok = true;
-        if (tid == 0) acc_ok = ok && tc::mbar_wait(&accb, (unsigned) (tap & 1), kConvPolls);
-        if (__syncthreads_or(!acc_ok || s_fail)) {
-            if (tid == 0 && err) atomicExch(err, 1);
-            break;
-        }
-        tc::tc_fence_after();
-        // lane = output channel co, columns = input channels
-        for (int c0 = 0; c0 < s.cin; c0 += 16) {
-            float v[16];
-            tc::tmem_ld16(tmem + ((uint32_t) (32 * warp) << 16) + (uint32_t) c0, v);
-            if (tid < s.cout) {
-                float *d = dw + ((size_t) tap * s.cout + tid) * s.cin + c0;
-#pragma unroll
-                for (int i = 0; i < 16; i++) atomicAdd(d + i, v[i]);
-            }
-        }
-        tc::tc_fence_before();
+    for (int it = 0; it < my_tiles && ok; it++) {
+        cp_async_done();
+        tc::fence_proxy_async();
         __syncthreads();
+        if (tid == 0) {
+            tc::tc_fence_after();
+            const uint8_t *a = cv_sm + (size_t) (it & 1) * stage_bytes, *b = a + p.a_bytes;
+            for (int t = 0; t < nt; t++) {
+                const uint8_t *bt = b + ((t0 + t) / 3) * kRowB + ((t0 + t) % 3) * 16;
+#pragma unroll
+                for (int kk = 0; kk < kTy / 2; kk++)  // 16 voxels (two y rows) per MMA
+                    tc::mma_bf16(tmem + (uint32_t) (t * 3 * p.ct),
+                                 tc::smem_desc(a + kk * 2 * kTx * 16, kTx * 16, kTx * kTy * 16),
+                                 tc::smem_desc(bt + kk * 2 * kRowB, kRowB, kGroupB), idesc, (it | kk) != 0);
+            }
+            tc::mma_commit(&done[it & 1]);
+        }
+        const int n = it + 1;
+        if (n < my_tiles) {
+            if (n >= 2) ok = tc::mbar_wait(&done[n & 1], (unsigned) (((n - 2) >> 1) & 1), kConvPolls);
+            if (ok) load(n);
+            ok = !__syncthreads_or(!ok);
+        }
+    }
+    if (ok) ok = tc::mbar_wait(&done[(my_tiles - 1) & 1], (unsigned) (((my_tiles - 1) >> 1) & 1), kConvPolls);
+    if (__syncthreads_or(!ok)) {
+        if (tid == 0 && err) atomicExch(err, 1);
+        cp_async_done();
+    } else {
+        tc::tc_fence_after();
+        // lane = output channel co, columns = (pair, dz, input channel)
+        const int co = 32 * (warp & 3) + lane;
+        const uint32_t src = tmem + ((uint32_t) (32 * (warp & 3)) << 16);
+        const int nc = nt * 3 * p.ct / 16;
+        if (32 * (warp & 3) < s.cout)
+            for (int q = warp >> 2; q < nc; q += 2) {
+                const int c = 16 * q, pair = t0 + c / (3 * p.ct), dz = c / p.ct % 3, ci = ci0 + c % p.ct;
+                float v[16];
+                tc::tmem_ld16(src + (uint32_t) c, v);
+                if (co < s.cout) {
+                    float *d = dw + ((size_t) (9 * dz + pair) * s.cout + co) * s.cin + ci;
+#pragma unroll
+                    for (int i = 0; i < 16; i++) atomicAdd(d + i, v[i]);
+                }
+            }
+        tc::tc_fence_before();
     }
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tmem, tcols);
+    tc::tc_fence_after();
+    if (warp == 0) tc::tmem_dealloc(tmem, (unsigned) p.cols);
 }
 
-PFN_cuTensorMapEncodeTiled_v12000 g_enc = nullptr;
-std::once_flag g_enc_once;
-
-// map of a [D][H][W][c] activation whose box lands as [box_chunks][th][tw][8]
-int encode_act_map(const __nv_bfloat16 *x, const ConvShape &s, int c, int box_chunks, CUtensorMap *m);
-
-int encode_x_map(const __nv_bfloat16 *x, const ConvShape &s, CUtensorMap *m) {
-    return encode_act_map(x, s, s.cin, s.cin / 8, m);
+int tmem_cols(int n) {
+    int c = 32;
+    while (c < n) c *= 2;
+    return c;
 }
 
-int encode_act_map(const __nv_bfloat16 *x, const ConvShape &s, int c, int box_chunks, CUtensorMap *m) {
-    std::call_once(g_enc_once, [] {
-        cudaDriverEntryPointQueryResult q;
-        void *fn = nullptr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            g_enc = (PFN_cuTensorMapEncodeTiled_v12000) fn;
-    });
-    if (!g_enc) { set_error("cuTensorMapEncodeTiled is not available"); return ARTSS_ERR_CUDA; }
-    // dims: channel-in-chunk (8), x, y, z, chunk -> a box lands as [chunk][z][y][x][8]
-    const cuuint64_t dim[5] = {8, (cuuint64_t) s.W, (cuuint64_t) s.H, (cuuint64_t) s.D, (cuuint64_t) (c / 8)};
-    const cuuint64_t es = 2;
-    const cuuint64_t stride[4] = {(cuuint64_t) c * es, (cuuint64_t) s.W * c * es, (cuuint64_t) s.H * s.W * c * es, 16};
-    const cuuint32_t box[5] = {8, (cuuint32_t) s.tw, (cuuint32_t) s.th, (cuuint32_t) s.tz, (cuuint32_t) box_chunks};
-    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    const CUresult r = g_enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, (void *) x, dim, stride, box, estr,
-                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) { set_error("conv3d: input tensor map rejected"); return ARTSS_ERR_ARG; }
-    return ARTSS_OK;
-}
-
-// stages of `bytes` each that fit the dynamic shared memory with kConvGuardMin
-// left over, at most kConvMaxStages
-constexpr size_t kConvGuardMin = 16 * 1024;
-int conv_stages(size_t bytes) {
-    return (int) std::min<size_t>(kConvMaxStages, (kConvSmemMax - kConvGuardMin) / bytes);
+// the largest divisor of c that is a multiple of 16 and at most `most`
+int channel_tile(int c, int most) {
+    for (int t = std::min(c, most) / 16 * 16; t > 16; t -= 16)
+        if (c % t == 0) return t;
+    return 16;
 }
 
 int conv_shape(const artss_conv_desc *d, ConvShape *s) {
@@ -332,27 +339,50 @@ int conv_shape(const artss_conv_desc *d, ConvShape *s) {
         set_error("conv3d: channels must be multiples of 16, at most 256");
         return ARTSS_ERR_ARG;
     }
-    s->D = d->D; s->H = d->H; s->W = d->W; s->cin = d->cin; s->cout = d->cout;
-    s->tz = 1;
-    if (d->W % 128 == 0) { s->tw = 128; s->th = 1; }
-    else if (128 % d->W == 0 && d->W * d->H >= 128 && d->H % (128 / d->W) == 0) { s->tw = d->W; s->th = 128 / d->W; }
-    else if (128 % (d->W * d->H) == 0 && d->D % (128 / (d->W * d->H)) == 0) {
-        s->tw = d->W; s->th = d->H; s->tz = 128 / (d->W * d->H);
-    } else {
+    if (!(d->W % 128 == 0 || (128 % d->W == 0 && d->W * d->H >= 128 && d->H % (128 / d->W) == 0) ||
+          (128 % (d->W * d->H) == 0 && d->D % (128 / (d->W * d->H)) == 0))) {
         set_error("conv3d: 128-voxel tiles must fit: W a multiple of 128, or W dividing 128 with H a multiple of "
                   "128/W, or W*H dividing 128 with D a multiple of 128/(W*H)");
         return ARTSS_ERR_ARG;
     }
-    s->tiles_x = d->W / s->tw;
-    s->tiles_y = d->H / s->th;
-    s->tiles_z = d->D / s->tz;
-    s->tiles = s->tiles_x * s->tiles_y * s->tiles_z;
-    s->a_bytes = 128u * (unsigned) d->cin * 2u;
-    s->b_bytes = (unsigned) d->cout * (unsigned) d->cin * 2u;
-    s->stage_bytes = (s->a_bytes + s->b_bytes + 1023u) & ~1023u;
-    s->stages = conv_stages(s->stage_bytes);
-    if (s->stages < 2) { set_error("conv3d: stages too large"); return ARTSS_ERR_LIMIT; }
+    // 128 voxels x C_in and C_out x C_in operands of more than 104 KB together are not taken
+    if ((size_t) 2 * d->cin * (128 + d->cout) > 104 * 1024) { set_error("conv3d: stages too large"); return ARTSS_ERR_LIMIT; }
+    *s = ConvShape{d->D, d->H, d->W, d->cin, d->cout, (d->W + kTx - 1) / kTx, (d->H + kTy - 1) / kTy};
     return ARTSS_OK;
+}
+
+// zb and nt of the forward kernel: the pair with the least
+//     waves x (shared-memory cycles of its MMAs + cycles of its loads)
+// where one MMA reads 4 KB of A and 96 nt bytes of B at 128 bytes a cycle and
+// loads arrive at some 48 bytes a cycle and multiprocessor.  At 64 x 64 x 128
+// this takes 8 planes for the 16-channel layers (512 blocks, 3 a multiprocessor)
+// and 1 plane with 32 of the 64 channels on 16 x 16 x 32 (128 blocks: 64 with all
+// channels would leave half of the chip idle).
+ConvPlan conv_plan(const ConvShape &s, int sms) {
+    ConvPlan best{};
+    double least = 0;
+    for (int zb = 8; zb >= 1; zb /= 2)
+        for (int nt = channel_tile(s.cout, 64); nt >= 16; nt = nt > 16 ? channel_tile(s.cout, nt - 16) : 0) {
+            ConvPlan p{};
+            p.zb = zb;
+            p.nt = nt;
+            p.tiles_z = (s.D + zb - 1) / zb;
+            p.cols = tmem_cols(zb * nt);
+            p.a_bytes = (unsigned) (zb + 2) * 2 * kGroupB;
+            p.b_bytes = (unsigned) (54 * nt * 16);
+            const size_t stage = p.a_bytes + p.b_bytes;
+            if (p.cols > 256 || stage > kConvSmemMax / 2) continue;  // two blocks a multiprocessor
+            p.stages = s.cin > 16 && 2 * stage <= kConvSmemMax / 2 ? 2 : 1;
+            p.smem = p.stages * stage;
+            const int64_t blocks = (int64_t) s.tiles_x * s.tiles_y * p.tiles_z * (s.cout / nt);
+            const double cost = (double) ((blocks + sms - 1) / sms) *
+                                ((zb + 2) * 9. * (32. + 0.75 * nt) + (double) stage / 48.);
+            if (least == 0 || cost < least) {
+                least = cost;
+                best = p;
+            }
+        }
+    return best;
 }
 
 }  // namespace
@@ -361,26 +391,27 @@ int conv3d_wgrad(artss_ctx *ctx, const artss_conv_desc *d, const void *x, const 
     ConvShape s;
     int st = conv_shape(d, &s);
     if (st) return st;
-    if (d->cout > kWgradMRows || d->cin > 128) { set_error("conv3d wgrad: C_out and C_in at most 128"); return ARTSS_ERR_ARG; }
+    if (d->cout > 128 || d->cin > 128) { set_error("conv3d wgrad: C_out and C_in at most 128"); return ARTSS_ERR_ARG; }
     if (((uintptr_t) x & 15) || ((uintptr_t) dy & 15)) { set_error("conv3d: arrays must be 16-byte aligned"); return ARTSS_ERR_ARG; }
-    CUtensorMap mx, mdy;
-    if ((st = encode_act_map((const __nv_bfloat16 *) x, s, s.cin, s.cin / 8, &mx))) return st;
-    if ((st = encode_act_map((const __nv_bfloat16 *) dy, s, s.cout, kWgradMRows / 8, &mdy))) return st;
-    // stage: dY tile (128 voxels x 128 padded channels) + x tile
-    const unsigned stage = ((unsigned) kWgradMRows * 128u * 2u + s.a_bytes + 1023u) & ~1023u;
-    s.stage_bytes = stage;
-    s.stages = conv_stages(stage);
-    if (s.stages < 2) { set_error("conv3d wgrad: stages too large"); return ARTSS_ERR_LIMIT; }
-    const size_t stages = (size_t) stage * s.stages;
-    const size_t smem = stages + std::min<size_t>(kConvGuard, kConvSmemMax - stages);
-    ARTSS_CK(cudaFuncSetAttribute(k_conv3d_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    const int grid = std::min(s.tiles, sms);
-    const int per = (s.tiles + grid - 1) / grid;
-    const int blocks = (s.tiles + per - 1) / per;
-    ARTSS_LAUNCH(ctx, FAM_CONV, k_conv3d_wgrad<<<blocks, kConvThreads, smem, ctx->stream>>>(
-                                    mx, mdy, dw, s, per, &ctx->d_loop[kNnErrSlot].pad));
+    WgradPlan p{};
+    p.ct = channel_tile(s.cin, 64);            // N = 3 ct <= 192
+    p.tg = std::min(9, 512 / (3 * p.ct));      // accumulators of tg pairs fill tensor memory
+    if (p.tg < 9) p.tg = p.tg >= 3 ? 3 : 1;    // whole dy rows
+    p.groups = (9 + p.tg - 1) / p.tg;
+    p.cols = tmem_cols(p.tg * 3 * p.ct);
+    p.a_bytes = (unsigned) (s.cout / 8) * kTx * kTy * 16;
+    p.b_bytes = 3u * (unsigned) (p.ct / 8) * kGroupB;
+    // the A operand's rows past C_out read on behind the dY tile, within the block's shared memory
+    p.smem = std::max<size_t>(2 * ((size_t) p.a_bytes + p.b_bytes),
+                              (size_t) p.a_bytes + p.b_bytes + 16 * kTx * kTy * 16);
+    if (p.smem > kConvSmemMax) { set_error("conv3d wgrad: stages too large"); return ARTSS_ERR_LIMIT; }
+    ARTSS_CK(cudaFuncSetAttribute(k_conv3d_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kConvSmemMax));
+    const int tiles = s.tiles_x * s.tiles_y * s.D, yb = p.groups * (s.cin / p.ct);
+    // one block a multiprocessor (tensor memory), the parts of dW side by side
+    const int gx = std::max(1, std::min(tiles, std::max(ctx->sm_count, 1) / yb));
+    ARTSS_LAUNCH(ctx, FAM_CONV, k_conv3d_wgrad<<<dim3((unsigned) gx, (unsigned) yb), kConvThreads, p.smem, ctx->stream>>>(
+                                    (const __nv_bfloat16 *) x, (const __nv_bfloat16 *) dy, dw, s, p,
+                                    &ctx->d_loop[kNnErrSlot].pad));
     ARTSS_LAUNCH_CK(ctx);
     return ARTSS_OK;
 }
@@ -392,17 +423,12 @@ int conv3d_fwd(artss_ctx *ctx, const artss_conv_desc *d, const void *x, const vo
     if (((uintptr_t) x & 15) || ((uintptr_t) wp & 15) || ((uintptr_t) y & 15)) {
         set_error("conv3d: arrays must be 16-byte aligned"); return ARTSS_ERR_ARG;
     }
-    CUtensorMap m;
-    if ((st = encode_x_map((const __nv_bfloat16 *) x, s, &m))) return st;
-    const size_t stages = (size_t) s.stage_bytes * s.stages;
-    const size_t smem = stages + std::min<size_t>(kConvGuard, kConvSmemMax - stages);
-    ARTSS_CK(cudaFuncSetAttribute(k_conv3d_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    const int grid = std::min(s.tiles, sms);
-    ARTSS_LAUNCH(ctx, FAM_CONV, k_conv3d_fwd<<<grid, kConvFwdThreads, smem, ctx->stream>>>(
-                                    m, (const __nv_bfloat16 *) wp, bias, (__nv_bfloat16 *) y, s, d->relu,
-                                    &ctx->d_loop[kNnErrSlot].pad));
+    const ConvPlan p = conv_plan(s, std::max(ctx->sm_count, 1));
+    ARTSS_CK(cudaFuncSetAttribute(k_conv3d_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kConvSmemMax));
+    const dim3 grid((unsigned) (s.tiles_x * s.tiles_y * p.tiles_z), (unsigned) (s.cout / p.nt));
+    ARTSS_LAUNCH(ctx, FAM_CONV, k_conv3d_fwd<<<grid, kConvThreads, p.smem, ctx->stream>>>(
+                                    (const __nv_bfloat16 *) x, (const __nv_bfloat16 *) wp, bias, (__nv_bfloat16 *) y, s,
+                                    p, d->relu, &ctx->d_loop[kNnErrSlot].pad));
     ARTSS_LAUNCH_CK(ctx);
     return ARTSS_OK;
 }

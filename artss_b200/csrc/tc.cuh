@@ -1,6 +1,6 @@
 // sm_100a building blocks of the tensor-core kernels: mbarriers with bounded
-// waits, TMA (tensor and 1-D bulk) loads, tcgen05 tensor-memory allocation,
-// MMA issue (kind::f16, BF16 inputs, FP32 accumulation), commit and loads.
+// waits, tcgen05 tensor-memory allocation, MMA issue (kind::f16, BF16 inputs,
+// FP32 accumulation), commit and loads.
 //
 // Shared-memory operands use the canonical no-swizzle layouts of the UMMA
 // matrix descriptor: "core matrices" of 8 rows x 16 bytes stored as 128
@@ -45,32 +45,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, int po
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 __device__ __forceinline__ void fence_barrier_init() {
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-}
-
-// ---- TMA loads (no multicast)
-__device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, int c4,
-                                            uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, "
-        "%6}], [%7];\n" ::"r"(smem_addr(dst)),
-        "l"((uint64_t) map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_addr(bar))
-        : "memory");
-}
-__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3,
-                                            uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-        "[%6];\n" ::"r"(smem_addr(dst)),
-        "l"((uint64_t) map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_addr(bar))
-        : "memory");
-}
-// 1-D bulk copy: both addresses 16-byte aligned, bytes a multiple of 16
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes, uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-            smem_addr(dst)),
-        "l"((uint64_t) src), "r"(bytes), "r"(smem_addr(bar))
-        : "memory");
 }
 
 // ---- tensor memory
