@@ -18,94 +18,192 @@ inline unsigned nblk(int64_t n, int t = 256) {
 
 #define NN_LOOP(n) for (int64_t q = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; q < (n); q += (int64_t) gridDim.x * blockDim.x)
 
+// The activation kernels are bound by memory: each thread moves V channels of a
+// voxel at once, V = 8 (one 16-byte access) where the channel counts and offsets
+// are multiples of 8 and the arrays 16-byte aligned, which every layer of the
+// network is, else V = 1.  With 2-byte accesses the six of a 64 x 64 x 128
+// inference took 197 us, with these some 60.
+template <int V>
+struct Ch {
+    float v[V];
+};
+template <int V>
+__device__ __forceinline__ Ch<V> ch_load(const __nv_bfloat16 *__restrict__ p) {
+    Ch<V> r;
+    if constexpr (V == 8) {
+        const uint4 u = *reinterpret_cast<const uint4 *>(p);
+        const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&u);
+#pragma unroll
+        for (int i = 0; i < 8; i++) r.v[i] = bf(e[i]);
+    } else {
+        r.v[0] = bf(*p);
+    }
+    return r;
+}
+template <int V>
+__device__ __forceinline__ void ch_store(__nv_bfloat16 *__restrict__ p, const Ch<V> &r) {
+    if constexpr (V == 8) {
+        uint4 u;
+        __nv_bfloat16 *e = reinterpret_cast<__nv_bfloat16 *>(&u);
+#pragma unroll
+        for (int i = 0; i < 8; i++) e[i] = __float2bfloat16_rn(r.v[i]);
+        *reinterpret_cast<uint4 *>(p) = u;
+    } else {
+        *p = __float2bfloat16_rn(r.v[0]);
+    }
+}
+inline bool vec8(std::initializer_list<const void *> ptrs, std::initializer_list<int> channels) {
+    for (const void *p : ptrs)
+        if ((uintptr_t) p & 15) return false;
+    for (int c : channels)
+        if (c % 8) return false;
+    return true;
+}
+
 // dy *= (y > 0): ReLU backward through the stored forward output
+template <int V>
 __global__ void k_relu_bwd(__nv_bfloat16 *__restrict__ dy, const __nv_bfloat16 *__restrict__ y, int64_t n) {
-    NN_LOOP(n) if (!(bf(y[q]) > 0.f)) dy[q] = __float2bfloat16_rn(0.f);
+    NN_LOOP(n / V) {
+        const Ch<V> a = ch_load<V>(y + q * V);
+        Ch<V> g = ch_load<V>(dy + q * V);
+#pragma unroll
+        for (int i = 0; i < V; i++)
+            if (!(a.v[i] > 0.f)) g.v[i] = 0.f;
+        ch_store<V>(dy + q * V, g);
+    }
 }
 
 // 2x2x2 average pooling, [D][H][W][C] -> [D/2][H/2][W/2][C]
+template <int V>
 __global__ void k_pool2(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ y, int D, int H, int W, int C) {
-    const int64_t n = (int64_t) (D / 2) * (H / 2) * (W / 2) * C;
+    const int64_t n = (int64_t) (D / 2) * (H / 2) * (W / 2) * (C / V);
     NN_LOOP(n) {
-        const int c = (int) (q % C);
-        int64_t v = q / C;
+        const int c = (int) (q % (C / V)) * V;
+        int64_t v = q / (C / V);
         const int xo = (int) (v % (W / 2)); v /= (W / 2);
         const int yo = (int) (v % (H / 2));
         const int zo = (int) (v / (H / 2));
-        float s = 0.f;
+        Ch<V> s{};
 #pragma unroll
-        for (int o = 0; o < 8; o++)
-            s += bf(x[(((int64_t) (2 * zo + (o >> 2)) * H + 2 * yo + ((o >> 1) & 1)) * W + 2 * xo + (o & 1)) * C + c]);
-        y[q] = __float2bfloat16_rn(0.125f * s);
+        for (int o = 0; o < 8; o++) {
+            const Ch<V> e = ch_load<V>(
+                x + (((int64_t) (2 * zo + (o >> 2)) * H + 2 * yo + ((o >> 1) & 1)) * W + 2 * xo + (o & 1)) * C + c);
+#pragma unroll
+            for (int i = 0; i < V; i++) s.v[i] += e.v[i];
+        }
+#pragma unroll
+        for (int i = 0; i < V; i++) s.v[i] = 0.125f * s.v[i];
+        ch_store<V>(y + q * V, s);
     }
 }
 
 // backward of the pooling: dx = dy / 8 on each of the 8 children
+template <int V>
 __global__ void k_pool2_bwd(const __nv_bfloat16 *__restrict__ dy, __nv_bfloat16 *__restrict__ dx, int D, int H, int W,
                             int C) {
-    const int64_t n = (int64_t) D * H * W * C;
+    const int64_t n = (int64_t) D * H * W * (C / V);
     NN_LOOP(n) {
-        const int c = (int) (q % C);
-        int64_t v = q / C;
+        const int c = (int) (q % (C / V)) * V;
+        int64_t v = q / (C / V);
         const int x = (int) (v % W); v /= W;
         const int y = (int) (v % H);
         const int z = (int) (v / H);
-        dx[q] = __float2bfloat16_rn(0.125f * bf(dy[(((int64_t) (z / 2) * (H / 2) + y / 2) * (W / 2) + x / 2) * C + c]));
+        Ch<V> g = ch_load<V>(dy + (((int64_t) (z / 2) * (H / 2) + y / 2) * (W / 2) + x / 2) * C + c);
+#pragma unroll
+        for (int i = 0; i < V; i++) g.v[i] = 0.125f * g.v[i];
+        ch_store<V>(dx + q * V, g);
     }
 }
 
 // nearest 2x upsampling of [D][H][W][C] into channels [c_off, c_off + C) of a
 // [2D][2H][2W][c_total] tensor (the concatenation with a skip connection)
+template <int V>
 __global__ void k_up2(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ y, int D, int H, int W, int C,
                       int c_total, int c_off) {
-    const int64_t n = (int64_t) 8 * D * H * W * C;
+    const int64_t n = (int64_t) 8 * D * H * W * (C / V);
     NN_LOOP(n) {
-        const int c = (int) (q % C);
-        int64_t v = q / C;
+        const int c = (int) (q % (C / V)) * V;
+        int64_t v = q / (C / V);
         const int xf = (int) (v % (2 * W)); v /= (2 * W);
         const int yf = (int) (v % (2 * H));
         const int zf = (int) (v / (2 * H));
-        y[(((int64_t) zf * 2 * H + yf) * 2 * W + xf) * c_total + c_off + c] =
-            x[(((int64_t) (zf / 2) * H + yf / 2) * W + xf / 2) * C + c];
+        ch_store<V>(y + (((int64_t) zf * 2 * H + yf) * 2 * W + xf) * c_total + c_off + c,
+                    ch_load<V>(x + (((int64_t) (zf / 2) * H + yf / 2) * W + xf / 2) * C + c));
     }
 }
 
 // backward of k_up2: dx = sum of the 8 children's gradients
+template <int V>
 __global__ void k_up2_bwd(const __nv_bfloat16 *__restrict__ dy, __nv_bfloat16 *__restrict__ dx, int D, int H, int W,
                           int C, int c_total, int c_off) {
-    const int64_t n = (int64_t) D * H * W * C;
+    const int64_t n = (int64_t) D * H * W * (C / V);
     NN_LOOP(n) {
-        const int c = (int) (q % C);
-        int64_t v = q / C;
+        const int c = (int) (q % (C / V)) * V;
+        int64_t v = q / (C / V);
         const int x = (int) (v % W); v /= W;
         const int y = (int) (v % H);
         const int z = (int) (v / H);
-        float s = 0.f;
+        Ch<V> s{};
 #pragma unroll
-        for (int o = 0; o < 8; o++)
-            s += bf(dy[(((int64_t) (2 * z + (o >> 2)) * 2 * H + 2 * y + ((o >> 1) & 1)) * 2 * W + 2 * x + (o & 1)) * c_total +
-                       c_off + c]);
-        dx[q] = __float2bfloat16_rn(s);
+        for (int o = 0; o < 8; o++) {
+            const Ch<V> e = ch_load<V>(
+                dy + (((int64_t) (2 * z + (o >> 2)) * 2 * H + 2 * y + ((o >> 1) & 1)) * 2 * W + 2 * x + (o & 1)) * c_total +
+                c_off + c);
+#pragma unroll
+            for (int i = 0; i < V; i++) s.v[i] += e.v[i];
+        }
+        ch_store<V>(dx + q * V, s);
     }
 }
 
 // copy channels: dst[v][d_off + c] = src[v][s_off + c], c < C (concat / split)
+template <int V>
 __global__ void k_copy_channels(const __nv_bfloat16 *__restrict__ src, int s_total, int s_off,
                                 __nv_bfloat16 *__restrict__ dst, int d_total, int d_off, int C, int64_t voxels,
                                 int accumulate) {
-    const int64_t n = voxels * C;
+    const int64_t n = voxels * (C / V);
     NN_LOOP(n) {
-        const int c = (int) (q % C);
-        const int64_t v = q / C;
-        const __nv_bfloat16 s = src[v * s_total + s_off + c];
-        __nv_bfloat16 &d = dst[v * d_total + d_off + c];
-        d = accumulate ? __float2bfloat16_rn(bf(d) + bf(s)) : s;
+        const int c = (int) (q % (C / V)) * V;
+        const int64_t v = q / (C / V);
+        Ch<V> s = ch_load<V>(src + v * s_total + s_off + c);
+        __nv_bfloat16 *d = dst + v * d_total + d_off + c;
+        if (accumulate) {
+            const Ch<V> o = ch_load<V>(d);
+#pragma unroll
+            for (int i = 0; i < V; i++) s.v[i] = o.v[i] + s.v[i];
+        }
+        ch_store<V>(d, s);
     }
 }
 
-// db[c] += sum_v dy[v][c]
+// db[c] += sum_v dy[v][c]: a thread sums V channels of every (threads V / C)-th
+// voxel, the block adds its threads' sums of a channel in shared memory, one
+// atomic per block and channel (one block per channel and 2-byte accesses read
+// every sector C times before)
+template <int V>
 __global__ void k_bias_grad(const __nv_bfloat16 *__restrict__ dy, float *__restrict__ db, int64_t voxels, int C) {
-    // one block per channel slice: threads stride over voxels
+    extern __shared__ float sum[];  // [C]
+    const int per = C / V;                       // threads of a voxel
+    const int rows = (int) blockDim.x / per;     // voxels of a block's step
+    for (int c = (int) threadIdx.x; c < C; c += (int) blockDim.x) sum[c] = 0.f;
+    __syncthreads();
+    const int row = (int) threadIdx.x / per, c = ((int) threadIdx.x % per) * V;
+    if (row < rows) {
+        Ch<V> s{};
+        for (int64_t v = blockIdx.x * (int64_t) rows + row; v < voxels; v += (int64_t) gridDim.x * rows) {
+            const Ch<V> e = ch_load<V>(dy + v * C + c);
+#pragma unroll
+            for (int i = 0; i < V; i++) s.v[i] += e.v[i];
+        }
+#pragma unroll
+        for (int i = 0; i < V; i++) atomicAdd(sum + c + i, s.v[i]);
+    }
+    __syncthreads();
+    for (int k = (int) threadIdx.x; k < C; k += (int) blockDim.x) atomicAdd(db + k, sum[k]);
+}
+
+// the same for more channels than a block has threads: a block per channel
+__global__ void k_bias_grad_any(const __nv_bfloat16 *__restrict__ dy, float *__restrict__ db, int64_t voxels, int C) {
     for (int c = blockIdx.y; c < C; c += gridDim.y) {
         float s = 0.f;
         for (int64_t v = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; v < voxels; v += (int64_t) gridDim.x * blockDim.x)
@@ -210,6 +308,7 @@ __global__ void k_nn_target(const double *__restrict__ p_star, const double *__r
 
 // loss 0.5 * sum over inner cells (y[v][0] - t[v])^2 and its gradient into
 // channel 0 of dy (other channels zero); block partials of the loss
+template <int V>
 __global__ void k_mse(const __nv_bfloat16 *__restrict__ y, int C, const float *__restrict__ t,
                       const __nv_bfloat16 *__restrict__ mask_in, __nv_bfloat16 *__restrict__ dy, int64_t voxels,
                       float inv_n, float *__restrict__ partials) {
@@ -219,8 +318,17 @@ __global__ void k_mse(const __nv_bfloat16 *__restrict__ y, int C, const float *_
         const bool in = bf(mask_in[q * C + 1]) > 0.5f;
         const float d = in ? bf(y[q * C]) - t[q] : 0.f;
         acc += 0.5f * d * d;
-        dy[q * C] = __float2bfloat16_rn(d * inv_n);
-        for (int c = 1; c < C; c++) dy[q * C + c] = __float2bfloat16_rn(0.f);
+        if constexpr (V == 8) {
+            Ch<8> g{};
+            g.v[0] = d * inv_n;
+            for (int c = 0; c < C; c += 8) {
+                ch_store<8>(dy + q * C + c, g);
+                g.v[0] = 0.f;
+            }
+        } else {
+            dy[q * C] = __float2bfloat16_rn(d * inv_n);
+            for (int c = 1; c < C; c++) dy[q * C + c] = __float2bfloat16_rn(0.f);
+        }
     }
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = acc;
@@ -238,6 +346,12 @@ __global__ void k_mse(const __nv_bfloat16 *__restrict__ y, int C, const float *_
 using namespace artss;
 
 #define NN_CK(ctx) ARTSS_LAUNCH_CK(ctx)
+// kernel K<8> over n / 8 threads where `wide`, else K<1> over n
+#define NN_LAUNCH(wide, K, n, ...)                                                                       \
+    do {                                                                                                 \
+        if (wide) ARTSS_LAUNCH(ctx, FAM_NN, K<8><<<nblk((n) / 8), 256, 0, ctx->stream>>>(__VA_ARGS__));  \
+        else ARTSS_LAUNCH(ctx, FAM_NN, K<1><<<nblk(n), 256, 0, ctx->stream>>>(__VA_ARGS__));             \
+    } while (0)
 #define NN_ARGS_OK(...) do { if (!(__VA_ARGS__)) { set_error("invalid argument"); return ARTSS_ERR_ARG; } } while (0)
 
 extern "C" {
@@ -250,7 +364,7 @@ int artss_nn_zero(artss_ctx *ctx, void *p, int64_t bytes) {
 
 int artss_nn_relu_bwd(artss_ctx *ctx, void *dy, const void *y, int64_t n) {
     NN_ARGS_OK(ctx && dy && y && n >= 0);
-    ARTSS_LAUNCH(ctx, FAM_NN, k_relu_bwd<<<nblk(n), 256, 0, ctx->stream>>>((__nv_bfloat16 *) dy, (const __nv_bfloat16 *) y, n));
+    NN_LAUNCH(n % 8 == 0 && vec8({dy, y}, {}), k_relu_bwd, n, (__nv_bfloat16 *) dy, (const __nv_bfloat16 *) y, n);
     NN_CK(ctx);
     return ARTSS_OK;
 }
@@ -259,9 +373,9 @@ int artss_nn_pool2(artss_ctx *ctx, const void *x, void *y, int D, int H, int W, 
     NN_ARGS_OK(ctx && x && y && D % 2 == 0 && H % 2 == 0 && W % 2 == 0 && C > 0);
     const int64_t n = backward ? (int64_t) D * H * W * C : (int64_t) D * H * W * C / 8;
     if (backward)
-        ARTSS_LAUNCH(ctx, FAM_NN, k_pool2_bwd<<<nblk(n), 256, 0, ctx->stream>>>((const __nv_bfloat16 *) x, (__nv_bfloat16 *) y, D, H, W, C));
+        NN_LAUNCH(vec8({x, y}, {C}), k_pool2_bwd, n, (const __nv_bfloat16 *) x, (__nv_bfloat16 *) y, D, H, W, C);
     else
-        ARTSS_LAUNCH(ctx, FAM_NN, k_pool2<<<nblk(n), 256, 0, ctx->stream>>>((const __nv_bfloat16 *) x, (__nv_bfloat16 *) y, D, H, W, C));
+        NN_LAUNCH(vec8({x, y}, {C}), k_pool2, n, (const __nv_bfloat16 *) x, (__nv_bfloat16 *) y, D, H, W, C);
     NN_CK(ctx);
     return ARTSS_OK;
 }
@@ -269,12 +383,12 @@ int artss_nn_pool2(artss_ctx *ctx, const void *x, void *y, int D, int H, int W, 
 int artss_nn_up2(artss_ctx *ctx, const void *x, void *y, int D, int H, int W, int C, int c_total, int c_off,
                  int backward) {
     NN_ARGS_OK(ctx && x && y && C > 0 && c_off >= 0 && c_off + C <= c_total);
+    const bool wide = vec8({x, y}, {C, c_total, c_off});
+    const int64_t n = (int64_t) D * H * W * C;
     if (backward)
-        ARTSS_LAUNCH(ctx, FAM_NN, k_up2_bwd<<<nblk((int64_t) D * H * W * C), 256, 0, ctx->stream>>>(
-                                     (const __nv_bfloat16 *) x, (__nv_bfloat16 *) y, D, H, W, C, c_total, c_off));
+        NN_LAUNCH(wide, k_up2_bwd, n, (const __nv_bfloat16 *) x, (__nv_bfloat16 *) y, D, H, W, C, c_total, c_off);
     else
-        ARTSS_LAUNCH(ctx, FAM_NN, k_up2<<<nblk((int64_t) 8 * D * H * W * C), 256, 0, ctx->stream>>>(
-                                     (const __nv_bfloat16 *) x, (__nv_bfloat16 *) y, D, H, W, C, c_total, c_off));
+        NN_LAUNCH(wide, k_up2, 8 * n, (const __nv_bfloat16 *) x, (__nv_bfloat16 *) y, D, H, W, C, c_total, c_off);
     NN_CK(ctx);
     return ARTSS_OK;
 }
@@ -282,17 +396,26 @@ int artss_nn_up2(artss_ctx *ctx, const void *x, void *y, int D, int H, int W, in
 int artss_nn_copy_channels(artss_ctx *ctx, const void *src, int s_total, int s_off, void *dst, int d_total, int d_off,
                            int C, int64_t voxels, int accumulate) {
     NN_ARGS_OK(ctx && src && dst && C > 0 && s_off + C <= s_total && d_off + C <= d_total && voxels >= 0);
-    ARTSS_LAUNCH(ctx, FAM_NN, k_copy_channels<<<nblk(voxels * C), 256, 0, ctx->stream>>>(
-                                 (const __nv_bfloat16 *) src, s_total, s_off, (__nv_bfloat16 *) dst, d_total, d_off, C,
-                                 voxels, accumulate));
+    NN_LAUNCH(vec8({src, dst}, {C, s_total, s_off, d_total, d_off}), k_copy_channels, voxels * C,
+              (const __nv_bfloat16 *) src, s_total, s_off, (__nv_bfloat16 *) dst, d_total, d_off, C, voxels, accumulate);
     NN_CK(ctx);
     return ARTSS_OK;
 }
 
 int artss_nn_bias_grad(artss_ctx *ctx, const void *dy, float *db, int64_t voxels, int C) {
     NN_ARGS_OK(ctx && dy && db && C > 0);
-    const dim3 g((unsigned) std::min<int64_t>(512, (voxels + 255) / 256 + 1), (unsigned) C);
-    ARTSS_LAUNCH(ctx, FAM_NN, k_bias_grad<<<g, 256, 0, ctx->stream>>>((const __nv_bfloat16 *) dy, db, voxels, C));
+    // a voxel's threads sit in one block
+    const bool wide = vec8({dy}, {C}) && C <= 2048;
+    const int per = wide ? C / 8 : C;
+    if (per <= 256) {
+        const unsigned g = nblk(voxels * per / 8);  // some 8 voxels a thread
+        const unsigned blocks = std::min<unsigned>(g, (unsigned) (4 * std::max(ctx->sm_count, 1)));
+        if (wide) ARTSS_LAUNCH(ctx, FAM_NN, k_bias_grad<8><<<blocks, 256, C * sizeof(float), ctx->stream>>>((const __nv_bfloat16 *) dy, db, voxels, C));
+        else ARTSS_LAUNCH(ctx, FAM_NN, k_bias_grad<1><<<blocks, 256, C * sizeof(float), ctx->stream>>>((const __nv_bfloat16 *) dy, db, voxels, C));
+    } else {
+        const dim3 g((unsigned) std::min<int64_t>(512, (voxels + 255) / 256 + 1), (unsigned) C);
+        ARTSS_LAUNCH(ctx, FAM_NN, k_bias_grad_any<<<g, 256, 0, ctx->stream>>>((const __nv_bfloat16 *) dy, db, voxels, C));
+    }
     NN_CK(ctx);
     return ARTSS_OK;
 }
@@ -358,9 +481,14 @@ int artss_nn_target(artss_ctx *ctx, int level, const double *p_star, const doubl
 int artss_nn_mse(artss_ctx *ctx, const void *y, int C, const float *target, const void *inputs, void *dy,
                  int64_t voxels, float inv_n, float *partials, int n_partials) {
     NN_ARGS_OK(ctx && y && target && inputs && dy && partials && n_partials >= 1);
-    ARTSS_LAUNCH(ctx, FAM_NN, k_mse<<<(unsigned) n_partials, 256, 0, ctx->stream>>>(
-                                 (const __nv_bfloat16 *) y, C, target, (const __nv_bfloat16 *) inputs,
-                                 (__nv_bfloat16 *) dy, voxels, inv_n, partials));
+    if (vec8({dy}, {C}))
+        ARTSS_LAUNCH(ctx, FAM_NN, k_mse<8><<<(unsigned) n_partials, 256, 0, ctx->stream>>>(
+                                     (const __nv_bfloat16 *) y, C, target, (const __nv_bfloat16 *) inputs,
+                                     (__nv_bfloat16 *) dy, voxels, inv_n, partials));
+    else
+        ARTSS_LAUNCH(ctx, FAM_NN, k_mse<1><<<(unsigned) n_partials, 256, 0, ctx->stream>>>(
+                                     (const __nv_bfloat16 *) y, C, target, (const __nv_bfloat16 *) inputs,
+                                     (__nv_bfloat16 *) dy, voxels, inv_n, partials));
     NN_CK(ctx);
     return ARTSS_OK;
 }
