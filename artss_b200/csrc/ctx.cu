@@ -280,6 +280,8 @@ int artss_ctx_destroy(artss_ctx *ctx) {
         for (int t = 0; t < kFieldTypes; t++) {
             BcProgram &p = ctx->bc[l][t];
             cudaFree(p.d_target); cudaFree(p.d_root); cudaFree(p.d_depth); cudaFree(p.d_neg); cudaFree(p.d_value);
+            BcProgram::Flat &x = p.flat;
+            cudaFree(x.d_target); cudaFree(x.d_root); cudaFree(x.d_depth); cudaFree(x.d_neg); cudaFree(x.d_value);
         }
     }
     for (uint8_t *t : ctx->d_sweep3_obst) if (t) cudaFree(t);

@@ -24,6 +24,8 @@ constexpr int kFieldTypes = ARTSS_NUM_FIELD_TYPES;
 constexpr int kCopySlots = 8;           // uploads on the copy stream waited for by slot
 constexpr int kParams = 16;             // parameter slots of captured steps
 constexpr int kBcMaxDepth = 4;          // boundary assignments folded per thread
+constexpr int64_t kBcMaxHazards = 4096; // of a flat program, staged in one block's shared memory
+constexpr uint8_t kBcLagged = 0x80;     // flat program: the root is itself a target
 constexpr int kReduceThreads = 256;
 constexpr int kMaxPartials = 1 << 16;   // per-block partial sums of up to two reduction passes
 constexpr int kNnErrSlot = 15;          // loop slot whose error flag the network kernels raise
@@ -55,6 +57,19 @@ struct BcProgram {
     std::vector<int64_t> h_root;       // roots, host copy
     std::vector<int8_t> h_sign;        // sign of x_t = +-x_r with every value zero, host copy
     bool zero_values = false;          // every value of the program is +0.0: x_t = +-x_r + 0
+    // A program of several waves folded onto the values from before it: one
+    // assignment per target, its root a cell's value before the program.  The
+    // first `hazards` ones read a cell that another one writes or write one that
+    // is read; depth bit 7: the root is a target.  n = 0: not folded (a chain is
+    // longer than kBcMaxDepth, or too many hazards for one block)
+    struct Flat {
+        int64_t n = 0, hazards = 0;
+        int64_t *d_target = nullptr, *d_root = nullptr;
+        uint8_t *d_depth = nullptr, *d_neg = nullptr;
+        double *d_value = nullptr;         // [kBcMaxDepth][n]
+        std::vector<int64_t> h_target, h_root;
+        std::vector<uint8_t> h_depth;
+    } flat;
     // plan of the pipelined coarse solve: state -2 unknown, -1 not eligible, 1 planned
     int pipe_state = -2;
     std::vector<int> pipe_kb;          // plane split, ranks + 1 entries

@@ -838,8 +838,7 @@ k_mg_coarse_block(TS *__restrict__ out, TS *__restrict__ tmp, const TS *__restri
 //
 // VCycleMG::call_solve_jacobi (src/pressure/VCycleMG.cpp:725-798) on the
 // cluster with every access to the rank's own shared memory and one cluster
-// barrier per sweep, for boundary programs of a single wave (every
-// configuration of the reference's tests):
+// barrier per sweep, for boundary programs of a single wave or flat ones:
 //  * rank r owns the z-planes [kb[r], kb[r+1]) of a split chosen on the host
 //    so that no boundary assignment with an inner root crosses a rank; it
 //    keeps them plus one halo plane on each side, in three buffers of the
@@ -852,7 +851,10 @@ k_mg_coarse_block(TS *__restrict__ out, TS *__restrict__ tmp, const TS *__restri
 //    root is ever a target, so a root is either an inner cell, and the thread
 //    that computes the root's new value also evaluates the target's chain
 //    from it (a per-thread target list built at launch), or a cell that
-//    nothing writes, whose targets are set once before the loop;
+//    nothing writes, whose targets are set once before the loop; a flat program's
+//    root may also be a target, and stands for that cell's value before the
+//    program, which in the reference's array is the value of two sweeps ago (the
+//    arrays swap): it is read from the buffer of iterate k-2, complete by then;
 //  * the residual of iterate k-1 is summed in the pass that computes iterate
 //    k (both read only iterate k-1), so the loop decision for k arrives one
 //    sweep late.  Three buffers keep iterates k-2, k-1 and k apart and the
@@ -867,7 +869,7 @@ struct HaloTarget {
     double val[kBcMaxDepth];
     uint32_t dst, root;
     uint32_t depth_neg;  // depth | neg << 8
-    uint32_t pad;
+    uint32_t lagged;     // the root is a target: its value is iterate k-2's
 };
 
 // ranks of the pipelined coarse solve: up to 16 CTAs (a non-portable cluster size)
@@ -975,18 +977,20 @@ k_mg_coarse_jacobi_pipe(TS *__restrict__ out, TS *__restrict__ tmp, const TS *__
         const bool own_t = kt >= kb0 && kt < kb1, own_r = kr >= kb0 && kr < kb1;
         const bool halo_t = kt == kb0 - 1 || kt == kb1, halo_r = kr == kb0 - 1 || kr == kb1;
         if (!own_t && !own_r) continue;
-        const int d = __ldg(bc.depth + qq);
+        const int d = __ldg(bc.depth + qq) & ~kBcLagged;
+        const bool lagged = (__ldg(bc.depth + qq) & kBcLagged) != 0;
         const uint8_t mneg = __ldg(bc.neg + qq);
         if (own_t) {
-            double x = X[(kr - kb0 + 1) * nk + (r - kr * nk)];
+            double x = (double) out[r];  // from before the program, also where X holds a target of it
 #pragma unroll
             for (int s = 0; s < kBcMaxDepth; s++)
                 if (s < d) x = ((mneg >> s) & 1 ? -x : x) + (bc.value ? __ldg(bc.value + s * bc.n + qq) : 0.0);
             X[(kt - kb0 + 1) * nk + (t - kt * nk)] = x;
         }
-        if (!(__ldg(flags + r) & kInner)) continue;  // constant root: set once above
+        if (!(__ldg(flags + r) & kInner) && !lagged) continue;  // constant root: set once above
+        if (lagged && !own_t) continue;  // the rank of the target evaluates it
         HaloTarget *h = nullptr;
-        if (own_t && own_r) {
+        if (own_t && (own_r || (lagged && halo_r))) {
             const int slot = atomicAdd(&s_nt, 1);
             if (slot < target_cap) h = &tg[slot];
         } else if ((own_t && halo_r) || (own_r && halo_t)) {
@@ -1002,7 +1006,7 @@ k_mg_coarse_jacobi_pipe(TS *__restrict__ out, TS *__restrict__ tmp, const TS *__
         h->dst = (uint32_t) ((kt - kb0 + 1) * nk + (t - kt * nk));
         h->root = (uint32_t) ((kr - kb0 + 1) * nk + (r - kr * nk));
         h->depth_neg = (uint32_t) d | (uint32_t) mneg << 8;
-        h->pad = 0;
+        h->lagged = lagged ? 1u : 0u;
     }
     __syncthreads();
     const int nt = min(s_nt, target_cap), nf = min(s_nf, fix_cap);
@@ -1063,6 +1067,7 @@ k_mg_coarse_jacobi_pipe(TS *__restrict__ out, TS *__restrict__ tmp, const TS *__
         for (long long k = 1;; k++, sp_ = sn, sn = sn == 2 ? 0 : sn + 1) {
             const double *P = X + sp_ * bstride;
             double *N = X + sn * bstride;
+            const double *Q = X + (3 - sp_ - sn) * bstride;  // iterate k-2 (0 for k = 1)
             const bool sweep = k - 1 < max_it, resid = k >= 2 || rel;
             if (unwaited) {
                 // halos of iterate k-1 (sent in phase k-1) must have landed
@@ -1124,7 +1129,7 @@ k_mg_coarse_jacobi_pipe(TS *__restrict__ out, TS *__restrict__ tmp, const TS *__
                 reduced = resid;
                 for (int t = tid; t < nt; t += kClusterThreads) {
                     const HaloTarget &h = tg[t];
-                    double x = N[h.root];
+                    double x = (h.lagged ? Q : N)[h.root];
                     const int d = (int) (h.depth_neg & 0xffu);
                     const uint32_t mneg = h.depth_neg >> 8;
 #pragma unroll
@@ -1235,9 +1240,9 @@ bool cluster_fits(const artss_ctx *ctx, int level, int buffers, int *plane_cap, 
 }
 
 // Launch data of k_mg_coarse_jacobi_pipe for the level, or false when its
-// pressure boundary program does not qualify (more than one wave, an inner
-// target, a chain leaving its target's neighbouring planes, no plane split
-// that keeps every inner root with its target) or the level does not fit.
+// pressure boundary program does not qualify (several waves and no flat form, an
+// inner target, no plane split that keeps chains over more than neighbouring planes
+// and every inner root with its target) or the level does not fit.
 // The split cuts the planes as evenly as the forbidden cuts allow.
 struct PipeLaunch {
     PlaneSplit split;
@@ -1278,16 +1283,21 @@ bool coarse_pipe_plan_new(artss_ctx *ctx, int level, PipeLaunch *pl) {
     const std::vector<bool> &in = ctx->h_inner[level];
     const int nz = (int) L.Nz;
     if (cluster_ranks(L) < 2 || L.nxy() % 2 || in.empty() || (int64_t) in.size() != L.size()) return false;
-    if (p.present && p.waves > 1) return false;
+    const bool flat = p.flat.n > 0;
+    if (p.present && p.waves > 1 && !flat) return false;
+    const std::vector<int64_t> &ht = flat ? p.flat.h_target : p.h_target, &hr = flat ? p.flat.h_root : p.h_root;
     // forbidden[c]: no rank boundary between planes c-1 and c; the ghost planes
     // stay with their neighbour (a rank of a ghost plane alone has no cells)
     std::vector<char> forbidden(nz + 1, 0);
     forbidden[1] = forbidden[nz - 1] = 1;
-    const int64_t n = p.present ? p.n : 0;
+    const int64_t n = !p.present ? 0 : flat ? p.flat.n : p.n;
     for (int64_t q = 0; q < n; q++) {
-        const int64_t t = p.h_target[q], r = p.h_root[q];
+        const int64_t t = ht[q], r = hr[q];
         const int kt = (int) (t / L.nxy()), kr = (int) (r / L.nxy());
-        if (in[(size_t) t] || kr < kt - 1 || kr > kt + 1) return false;
+        if (in[(size_t) t]) return false;
+        // a chain that spans more than neighbouring planes stays within one rank
+        if (kr < kt - 1 || kr > kt + 1)
+            for (int c = std::min(kr, kt) + 1; c <= std::max(kr, kt); c++) forbidden[c] = 1;
     }
     static bool attr_set = false;
     if (!attr_set) {
@@ -1325,9 +1335,14 @@ bool coarse_pipe_plan_new(artss_ctx *ctx, int level, PipeLaunch *pl) {
             if (z1 >= z0 && (z1 - z0 + 1) * nxy_in > (int64_t) kClusterThreads * kPipeCells) ok = false;
             int nt = 0, nf = 0;
             for (int64_t q = 0; q < n; q++) {
-                if (!in[(size_t) p.h_root[q]]) continue;
-                const int kt = (int) (p.h_target[q] / L.nxy()), kr = (int) (p.h_root[q] / L.nxy());
+                const bool lagged = flat && (p.flat.h_depth[(size_t) q] & kBcLagged);
+                if (!in[(size_t) hr[q]] && !lagged) continue;
+                const int kt = (int) (ht[q] / L.nxy()), kr = (int) (hr[q] / L.nxy());
                 const bool own_t = kt >= a && kt < e, own_r = kr >= a && kr < e;
+                if (lagged) {
+                    if (own_t) nt++;
+                    continue;
+                }
                 if (own_t && own_r) nt++;
                 else if ((own_t && (kr == a - 1 || kr == e)) || (own_r && (kt == a - 1 || kt == e))) nf++;
                 // a rank of one plane sends its plane both ways before such a
@@ -1438,6 +1453,16 @@ BcView bc_view(const artss_ctx *ctx, int level) {
     return v;
 }
 
+// the program as the pipelined coarse solve takes it: the flat form where it has one
+BcView pipe_view(const artss_ctx *ctx, int level) {
+    const BcProgram &p = ctx->bc[level][ARTSS_FIELD_P];
+    const BcProgram::Flat &x = p.flat;
+    if (!p.present || !x.n) return bc_view(ctx, level);
+    BcView v{x.d_target, x.d_root, x.d_depth, x.d_neg, x.d_value, x.n, 1, {}};
+    v.begin[1] = x.n;
+    return v;
+}
+
 // out = 0 (the coarse solve's start on the cluster path)
 __global__ void k_fill_f32(float *__restrict__ f, int64_t n, const LoopState *__restrict__ pred) {
     pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
@@ -1530,9 +1555,12 @@ int coarse_cluster_f32(artss_ctx *ctx, float *out, const float *b, int level, in
     if (cgs)
         return launch_coarse_cluster<true, float>(ctx, out, nullptr, b, level, c, c.ax, c.ay, c.az, v, tol, 1, max_it,
                                                   cap, smem, nullptr, pred);
-    if (pipe)
+    if (pipe) {
+        v = pipe_view(ctx, level);
+        v.value = nullptr;
         return launch_coarse_pipe<float>(ctx, out, nullptr, b, level, c, c.ax, c.ay, c.az, v, tol, 1, max_it, pl, nullptr,
                                          pred);
+    }
     return launch_coarse_cluster<false, float>(ctx, out, nullptr, b, level, c, c.ax, c.ay, c.az, v, tol, 1, max_it, cap,
                                                smem, nullptr, pred);
 }
@@ -1565,8 +1593,8 @@ int mg_coarse_solve(artss_mg *mg, double *out, double *tmp, const double *b, int
     int64_t csmem = 0;
     PipeLaunch pl{};
     if (mg->cluster_coarse && !cgs && mg->pipelined_coarse && coarse_pipe_plan(ctx, level, &pl))
-        return launch_coarse_pipe<double>(ctx, out, tmp, b, level, c, rx, ry, rz, v, tol, 0, mi, pl, ctx->d_loop + 1,
-                                          nullptr);
+        return launch_coarse_pipe<double>(ctx, out, tmp, b, level, c, rx, ry, rz, pipe_view(ctx, level), tol, 0, mi, pl,
+                                          ctx->d_loop + 1, nullptr);
     if (mg->cluster_coarse && cluster_fits(ctx, level, cgs ? 1 : 2, &cap, &csmem)) {
         if (cgs)
             return launch_coarse_cluster<true, double>(ctx, out, tmp, b, level, c, rx, ry, rz, v, tol, 0, mi, cap, csmem,
