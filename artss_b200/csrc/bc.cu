@@ -420,6 +420,15 @@ int artss_set_boundary_program(artss_ctx *ctx, int level, int field_type, const 
         std::memcpy(&bits, &v, sizeof bits);
         if (bits != 0) p.zero_values = false;
     }
+    p.homogeneous = waves <= 1;
+    for (int64_t q = 0; q < n && p.homogeneous; q++) {
+        // the steps x -> +-x + z from the last one back: x + (-0) is x; the step before
+        // them adds +0, or there is none
+        int d = folded[q].depth;
+        for (int s = 0; s < d; s++) p.homogeneous = p.homogeneous && folded[q].value[s] == 0.0;
+        while (d > 0 && std::signbit(folded[q].value[d - 1]) && !(folded[q].neg >> (d - 1) & 1)) d--;
+        if (d > 0 && std::signbit(folded[q].value[d - 1])) p.homogeneous = false;
+    }
     if (n == 0) return ARTSS_OK;
     ARTSS_CK(cudaMalloc(&p.d_target, n * sizeof(int64_t)));
     ARTSS_CK(cudaMalloc(&p.d_root, n * sizeof(int64_t)));

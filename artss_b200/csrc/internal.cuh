@@ -57,6 +57,9 @@ struct BcProgram {
     std::vector<int64_t> h_root;       // roots, host copy
     std::vector<int8_t> h_sign;        // sign of x_t = +-x_r with every value zero, host copy
     bool zero_values = false;          // every value of the program is +0.0: x_t = +-x_r + 0
+    // no lagged reads (one wave), every value a zero, and every assignment x_t = +-x_r
+    // + 0 or x_t = x_r: zeros satisfy it and so do sums of arrays that do, bit for bit
+    bool homogeneous = false;
     // A program of several waves folded onto the values from before it: one
     // assignment per target, its root a cell's value before the program.  The
     // first `hazards` ones read a cell that another one writes or write one that
@@ -380,7 +383,7 @@ inline dim3 col_grid(const Box3 &b, const ColShape &s) {
 // Kernel ids of the launch-shape tuner (TuneKey::kernel; 0 is the sweep variant)
 enum ColKernel : int {
     kTuneAdvect1 = 101, kTuneAdvect3, kTuneSmagorinsky, kTuneDivergence, kTuneProjection, kTuneBuoyancy,
-    kTuneMgJacobi, kTuneMgResiduum, kTuneMgRestrict, kTuneMgProlongate,
+    kTuneMgJacobi, kTuneMgResiduum, kTuneMgRestrict, kTuneMgProlongate, kTuneMgJacobi0, kTuneMgDown,
     kTuneMxJacobi0, kTuneMxJacobi, kTuneMxResiduum, kTuneMxRestrict
 };
 
