@@ -1895,8 +1895,9 @@ int mg_prolongate_add(artss_mg *mg, double *fine, const double *coarse, int coar
 // the coarse cells) take the short way, with the same values: smoothing between two
 // arrays instead of after a copy, residual and restriction in one pass, correction
 // added where it is prolongated, no array of zeros filled and read, nothing formed
-// on the coarsest level.  At 256 x 128 x 128 with 4 levels a cycle is 30 launches
-// instead of 52 and moves 0.45 instead of 0.75 GB.
+// on the coarsest level.  At 256 x 128 x 128 with 4 levels a cycle is 24 launches
+// instead of 54 and moves 0.38 instead of 0.70 GB; the two of a later-step call
+// take 354 instead of 477 us (three calls in turn).
 int mg_vcycle(artss_mg *mg, double *out, int64_t *coarse_its, const double *b0 = nullptr, bool satisfied = false) {
     artss_ctx *ctx = mg->ctx;
     const int L = mg->L;
