@@ -28,123 +28,176 @@
 
 namespace artss {
 
-__global__ void k_bc_wave(double *__restrict__ f, const int64_t *__restrict__ target,
-                          const int64_t *__restrict__ root, const uint8_t *__restrict__ depth,
-                          const uint8_t *__restrict__ neg, const double *__restrict__ value,
-                          int64_t begin, int64_t end, int64_t n_total, const LoopState *__restrict__ pred) {
+// A program as the kernels take it: assignments [begin, end) of a wave, or a flat
+// program with its hazards first.
+struct BcRun {
+    double *f;
+    const int64_t *target, *root;
+    const uint8_t *depth, *neg;
+    const double *value;
+    int64_t begin, end, n;  // n: stride of value
+    int64_t hazards;        // flat programs: the first block's share, staged in shared memory
+};
+
+// loop step of the last block of a launch; partials = nullptr: none
+struct BcStep {
+    const double *partials;
+    int nblocks;
+    const LoopState *rd;
+    LoopState *wr;
+    double tol;
+    long long max_it;
+};
+
+// block `block` of `blocks` of a program
+__device__ __forceinline__ void bc_blocks(const BcRun &p, int block, int blocks, const LoopState *pred, double *staged) {
+    // FLAT: its values depend on cells from before the program only, so the
+    // assignments may run in any order as long as every read of a cell comes before its
+    // write: block 0 reads for all hazards, then writes them; the other blocks'
+    // assignments touch no cell that another one touches
+    const bool first = p.hazards > 0 && block == 0;
+    const int64_t end = first ? p.hazards : p.end;
+    int64_t q = (first ? 0 : p.begin + p.hazards) + threadIdx.x;
+    int64_t stride = blockDim.x;
+    if (!first) {
+        const int skip = p.hazards > 0 ? 1 : 0;
+        q += (int64_t) (block - skip) * blockDim.x;
+        stride *= blocks - skip;
+    }
     // the program's tables are constant: the first assignment's entries are
     // read before waiting for the kernel that wrote f
-    const int64_t stride = (int64_t) gridDim.x * blockDim.x;
-    int64_t q = begin + blockIdx.x * (int64_t) blockDim.x + threadIdx.x;
-    int64_t t = 0, r = 0;
-    int d = 0;
-    uint8_t m = 0;
-    double val[kBcMaxDepth];
-    if (q < end) {
-        t = target[q];
-        r = root[q];
-        d = depth[q];
-        m = neg[q];
-    }
-#pragma unroll
-    for (int s = 0; s < kBcMaxDepth; s++) val[s] = (q < end && s < d) ? value[s * n_total + q] : 0.0;
-    pdl_wait();
-    pdl_trigger();
-    if (pred && !pred->cond) return;
-    while (q < end) {
-        double x = f[r];
-#pragma unroll
-        for (int s = 0; s < kBcMaxDepth; s++) {
-            if (s < d) x = ((m >> s) & 1 ? -x : x) + val[s];
-        }
-        f[t] = x;
-        q += stride;
-        if (q >= end) break;
-        t = target[q];
-        r = root[q];
-        d = depth[q];
-        m = neg[q];
-#pragma unroll
-        for (int s = 0; s < kBcMaxDepth; s++) val[s] = s < d ? value[s * n_total + q] : 0.0;
-    }
-}
-
-// A flat program in one launch.  Its values depend on cells from before the
-// program only, so the assignments may run in any order as long as every read of
-// a cell comes before its write: block 0 reads for all hazards, then writes them;
-// the other blocks' assignments touch no cell that another one touches.  On the
-// room with a door (32^3, seven touching walls, 10952 assignments in three waves of
-// 10836, 114 and 2) one launch instead of three, 171 -> 57 in a step.
-__global__ void k_bc_flat(double *__restrict__ f, const int64_t *__restrict__ target,
-                          const int64_t *__restrict__ root, const uint8_t *__restrict__ depth,
-                          const uint8_t *__restrict__ neg, const double *__restrict__ value, int64_t hazards,
-                          int64_t n, const LoopState *__restrict__ pred) {
-    extern __shared__ double staged[];  // [hazards]
-    const bool first = blockIdx.x == 0;
-    const int64_t begin = first ? 0 : hazards, end = first ? hazards : n;
-    const int64_t stride = first ? blockDim.x : (int64_t) (gridDim.x - 1) * blockDim.x;
-    int64_t q = begin + (first ? 0 : (int64_t) (blockIdx.x - 1) * blockDim.x) + threadIdx.x;
-    // the program's tables are constant: the first assignment's entries are read
-    // before waiting for the kernel that wrote f
     int64_t t = 0, r = 0;
     int d = 0;
     uint8_t m = 0;
     double val[kBcMaxDepth];
     auto entry = [&]() {
         if (q < end) {
-            t = target[q];
-            r = root[q];
-            d = depth[q] & ~kBcLagged;
-            m = neg[q];
+            t = p.target[q];
+            r = p.root[q];
+            d = p.depth[q] & ~kBcLagged;
+            m = p.neg[q];
         }
 #pragma unroll
-        for (int s = 0; s < kBcMaxDepth; s++) val[s] = (q < end && s < d) ? value[s * n + q] : 0.0;
+        for (int s = 0; s < kBcMaxDepth; s++) val[s] = (q < end && s < d) ? p.value[s * p.n + q] : 0.0;
     };
     entry();
     pdl_wait();
     pdl_trigger();
     if (pred && !pred->cond) return;
     while (q < end) {
-        double x = f[r];
+        double x = p.f[r];
 #pragma unroll
         for (int s = 0; s < kBcMaxDepth; s++)
             if (s < d) x = ((m >> s) & 1 ? -x : x) + val[s];
         if (first) staged[q] = x;
-        else f[t] = x;
+        else p.f[t] = x;
         q += stride;
         if (q < end) entry();
     }
     if (first) {
         __syncthreads();
-        for (int64_t h = threadIdx.x; h < hazards; h += blockDim.x) f[target[h]] = staged[h];
+        for (int64_t h = threadIdx.x; h < p.hazards; h += blockDim.x) p.f[p.target[h]] = staged[h];
     }
 }
 
+__global__ void k_bc(BcRun p, BcStep step, const LoopState *__restrict__ pred) {
+    extern __shared__ double staged[];  // [hazards]
+    __shared__ double smem[32];
+    const int blocks = (int) gridDim.x - (step.partials ? 1 : 0);
+    if ((int) blockIdx.x == blocks) {
+        pdl_wait();
+        pdl_trigger();
+        artss_loop_step(step.partials, step.nblocks, step.rd, step.wr, step.tol, step.max_it, smem);
+        return;
+    }
+    bc_blocks(p, (int) blockIdx.x, blocks, pred, staged);
+}
+
+// three programs side by side, a row of blocks each
+__global__ void k_bc3(BcRun a, BcRun b, BcRun c) {
+    extern __shared__ double staged[];
+    bc_blocks(blockIdx.y == 0 ? a : blockIdx.y == 1 ? b : c, (int) blockIdx.x, (int) gridDim.x, nullptr, staged);
+}
+
+namespace {
+
+// the program as one launch, or false (several waves, not folded)
+bool one_run(const BcProgram &p, double *f, BcRun *r) {
+    if (p.flat.n) {
+        const BcProgram::Flat &x = p.flat;
+        *r = BcRun{f, x.d_target, x.d_root, x.d_depth, x.d_neg, x.d_value, 0, x.n, x.n, x.hazards};
+        return true;
+    }
+    if (p.waves > 1) return false;
+    *r = BcRun{f, p.d_target, p.d_root, p.d_depth, p.d_neg, p.d_value, p.wave_begin[0], p.wave_begin[p.waves], p.n, 0};
+    return true;
+}
+unsigned run_blocks(const BcRun &r) {
+    const int64_t rest = r.end - r.begin - r.hazards;
+    return (r.hazards > 0 ? 1u : 0u) + (rest > 0 ? flat_blocks(rest) : 0u);
+}
+
+}  // namespace
+
+// One launch for a program of one wave or a flat one, else one per wave.  On the
+// room with a door (32^3, seven touching walls, 10952 assignments in three waves of
+// 10836, 114 and 2) the flat form takes 57 launches a step instead of 171.
 int apply_bc(artss_ctx *ctx, double *f, int level, int field_type, const LoopState *pred) {
     const BcProgram &p = ctx->bc[level][field_type];
     if (!p.present || p.n == 0) return ARTSS_OK;
-    if (p.flat.n) {
-        const BcProgram::Flat &x = p.flat;
-        const unsigned blocks = 1 + (x.n > x.hazards ? flat_blocks(x.n - x.hazards) : 0);
-        ARTSS_LAUNCH_PDL(ctx, FAM_BC, k_bc_flat, blocks, 256, x.hazards * sizeof(double), f,
-                         (const int64_t *) x.d_target, (const int64_t *) x.d_root, (const uint8_t *) x.d_depth,
-                         (const uint8_t *) x.d_neg, (const double *) x.d_value, x.hazards, x.n, pred);
+    BcRun r{};
+    if (one_run(p, f, &r)) {
+        ARTSS_LAUNCH_PDL(ctx, FAM_BC, k_bc, run_blocks(r), 256, r.hazards * sizeof(double), r, BcStep{}, pred);
         ARTSS_LAUNCH_CK(ctx);
         return ARTSS_OK;
     }
     for (int w = 0; w < p.waves; w++) {
-        const int64_t b = p.wave_begin[w], e = p.wave_begin[w + 1];
-        if (e <= b) continue;
-        cudaError_t err;
-        ARTSS_LAUNCH(ctx, FAM_BC,
-                     err = launch_pdl(ctx, k_bc_wave, dim3((unsigned) flat_blocks(e - b)), dim3(256), 0, f,
-                                      (const int64_t *) p.d_target, (const int64_t *) p.d_root,
-                                      (const uint8_t *) p.d_depth, (const uint8_t *) p.d_neg,
-                                      (const double *) p.d_value, b, e, p.n, pred));
-        if (err != cudaSuccess) return cuda_fail(err, "kernel launch");
+        r = BcRun{f, p.d_target, p.d_root, p.d_depth, p.d_neg, p.d_value, p.wave_begin[w], p.wave_begin[w + 1], p.n, 0};
+        if (r.end <= r.begin) continue;
+        ARTSS_LAUNCH_PDL(ctx, FAM_BC, k_bc, run_blocks(r), 256, 0, r, BcStep{}, pred);
         ARTSS_LAUNCH_CK(ctx);
     }
     return ARTSS_OK;
+}
+
+int apply_bc_step(artss_ctx *ctx, double *f, int level, int field_type, int slot, int parity, int nblocks, double tol,
+                  long long max_it) {
+    const BcProgram &p = ctx->bc[level][field_type];
+    const LoopState *rd = ctx->d_loop + slot + parity;
+    BcRun r{};
+    if (p.present && p.n > 0 && one_run(p, f, &r)) {
+        static_assert(kReduceThreads == 256, "the step block has the program's block size");
+        const BcStep s{ctx->d_partials, nblocks, rd, ctx->d_loop + slot + 1 - parity, tol, max_it};
+        ARTSS_LAUNCH_PDL(ctx, FAM_BC, k_bc, run_blocks(r) + 1, 256, r.hazards * sizeof(double), r, s, rd);
+        ARTSS_LAUNCH_CK(ctx);
+        return ARTSS_OK;
+    }
+    int st = apply_bc(ctx, f, level, field_type, rd);
+    return st ? st : finalize_loop_pair(ctx, slot, parity, nblocks, tol, max_it);
+}
+
+int apply_bc_uvw(artss_ctx *ctx, double *u, double *v, double *w) {
+    double *f[3] = {u, v, w};
+    const int ft[3] = {ARTSS_FIELD_U, ARTSS_FIELD_V, ARTSS_FIELD_W};
+    BcRun r[3]{};
+    bool one = u != v && v != w && u != w;
+    unsigned blocks = 0;
+    int64_t hazards = 0;
+    for (int c = 0; c < 3 && one; c++) {
+        const BcProgram &p = ctx->bc[0][ft[c]];
+        one = p.present && p.n > 0 && one_run(p, f[c], &r[c]);
+        if (!one) break;
+        blocks = std::max(blocks, run_blocks(r[c]));
+        hazards = std::max(hazards, r[c].hazards);
+    }
+    if (one) {
+        ARTSS_LAUNCH_PDL(ctx, FAM_BC, k_bc3, dim3(blocks, 3), 256, hazards * sizeof(double), r[0], r[1], r[2]);
+        ARTSS_LAUNCH_CK(ctx);
+        return ARTSS_OK;
+    }
+    int st = ARTSS_OK;
+    for (int c = 0; c < 3 && !st; c++) st = apply_bc(ctx, f[c], 0, ft[c]);
+    return st;
 }
 
 // The boundary program with every value taken as zero, on FP32 storage: the

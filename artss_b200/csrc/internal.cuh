@@ -28,6 +28,7 @@ constexpr int64_t kBcMaxHazards = 4096; // of a flat program, staged in one bloc
 constexpr uint8_t kBcLagged = 0x80;     // flat program: the root is itself a target
 constexpr int kReduceThreads = 256;
 constexpr int kMaxPartials = 1 << 16;   // per-block partial sums of up to two reduction passes
+constexpr int kDiffuseSlot = 8;         // loop states of the diffusion solvers, a pair (8, 9)
 constexpr int kNnErrSlot = 15;          // loop slot whose error flag the network kernels raise
 constexpr int kTmaBoxX = 72, kTmaBoxY = 12;  // TMA plane window (cells): a 64 x 8 tile, a 2-cell ring, x aligned to 2
 
@@ -457,6 +458,16 @@ inline int check_reduce_blocks(const dim3 &g) {
 // pred != NULL: every launch returns at once when pred->cond == 0 (predicated loop body)
 int apply_bc(artss_ctx *ctx, double *f, int level, int field_type, const LoopState *pred = nullptr);
 
+// The end of a predicated loop iteration: the boundary program on f and the loop
+// step (the sum of the sweep's `nblocks` partials, the residual, the decision) in one
+// launch where the program is one.  The program's blocks and the sweep read the
+// state `slot + parity`, the step writes the other one, slot + 1 - parity: no block
+// sees the decision of its own iteration.
+int apply_bc_step(artss_ctx *ctx, double *f, int level, int field_type, int slot, int parity, int nblocks, double tol,
+                  long long max_it);
+// u, v and w's boundary programs on level 0, in one launch where each is one
+int apply_bc_uvw(artss_ctx *ctx, double *u, double *v, double *w);
+
 // Homogeneous boundary program (values zero) on FP32 storage (bc.cu).
 int apply_bc_f32(artss_ctx *ctx, float *f, int level, int field_type, const LoopState *pred = nullptr);
 // FP64 cluster (block: one-block where the level fits) solve of a level's
@@ -494,6 +505,8 @@ struct GraphLoop {
     int begin(artss_ctx *c, int cond0);
     int end(int slot, long long cap);
 };
+// loop step from state slot + parity to state slot + 1 - parity
+int finalize_loop_pair(artss_ctx *ctx, int slot, int parity, int nblocks, double tol, long long max_it);
 // Plain sum of partials into loop slot (no iteration bookkeeping).
 int finalize_sum(artss_ctx *ctx, int slot, int nblocks);
 // sum of partials -> residual = sqrt(sum), no loop bookkeeping
@@ -516,6 +529,32 @@ __device__ __forceinline__ double artss_block_sum(double v, double *smem) {
         for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     }
     return v;
+}
+
+// One loop step by a block of artss::kReduceThreads threads: partials summed in a
+// fixed order, the next state written to `wr`.  A state whose loop has ended is
+// handed on unchanged.
+__device__ __forceinline__ void artss_loop_step(const double *__restrict__ partials, int nblocks,
+                                                const artss::LoopState *rd, artss::LoopState *wr, double tol,
+                                                long long max_it, double *smem) {
+    double v = 0.0;
+    if (rd->cond)
+        for (int b = threadIdx.x; b < nblocks; b += blockDim.x) v += partials[b];
+    v = artss_block_sum(v, smem);
+    if (threadIdx.x == 0) {
+        artss::LoopState s = *rd;
+        if (s.cond) {
+            s.sum = v;
+            s.residual = sqrt(v);
+            s.it += 1;
+            s.cond = (s.residual > tol && s.it < max_it) ? 1 : 0;
+        }
+        wr->sum = s.sum;
+        wr->residual = s.residual;
+        wr->it = s.it;
+        wr->cond = s.cond;
+        wr->pad = s.pad;
+    }
 }
 
 // Launches a kernel inside a ProfScope of the given family.

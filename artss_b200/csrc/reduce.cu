@@ -39,6 +39,14 @@ __global__ void k_finalize_loop(const double *__restrict__ partials, int nblocks
     }
 }
 
+__global__ void k_finalize_loop_pair(const double *__restrict__ partials, int nblocks, const LoopState *rd, LoopState *wr,
+                                     double tol, long long max_it) {
+    pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
+    pdl_trigger();
+    __shared__ double smem[32];
+    artss_loop_step(partials, nblocks, rd, wr, tol, max_it, smem);
+}
+
 __global__ void k_init_loop(LoopState *st, double r0, long long it0, int cond0) {
     pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
     pdl_trigger();
@@ -64,6 +72,13 @@ __global__ void k_loop_continue(LoopState *st, cudaGraphConditionalHandle h, lon
 
 int finalize_loop(artss_ctx *ctx, int slot, int nblocks, double tol, long long max_it) {
     ARTSS_LAUNCH_PDL(ctx, FAM_REDUCE, k_finalize_loop, 1, kReduceThreads, 0, ctx->d_partials, nblocks, ctx->d_loop + slot, tol, max_it, 0, nullptr);
+    ARTSS_LAUNCH_CK(ctx);
+    return ARTSS_OK;
+}
+
+int finalize_loop_pair(artss_ctx *ctx, int slot, int parity, int nblocks, double tol, long long max_it) {
+    ARTSS_LAUNCH_PDL(ctx, FAM_REDUCE, k_finalize_loop_pair, 1, kReduceThreads, 0, (const double *) ctx->d_partials, nblocks,
+                     (const LoopState *) (ctx->d_loop + slot + parity), ctx->d_loop + slot + 1 - parity, tol, max_it);
     ARTSS_LAUNCH_CK(ctx);
     return ARTSS_OK;
 }

@@ -1499,9 +1499,7 @@ int artss_advect_sl_uvw(artss_ctx *ctx, double *out_u, double *out_v, double *ou
              return ARTSS_OK;
          })))
         return st;
-    if ((st = apply_bc(ctx, out_u, 0, ARTSS_FIELD_U))) return st;
-    if ((st = apply_bc(ctx, out_v, 0, ARTSS_FIELD_V))) return st;
-    return apply_bc(ctx, out_w, 0, ARTSS_FIELD_W);
+    return apply_bc_uvw(ctx, out_u, out_v, out_w);
 }
 
 int artss_turb_const_smagorinsky(artss_ctx *ctx, double *nu_t, const double *u, const double *v, const double *w,
@@ -1565,9 +1563,7 @@ int artss_projection(artss_ctx *ctx, double *u, double *v, double *w, const doub
              return ARTSS_OK;
          })))
         return st;
-    if ((st = apply_bc(ctx, u, 0, ARTSS_FIELD_U))) return st;
-    if ((st = apply_bc(ctx, v, 0, ARTSS_FIELD_V))) return st;
-    return apply_bc(ctx, w, 0, ARTSS_FIELD_W);
+    return apply_bc_uvw(ctx, u, v, w);
 }
 
 int artss_buoyancy_force(artss_ctx *ctx, double *force, const double *T, const double *Ta, double beta, double g) {
@@ -1905,14 +1901,15 @@ int artss_diffuse_cgs(artss_ctx *ctx, double *out, double *in, const double *b, 
     const DiffCoef c = diff_coef(ctx, D, dt, cfg->w, 1.0);
     // out.copy_data(in) (ColoredGaussSeidelDiffuse.cpp:41,114), unless out holds in already
     if (!(flags & ARTSS_DIFFUSE_OUT_HOLDS_IN) && (st = artss_copy(ctx, out, in, 0))) return st;
-    const int slot = 0;
+    // iteration n reads loop state kDiffuseSlot + ((n - 1) & 1) and writes the other
+    const int slot = kDiffuseSlot;
     // while (res > tol_res && it < max_iter), res starts at 1
     long long it = 0;
     double res = 1.;
     bool cond = res > cfg->tol_res && it < cfg->max_iter;
     if ((st = init_loop(ctx, slot, res, 0, cond ? 1 : 0))) return st;
     LoopState ls{};
-    const LoopState *pred = ctx->d_loop + slot;
+    auto state = [&](long long n) { return ctx->d_loop + slot + ((n - 1) & 1); };
     int64_t batch = std::max<int64_t>(1, std::min<int64_t>(loop_hint(ctx, 0, field_type), cfg->max_iter));
     // The reference sweeps `out` in place after in.copy_data(out) (:69-76); here
     // iteration n reads iterate n-1 from one of {out, in} and writes iterate n
@@ -1944,11 +1941,10 @@ int artss_diffuse_cgs(artss_ctx *ctx, double *out, double *in, const double *b, 
             }
         }
     }
-    LoopState *pred_rw = ctx->d_loop + slot;
     int depth = 1;  // the sweep variant (launch_sweep_tma)
     if (tma && cond) {
         const int n1 = (s0 + 1) & 1;
-        if ((st = tune_sweep(ctx, ev != nullptr, one_phase, box, maps[1 - n1], buf[n1], L, c, pred_rw, &depth)))
+        if ((st = tune_sweep(ctx, ev != nullptr, one_phase, box, maps[1 - n1], buf[n1], L, c, state(1), &depth)))
             return st;
     }
     if (ctx->capturing) {
@@ -1962,17 +1958,17 @@ int artss_diffuse_cgs(artss_ctx *ctx, double *out, double *in, const double *b, 
                 const double *rd = buf[(s0 + n + 1) & 1];
                 if (tma) {
                     if ((st = launch_sweep_tma(ctx, ev != nullptr, depth, box, maps[(s0 + n + 1) & 1], w, L, c,
-                                               pred_rw, &nb)))
+                                               state(n), &nb)))
                         return st;
                 } else if (ev)
                     ARTSS_LAUNCH(ctx, FAM_CGS, k_cgs_sweep<true><<<g, dim3(kSwTx / 2, kSwTy), smem, ctx->stream>>>(
-                        w, rd, b, ev, ctx->d_flags[0], L, box, c, ctx->d_partials, pred));
+                        w, rd, b, ev, ctx->d_flags[0], L, box, c, ctx->d_partials, state(n)));
                 else
                     ARTSS_LAUNCH(ctx, FAM_CGS, k_cgs_sweep<false><<<g, dim3(kSwTx / 2, kSwTy), smem, ctx->stream>>>(
-                        w, rd, b, nullptr, ctx->d_flags[0], L, box, c, ctx->d_partials, pred));
+                        w, rd, b, nullptr, ctx->d_flags[0], L, box, c, ctx->d_partials, state(n)));
                 if (!tma) ARTSS_LAUNCH_CK(ctx);
-                if ((st = apply_bc(ctx, w, 0, field_type, pred))) return st;
-                if ((st = finalize_loop(ctx, slot, nb, cfg->tol_res, cfg->max_iter))) return st;
+                if ((st = apply_bc_step(ctx, w, 0, field_type, slot, (n - 1) & 1, nb, cfg->tol_res, cfg->max_iter)))
+                    return st;
             }
             if ((st = gl.end(slot, cfg->max_iter / 2 + 2))) return st;
             const int64_t n = L.size();
@@ -1990,20 +1986,20 @@ int artss_diffuse_cgs(artss_ctx *ctx, double *out, double *in, const double *b, 
             double *w = buf[(s0 + n) & 1];
             const double *rd = buf[(s0 + n + 1) & 1];
             if (tma) {
-                if ((st = launch_sweep_tma(ctx, ev != nullptr, depth, box, maps[(s0 + n + 1) & 1], w, L, c, pred_rw,
+                if ((st = launch_sweep_tma(ctx, ev != nullptr, depth, box, maps[(s0 + n + 1) & 1], w, L, c, state(n),
                                            &nb)))
                     return st;
             } else if (ev)
                 ARTSS_LAUNCH(ctx, FAM_CGS, k_cgs_sweep<true><<<g, dim3(kSwTx / 2, kSwTy), smem, ctx->stream>>>(
-                    w, rd, b, ev, ctx->d_flags[0], L, box, c, ctx->d_partials, pred));
+                    w, rd, b, ev, ctx->d_flags[0], L, box, c, ctx->d_partials, state(n)));
             else
                 ARTSS_LAUNCH(ctx, FAM_CGS, k_cgs_sweep<false><<<g, dim3(kSwTx / 2, kSwTy), smem, ctx->stream>>>(
-                    w, rd, b, nullptr, ctx->d_flags[0], L, box, c, ctx->d_partials, pred));
+                    w, rd, b, nullptr, ctx->d_flags[0], L, box, c, ctx->d_partials, state(n)));
             if (!tma) ARTSS_LAUNCH_CK(ctx);
-            if ((st = apply_bc(ctx, w, 0, field_type, pred))) return st;
-            if ((st = finalize_loop(ctx, slot, nb, cfg->tol_res, cfg->max_iter))) return st;
+            if ((st = apply_bc_step(ctx, w, 0, field_type, slot, (int) ((n - 1) & 1), nb, cfg->tol_res, cfg->max_iter)))
+                return st;
         }
-        if ((st = read_loop(ctx, slot, &ls))) return st;
+        if ((st = read_loop(ctx, slot + (int) ((it + batch) & 1), &ls))) return st;
         if (ls.pad) { set_error("colored Gauss-Seidel sweep: a TMA plane load did not arrive"); return ARTSS_ERR_CUDA; }
         it = ls.it;
         res = ls.residual;
