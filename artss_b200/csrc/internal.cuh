@@ -137,6 +137,11 @@ struct artss_ctx {
     artss::Level lvl[artss::kMaxLevel + 1]{};
     uint8_t *d_flags[artss::kMaxLevel + 1]{};
     std::vector<bool> h_inner[artss::kMaxLevel + 1];  // inner-cell bitmap per level, host copy
+    std::vector<bool> h_domain0;                      // domain-list bitmap of level 0, host copy
+    // per field type: the Jacobi diffusion may alternate between its two arrays
+    // (jacobi_alternates), decided for geometry alternates_version
+    int8_t alternates[artss::kFieldTypes] = {};
+    uint64_t alternates_version[artss::kFieldTypes] = {};
     int64_t n_inner[artss::kMaxLevel + 1]{};  // inner cells per level (artss_set_cell_lists)
     double *proj[artss::kMaxLevel + 1]{};     // scratch of artss_coarse_project (lazily, freed with fields)
     artss::BcProgram bc[artss::kMaxLevel + 1][artss::kFieldTypes];

@@ -1348,39 +1348,47 @@ __global__ void k_cgsm_correct(double *__restrict__ x, const float *__restrict__
 
 // One Jacobi step of JacobiDiffuse (laminar: JacobiDiffuse.cpp:241-249, note
 // the division by reciprocal_beta; turbulent: :345-362) + residual partials
-// of sum (rbeta * (out - in))^2 (:72-79).
+// of sum (rbeta * (out - in))^2 (:72-79).  Bound by memory (32 bytes a cell,
+// turbulent); the column march loads a plane's centre values once for the three
+// planes that read them.
 template <bool TURB>
-__global__ void k_jacobi_diffuse(double *__restrict__ out, const double *__restrict__ in, const double *__restrict__ b,
-                                 const double *__restrict__ ev, const uint8_t *__restrict__ flags, Level L, Box3 box,
-                                 DiffCoef c, double *__restrict__ partials, const LoopState *__restrict__ pred) {
+__global__ void __launch_bounds__(256, 4)
+k_jacobi_diffuse(double *__restrict__ out, const double *__restrict__ in, const double *__restrict__ b,
+                 const double *__restrict__ ev, const uint8_t *__restrict__ flags, Level L, Box3 box, DiffCoef c,
+                 double *__restrict__ partials, const LoopState *__restrict__ pred) {
     __shared__ double smem[32];
+    pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
+    pdl_trigger();
     if (pred && !pred->cond) return;  // iteration enqueued past convergence
     ARTSS_COLUMN(box);
     const int nj = (int) L.Nx, nk = (int) L.nxy();
     double acc = 0.0;
     if (col) {
-        for (int k = (int) box.z0 + (int) blockIdx.z; k <= (int) box.z1; k += (int) gridDim.z) {
-            const int q = i + (int) L.Nx * j + nk * k;
-            if (!(flags[q] & kInner)) continue;
-            double out_h, rb;
-            if (TURB) {
-                double ax, ay, az;
-                turb_alpha(c, ev[q], ax, ay, az, rb);
-                const double bb = 1. / rb;
-                const double d_ax = ax * (in[q + 1] + in[q - 1]);
-                const double d_ay = ay * (in[q + nj] + in[q - nj]);
-                const double d_az = az * (in[q + nk] + in[q - nk]);
-                out_h = bb * (c.dsign * b[q] + d_ax + d_ay + d_az);
-            } else {
-                rb = c.rbeta;
-                out_h = (c.dsign * b[q] + c.ax * (in[q + 1] + in[q - 1]) + c.ay * (in[q + nj] + in[q - nj])
-                         + c.az * (in[q + nk] + in[q - nk])) / c.rbeta;
-            }
-            const double nw = c.omw * in[q] + c.w * out_h;
-            out[q] = nw;
-            const double res = rb * (nw - in[q]);
-            acc += res * res;
-        }
+        struct NR { double nw, res2; };
+        column_march<2>(in, i + nj * j, nk, (int) box.z0, (int) box.z1, flags,
+            [&](int q, int, double km, double c0, double kp) {
+                double out_h, rb;
+                if (TURB) {
+                    double ax, ay, az;
+                    turb_alpha(c, ev[q], ax, ay, az, rb);
+                    const double bb = 1. / rb;
+                    const double d_ax = ax * (in[q + 1] + in[q - 1]);
+                    const double d_ay = ay * (in[q + nj] + in[q - nj]);
+                    const double d_az = az * (kp + km);
+                    out_h = bb * (c.dsign * b[q] + d_ax + d_ay + d_az);
+                } else {
+                    rb = c.rbeta;
+                    out_h = (c.dsign * b[q] + c.ax * (in[q + 1] + in[q - 1]) + c.ay * (in[q + nj] + in[q - nj])
+                             + c.az * (kp + km)) / c.rbeta;
+                }
+                const double nw = c.omw * c0 + c.w * out_h;
+                const double res = rb * (nw - c0);
+                return NR{nw, res * res};
+            },
+            [&](int q, int, NR v, uint8_t) {
+                out[q] = v.nw;
+                acc += v.res2;
+            });
     }
     acc = artss_block_sum(acc, smem);
     if (threadIdx.x == 0 && threadIdx.y == 0) partials[block_linear()] = acc;
@@ -1410,6 +1418,22 @@ __global__ void k_cgs_fixup(double *__restrict__ out, double *__restrict__ in, c
         const double v = in[i];
         if (!in_is_scratch) in[i] = out[i];
         out[i] = v;
+    }
+}
+
+// After a captured alternating Jacobi loop: the last iterate sits in `out` after an
+// odd number of iterations, else in `in`; the other one gets it over the domain list.
+__global__ void k_jacobi_fixup(double *__restrict__ out, double *__restrict__ in, const LoopState *__restrict__ st,
+                               const uint8_t *__restrict__ flags, Level L, Box3 box) {
+    const long long it = st->it;
+    if (it <= 0) return;
+    double *dst = it & 1 ? in : out;
+    const double *src = it & 1 ? out : in;
+    ARTSS_COLUMN(box);
+    if (!col) return;
+    for (int k = (int) box.z0 + (int) blockIdx.z; k <= (int) box.z1; k += (int) gridDim.z) {
+        const int q = i + (int) L.Nx * j + (int) L.nxy() * k;
+        if (flags[q] & kDomain) dst[q] = src[q];
     }
 }
 
@@ -2084,6 +2108,43 @@ int artss_diffuse_cgs_mixed(artss_ctx *ctx, double *out, double *in, const doubl
     return ARTSS_OK;
 }
 
+}  // extern "C"
+
+namespace {
+// JacobiDiffuse copies in = out over the domain list after every iteration
+// (JacobiDiffuse.cpp:85-89).  The two arrays may take turns instead where that copy
+// gives the next iteration exactly what the array just written holds: every face
+// neighbour of an inner cell is on the domain list (obstacles that leave cells off
+// it keep their old values in `in`), the cells on it are the inner ones and the
+// program's targets, and the program reads nothing that it writes (one wave).
+bool jacobi_alternates(artss_ctx *ctx, int ft) {
+    if (ctx->alternates[ft] && ctx->alternates_version[ft] == ctx->geom_version) return ctx->alternates[ft] > 0;
+    const Level &L = ctx->lvl[0];
+    const std::vector<bool> &in = ctx->h_inner[0], &dom = ctx->h_domain0;
+    const BcProgram &p = ctx->bc[0][ft];
+    bool ok = (int64_t) in.size() == L.size() && (int64_t) dom.size() == L.size() && (!p.present || p.waves <= 1);
+    if (ok) {
+        std::vector<bool> set(in);
+        for (int64_t t : p.h_target) {
+            ok = ok && dom[(size_t) t];
+            set[(size_t) t] = true;
+        }
+        for (int64_t r : p.h_root) ok = ok && dom[(size_t) r];
+        const int64_t off[6] = {-1, 1, -L.Nx, L.Nx, -L.nxy(), L.nxy()};
+        for (int64_t q = 0; q < L.size() && ok; q++) {
+            ok = dom[(size_t) q] == set[(size_t) q];
+            if (in[(size_t) q])
+                for (int64_t d : off) ok = ok && dom[(size_t) (q + d)];
+        }
+    }
+    ctx->alternates[ft] = ok ? 1 : -1;
+    ctx->alternates_version[ft] = ctx->geom_version;
+    return ok;
+}
+}  // namespace
+
+extern "C" {
+
 int artss_diffuse_jacobi(artss_ctx *ctx, double *out, double *in, const double *b, double D, const double *ev,
                          double dt, int field_type, const artss_iter_cfg *cfg, artss_iter_stats *stats) {
     int st = check_field_args(ctx, {out, in, b, cfg});
@@ -2096,54 +2157,74 @@ int artss_diffuse_jacobi(artss_ctx *ctx, double *out, double *in, const double *
     if ((st = check_reduce_blocks(g))) return st;
     const int nb = nblocks(g);
     const DiffCoef c = diff_coef(ctx, D, dt, cfg->w, 1.0);
-    const int slot = 0;
+    // iteration n reads loop state kDiffuseSlot + ((n - 1) & 1) and writes the other
+    const int slot = kDiffuseSlot;
+    auto state = [&](long long n) { return (const LoopState *) (ctx->d_loop + slot + ((n - 1) & 1)); };
     long long it = 0;
     double res = 1.;
     bool cond = res > cfg->tol_res && it < cfg->max_iter;
     if ((st = init_loop(ctx, slot, res, 0, cond ? 1 : 0))) return st;
     LoopState ls{};
-    const LoopState *pred = ctx->d_loop + slot;
     int64_t batch = std::max<int64_t>(1, std::min<int64_t>(loop_hint(ctx, 1, field_type), cfg->max_iter));
-    GraphLoop gl;
+    // the arrays take turns (iteration n odd: in -> out), or `in` follows `out` by a copy
+    const bool turns = out != in && b != in && b != out && ev != in && ev != out && jacobi_alternates(ctx, field_type);
+    auto iteration = [&](long long n) -> int {
+        double *w = turns && !(n & 1) ? in : out;
+        const double *rd = turns && !(n & 1) ? out : in;
+        if (ev)
+            ARTSS_LAUNCH_PDL(ctx, FAM_JACOBI, k_jacobi_diffuse<true>, g, box_block(), 0, w, rd, b, ev,
+                             (const uint8_t *) ctx->d_flags[0], L, box, c, ctx->d_partials, state(n));
+        else
+            ARTSS_LAUNCH_PDL(ctx, FAM_JACOBI, k_jacobi_diffuse<false>, g, box_block(), 0, w, rd, b,
+                             (const double *) nullptr, (const uint8_t *) ctx->d_flags[0], L, box, c, ctx->d_partials,
+                             state(n));
+        ARTSS_LAUNCH_CK(ctx);
+        if (turns)
+            return apply_bc_step(ctx, w, 0, field_type, slot, (int) ((n - 1) & 1), nb, cfg->tol_res, cfg->max_iter);
+        int e = apply_bc(ctx, out, 0, field_type, state(n));
+        if (e) return e;
+        // in = out before the loop decision: the residual partials are already taken
+        ARTSS_LAUNCH(ctx, FAM_COPY_DOMAIN, k_copy_domain<<<zgrid(dbox), box_block(), 0, ctx->stream>>>(
+            in, out, ctx->d_flags[0], L, dbox, state(n)));
+        ARTSS_LAUNCH_CK(ctx);
+        return finalize_loop_pair(ctx, slot, (int) ((n - 1) & 1), nb, cfg->tol_res, cfg->max_iter);
+    };
     if (ctx->capturing) {
-        // one iteration per body of a WHILE node decided on the device
+        // two iterations per body of a WHILE node decided on the device
         if (!cond) {
             if (stats) { stats->iterations = 0; stats->residual = res; }
             return ARTSS_OK;
         }
+        GraphLoop gl;
         if ((st = gl.begin(ctx, 1))) return st;
-        batch = 1;
+        for (int n = 1; n <= 2; n++)
+            if ((st = iteration(n))) return st;
+        if ((st = gl.end(slot, cfg->max_iter / 2 + 2))) return st;
+        if (turns) {
+            ARTSS_LAUNCH(ctx, FAM_COPY_DOMAIN, k_jacobi_fixup<<<zgrid(dbox), box_block(), 0, ctx->stream>>>(
+                out, in, ctx->d_loop + slot, ctx->d_flags[0], L, dbox));
+            ARTSS_LAUNCH_CK(ctx);
+        }
+        if (stats) { stats->iterations = -1; stats->residual = -1.0; }
+        return ARTSS_OK;
     }
     while (cond) {
-        for (int64_t r = 0; r < batch; r++) {
-            if (ev)
-                ARTSS_LAUNCH(ctx, FAM_JACOBI, k_jacobi_diffuse<true><<<g, box_block(), 0, ctx->stream>>>(
-                    out, in, b, ev, ctx->d_flags[0], L, box, c, ctx->d_partials, pred));
-            else
-                ARTSS_LAUNCH(ctx, FAM_JACOBI, k_jacobi_diffuse<false><<<g, box_block(), 0, ctx->stream>>>(
-                    out, in, b, nullptr, ctx->d_flags[0], L, box, c, ctx->d_partials, pred));
-            ARTSS_LAUNCH_CK(ctx);
-            if ((st = apply_bc(ctx, out, 0, field_type, pred))) return st;
-            // in = out before the loop decision: the residual partials are already taken
-            ARTSS_LAUNCH(ctx, FAM_COPY_DOMAIN, k_copy_domain<<<zgrid(dbox), box_block(), 0, ctx->stream>>>(
-                in, out, ctx->d_flags[0], L, dbox, pred));
-            ARTSS_LAUNCH_CK(ctx);
-            if ((st = finalize_loop(ctx, slot, nb, cfg->tol_res, cfg->max_iter))) return st;
-        }
-        if (ctx->capturing) {
-            if ((st = gl.end(slot, cfg->max_iter + 2))) return st;
-            if (stats) { stats->iterations = -1; stats->residual = -1.0; }
-            return ARTSS_OK;
-        }
-        if ((st = read_loop(ctx, slot, &ls))) return st;
+        for (int64_t r = 0; r < batch; r++)
+            if ((st = iteration(it + 1 + r))) return st;
+        if ((st = read_loop(ctx, slot + (int) ((it + batch) & 1), &ls))) return st;
         it = ls.it;
         res = ls.residual;
         cond = ls.cond != 0;
         batch = std::min<int64_t>(2 * batch, std::max<int64_t>(1, cfg->max_iter - it));
     }
     loop_hint(ctx, 1, field_type) = std::max<int64_t>(1, it);
-    // the final odd-count copy of JacobiDiffuse.cpp:92-99 repeats the last
-    // in = out over the domain list and changes nothing
+    // the copy of the last iteration; the final odd-count copy of
+    // JacobiDiffuse.cpp:92-99 repeats it and changes nothing
+    if (turns && it > 0) {
+        ARTSS_LAUNCH(ctx, FAM_COPY_DOMAIN, k_copy_domain<<<zgrid(dbox), box_block(), 0, ctx->stream>>>(
+            it & 1 ? in : out, it & 1 ? out : in, ctx->d_flags[0], L, dbox, nullptr));
+        ARTSS_LAUNCH_CK(ctx);
+    }
     if (stats) { stats->iterations = it; stats->residual = res; }
     return ARTSS_OK;
 }
