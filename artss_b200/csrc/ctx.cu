@@ -788,9 +788,11 @@ int artss_set_cell_lists(artss_ctx *ctx, int level, const int64_t *inner, int64_
     if (!check(inner, n_inner, 0, "inner") || !check(domain, n_domain, 1, "domain")) return ARTSS_ERR_ARG;
     ctx->h_inner[level].assign((size_t) L.size(), false);
     for (int64_t q = 0; q < n_inner; q++) ctx->h_inner[level][(size_t) inner[q]] = true;
+    ctx->inner_bits[level].reset(L.size());
+    for (int64_t q = 0; q < n_inner; q++) ctx->inner_bits[level].set(inner[q]);
     if (level == 0) {
-        ctx->h_domain0.assign((size_t) L.size(), false);
-        for (int64_t q = 0; q < n_domain; q++) ctx->h_domain0[(size_t) domain[q]] = true;
+        ctx->domain_bits.reset(L.size());
+        for (int64_t q = 0; q < n_domain; q++) ctx->domain_bits.set(domain[q]);
     }
     for (auto &prog : ctx->bc[level]) prog.pipe_state = -2;
     int64_t *d_list = nullptr;

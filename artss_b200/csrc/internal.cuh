@@ -81,6 +81,31 @@ struct BcProgram {
     int64_t pipe_smem = 0;
 };
 
+// Cells of a level as a bit map, for host checks of whole neighbourhoods: 64 cells
+// at a time, a level of 4 M cells and 6 neighbours in under a millisecond.
+struct CellBits {
+    std::vector<uint64_t> w;
+    int64_t n = 0;
+    void reset(int64_t cells) {
+        n = cells;
+        w.assign((size_t) ((cells + 63) / 64), 0);
+    }
+    void set(int64_t q) { w[(size_t) (q >> 6)] |= 1ull << (q & 63); }
+    bool get(int64_t q) const { return w[(size_t) (q >> 6)] >> (q & 63) & 1; }
+    uint64_t word(int64_t first) const {  // cells first .. first + 63, 0 outside
+        const int64_t i = first >> 6;
+        const int s = (int) (first & 63);
+        const auto at = [&](int64_t k) { return k >= 0 && k < (int64_t) w.size() ? w[(size_t) k] : 0ull; };
+        return s ? at(i) >> s | at(i + 1) << (64 - s) : at(i);
+    }
+    // every cell q of this one has q + off in `other`
+    bool neighbours_in(const CellBits &other, int64_t off) const {
+        for (int64_t i = 0; i < (int64_t) w.size(); i++)
+            if (w[(size_t) i] & ~other.word(64 * i + off)) return false;
+        return true;
+    }
+};
+
 // Device-resident control block of one bounded iteration loop.
 struct LoopState {
     double sum;        // reduction result of the last pass
@@ -137,7 +162,7 @@ struct artss_ctx {
     artss::Level lvl[artss::kMaxLevel + 1]{};
     uint8_t *d_flags[artss::kMaxLevel + 1]{};
     std::vector<bool> h_inner[artss::kMaxLevel + 1];  // inner-cell bitmap per level, host copy
-    std::vector<bool> h_domain0;                      // domain-list bitmap of level 0, host copy
+    artss::CellBits inner_bits[artss::kMaxLevel + 1], domain_bits;  // inner cells; domain list of level 0
     // per field type: the Jacobi diffusion may alternate between its two arrays
     // (jacobi_alternates), decided for geometry alternates_version
     int8_t alternates[artss::kFieldTypes] = {};

@@ -2028,35 +2028,31 @@ int artss_mg_create(artss_ctx *ctx, const artss_mg_cfg *cfg, artss_mg **out) {
     for (int l = 0; l < mg->L; l++) {
         const BcProgram &p = ctx->bc[l][ARTSS_FIELD_P];
         const Level &F = ctx->lvl[l];
-        const std::vector<bool> &in = ctx->h_inner[l];
-        if (!p.present || p.waves > 1 || (int64_t) in.size() != F.size()) continue;
-        std::vector<bool> known(in);
+        const CellBits &in = ctx->inner_bits[l], &cin = ctx->inner_bits[l + 1];
+        const Level &Cl = ctx->lvl[l + 1];
+        if (!p.present || p.waves > 1 || in.n != F.size() || cin.n != Cl.size()) continue;
+        CellBits known = in;
         bool ok = true;
-        for (int64_t t : p.h_target) known[(size_t) t] = true;
-        for (int64_t r : p.h_root) ok = ok && in[(size_t) r];
+        for (int64_t t : p.h_target) known.set(t);
+        for (int64_t r : p.h_root) ok = ok && in.get(r);
         // smoothing and residual read the 6 face neighbours, the prolongation from a
         // coarse level all 26
-        for (int64_t q = 0; q < F.size() && ok; q++) {
-            if (!in[(size_t) q]) continue;
-            for (int c = -1; c <= 1; c++)
-                for (int b = -1; b <= 1; b++)
-                    for (int a = -1; a <= 1; a++)
-                        if (l > 0 || abs(a) + abs(b) + abs(c) == 1) ok = ok && known[(size_t) (q + a + F.Nx * b + F.nxy() * c)];
-        }
-        // ... and the prolongation to this level writes known cells only
-        const Level &Cl = ctx->lvl[l + 1];
-        const std::vector<bool> &cin = ctx->h_inner[l + 1];
-        if ((int64_t) cin.size() != Cl.size()) continue;
-        for (int64_t k = 0; k < Cl.Nz && ok; k++)
-            for (int64_t j = 0; j < Cl.Ny && ok; j++)
-                for (int64_t i = 0; i < Cl.Nx && ok; i++) {
-                    if (!cin[(size_t) (i + Cl.Nx * j + Cl.nxy() * k)]) continue;
-                    for (int c = 0; c < 8 && ok; c++) {
-                        const int64_t fi = 2 * i - 1 + (c & 1), fj = 2 * j - 1 + (c >> 1 & 1), fk = 2 * k - 1 + (c >> 2);
-                        ok = fi >= 0 && fj >= 0 && fk >= 0 && fi < F.Nx && fj < F.Ny && fk < F.Nz &&
-                             known[(size_t) (fi + F.Nx * fj + F.nxy() * fk)];
-                    }
-                }
+        for (int c = -1; c <= 1; c++)
+            for (int b = -1; b <= 1; b++)
+                for (int a = -1; a <= 1; a++)
+                    if (l > 0 || abs(a) + abs(b) + abs(c) == 1)
+                        ok = ok && in.neighbours_in(known, a + F.Nx * b + F.nxy() * c);
+        // ... and the prolongation to this level, cells 2 c - 1 and 2 c of an inner
+        // coarse cell c, writes known cells only
+        ok = ok && 2 * Cl.i2 < F.Nx && 2 * Cl.j2 < F.Ny && 2 * Cl.k2 < F.Nz;
+        for (int64_t i = 0; i < (int64_t) known.w.size() && ok; i++)
+            for (uint64_t rest = ~known.w[(size_t) i]; rest && ok; rest &= rest - 1) {
+                const int64_t q = 64 * i + __builtin_ctzll(rest);
+                if (q >= F.size()) break;
+                const int64_t z = q / F.nxy(), y = q / F.Nx % F.Ny, x = q % F.Nx;
+                const int64_t ci = (x + 1) / 2, cj = (y + 1) / 2, ck = (z + 1) / 2;
+                ok = ci >= Cl.Nx || cj >= Cl.Ny || ck >= Cl.Nz || !cin.get(ci + Cl.Nx * cj + Cl.nxy() * ck);
+            }
         mg->closed[l] = ok;
     }
     *out = mg;

@@ -2120,22 +2120,15 @@ namespace {
 bool jacobi_alternates(artss_ctx *ctx, int ft) {
     if (ctx->alternates[ft] && ctx->alternates_version[ft] == ctx->geom_version) return ctx->alternates[ft] > 0;
     const Level &L = ctx->lvl[0];
-    const std::vector<bool> &in = ctx->h_inner[0], &dom = ctx->h_domain0;
+    const CellBits &in = ctx->inner_bits[0], &dom = ctx->domain_bits;
     const BcProgram &p = ctx->bc[0][ft];
-    bool ok = (int64_t) in.size() == L.size() && (int64_t) dom.size() == L.size() && (!p.present || p.waves <= 1);
+    bool ok = in.n == L.size() && dom.n == L.size() && (!p.present || p.waves <= 1);
     if (ok) {
-        std::vector<bool> set(in);
-        for (int64_t t : p.h_target) {
-            ok = ok && dom[(size_t) t];
-            set[(size_t) t] = true;
-        }
-        for (int64_t r : p.h_root) ok = ok && dom[(size_t) r];
-        const int64_t off[6] = {-1, 1, -L.Nx, L.Nx, -L.nxy(), L.nxy()};
-        for (int64_t q = 0; q < L.size() && ok; q++) {
-            ok = dom[(size_t) q] == set[(size_t) q];
-            if (in[(size_t) q])
-                for (int64_t d : off) ok = ok && dom[(size_t) (q + d)];
-        }
+        CellBits set = in;
+        for (int64_t t : p.h_target) set.set(t);
+        for (int64_t r : p.h_root) ok = ok && dom.get(r);
+        ok = ok && set.w == dom.w;
+        for (int64_t d : {(int64_t) -1, (int64_t) 1, -L.Nx, L.Nx, -L.nxy(), L.nxy()}) ok = ok && in.neighbours_in(dom, d);
     }
     ctx->alternates[ft] = ok ? 1 : -1;
     ctx->alternates_version[ft] = ctx->geom_version;
