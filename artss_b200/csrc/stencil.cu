@@ -333,31 +333,16 @@ __device__ __forceinline__ void turb_alpha(const DiffCoef &c, double ev, double 
 // two-colour sweep: red cells read only black neighbours (old), black cells
 // read only red neighbours (new).
 //
-// A block owns a tile of kSwTx x kSwTy columns over kSwZ planes and marches
-// up in z.  At plane step k it computes red on plane k for the tile plus a
-// one-cell ring (the ring's red values feed the tile's black cells; they are
-// recomputed, never written), then black on plane k-1 for the tile, and
-// writes plane k-1 of the tile to `out`.  Planes of `in`, `b` and `EV` (tile
-// plus a two-cell ring) stream through shared-memory ring buffers by
-// cp.async, kSwD planes ahead of use; a tile's red values replace the old
-// ones in the `in` plane buffer, since only black cells read them afterwards.
+// The marching kernels: a block owns a tile of kSwTx x kSwTy columns over some
+// planes and marches up in z.  At plane step k it computes red on plane k for the
+// tile plus a one-cell ring (the ring's red values feed the tile's black cells; they
+// are recomputed, never written), then black on an earlier plane for the tile, and
+// writes that plane to `out`.  Planes of `in`, `b` and `EV` (tile plus ring) stream
+// through shared-memory ring buffers ahead of use; a tile's red values replace the
+// old ones in the `in` plane buffer, since only black cells read them afterwards.
 // Non-inner cells of the tile are copied from `in`; the boundary program
 // rewrites the ones anything reads.
-constexpr int kSwTx = 64, kSwTy = 8, kSwZ = 16, kSwD = 2;
-constexpr int kSwThreads = (kSwTx / 2) * kSwTy;            // one thread per x-pair of the tile
-constexpr int kSwWx = kSwTx + 4, kSwWy = kSwTy + 4;         // staged window: tile + 2-cell ring
-constexpr int kSwPlane = kSwWx * kSwWy;
-constexpr int kSwSlotsX = kSwD + 4;                         // x planes k-2 .. k+1+D
-constexpr int kSwSlotsB = kSwD + 3;                         // b / EV planes k-1 .. k+1+D
-constexpr int kSwRedPairs = ((kSwTx + 2) / 2) * (kSwTy + 2);  // x-pairs of the tile + 1-cell ring
-
-inline dim3 sweep_grid(const Box3 &b) {
-    return dim3((unsigned) ((b.nx() + kSwTx - 1) / kSwTx), (unsigned) ((b.ny() + kSwTy - 1) / kSwTy),
-                (unsigned) ((b.nz() + kSwZ - 1) / kSwZ));
-}
-inline size_t sweep_smem(bool turb) {
-    return sizeof(double) * (size_t) kSwPlane * (kSwSlotsX + (turb ? 2 : 1) * kSwSlotsB);
-}
+constexpr int kSwTx = 64, kSwTy = 8, kSwD = 2;  // tile; planes staged ahead
 
 __device__ __forceinline__ void cp_async8(double *dst, const double *src) {
     const unsigned d = (unsigned) __cvta_generic_to_shared(dst);
@@ -367,133 +352,139 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
+// ---- the sweep on small blocks of cells --------------------------------------
+//
+// A block of 256 threads owns 32 x 8 x 4 cells: the old values of the block and a
+// two-cell ring arrive in shared memory at once, red runs on the block and a
+// one-cell ring (in place: red cells read black ones only), black on the block, and
+// the block is written.  Twice the red work of a march, but a level of 64^3 cells
+// is 256 blocks whose loads are all in flight together, where the marching kernels
+// have 64 blocks of 12 dependent planes.  Any row pitch and alignment.  A sweep
+// between events, turbulent: 64^3 12.9 us against 18.9 of the best march, 96^3 23
+// against 22, 256 x 128 x 128 78 against 52; on odd pitches, where a march fed by
+// cp.async was the only one, 161 x 97 x 49 25 against 44, 255 x 127 x 127 76 against
+// 105.
+constexpr int kSbX = 32, kSbY = 8, kSbZ = 4, kSbThreads = 256;
+constexpr int kSbWx = kSbX + 4, kSbWy = kSbY + 4, kSbWz = kSbZ + 4;           // staged window
+constexpr int kSbPairs = (kSbX + 2) / 2, kSbRed = kSbPairs * (kSbY + 2) * (kSbZ + 2);
+constexpr int kSbBlack = kSbX / 2 * kSbY * kSbZ;
+constexpr int kSbRedU = (kSbRed + kSbThreads - 1) / kSbThreads, kSbBlackU = kSbBlack / kSbThreads;
+constexpr int kSbMaxBlocks = 8192;  // blocks of a launch, one partial sum each; they loop over further tiles
+
+inline int64_t sweep_block_tiles(const Box3 &b) {
+    return ((b.nx() + kSbX - 1) / kSbX) * ((b.ny() + kSbY - 1) / kSbY) * ((b.nz() + kSbZ - 1) / kSbZ);
+}
+
 template <bool TURB>
-__global__ void __launch_bounds__(kSwThreads, 2)
-k_cgs_sweep(double *__restrict__ out, const double *__restrict__ in, const double *__restrict__ b,
-            const double *__restrict__ ev, const uint8_t *__restrict__ flags, Level L, Box3 box, DiffCoef c,
-            double *__restrict__ partials, const LoopState *__restrict__ pred) {
-    extern __shared__ double sw[];
+__global__ void __launch_bounds__(kSbThreads, 4)
+k_cgs_sweep_block(double *__restrict__ out, const double *__restrict__ in, const double *__restrict__ b,
+                  const double *__restrict__ ev, const uint8_t *__restrict__ flags, Level L, Box3 box, DiffCoef c,
+                  int ntx, int nty, int tiles, double *__restrict__ partials, const LoopState *__restrict__ pred) {
+    __shared__ double X[kSbWz * kSbWy * kSbWx];
     __shared__ double smem[32];
+    pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
+    pdl_trigger();
     if (pred && !pred->cond) return;  // iteration enqueued past convergence
-    if (blockDim.x != kSwTx / 2 || blockDim.y != kSwTy || blockDim.z != 1) return;  // launch shape is fixed
-    double *X = sw;                                  // [kSwSlotsX][kSwPlane]
-    double *B = sw + kSwSlotsX * kSwPlane;           // [kSwSlotsB][kSwPlane]
-    double *E = B + kSwSlotsB * kSwPlane;            // [kSwSlotsB][kSwPlane] (TURB)
-    const int tid = threadIdx.x + (kSwTx / 2) * threadIdx.y;
-    const int64_t nj = L.Nx, nk = L.nxy();
-    const int64_t wx0 = box.x0 + (int64_t) blockIdx.x * kSwTx - 2;  // global i of window column 0
-    const int64_t wy0 = box.y0 + (int64_t) blockIdx.y * kSwTy - 2;
-    const int64_t kc0 = box.z0 + (int64_t) blockIdx.z * kSwZ;
-    const int64_t kc1 = min(kc0 + kSwZ - 1, box.z1);
-
-    // stage plane p of x, b (and EV) into their ring slots; one commit group per plane
-    auto stage = [&](int64_t p) {
-        // planes kc0-2 .. kc1+2 are read; the ring is kept in step past them
-        if (p >= 0 && p < L.Nz && p <= kc1 + 2) {
-            double *xs = X + (int) ((p - kc0 + 2 + 2 * kSwSlotsX) % kSwSlotsX) * kSwPlane;
-            double *bs = B + (int) ((p - kc0 + 2 + 2 * kSwSlotsB) % kSwSlotsB) * kSwPlane;
-            double *es = E + (int) ((p - kc0 + 2 + 2 * kSwSlotsB) % kSwSlotsB) * kSwPlane;
-            for (int e = tid; e < kSwPlane; e += kSwThreads) {
-                const int ly = e / kSwWx, lx = e - ly * kSwWx;
-                const int64_t gi = wx0 + lx, gj = wy0 + ly;
-                if (gi < 0 || gi >= L.Nx || gj < 0 || gj >= L.Ny) continue;
-                const int64_t q = gi + nj * gj + nk * p;
-                cp_async8(xs + e, in + q);
-                // b and EV are read on the tile and its 1-cell ring only
-                if (lx >= 1 && lx <= kSwTx + 2 && ly >= 1 && ly <= kSwTy + 2) {
-                    cp_async8(bs + e, b + q);
-                    if (TURB) cp_async8(es + e, ev + q);
-                }
-            }
-        }
-        cp_async_commit();
-    };
-    auto xslot = [&](int64_t p) { return X + ((unsigned) (p - kc0 + 2) % (unsigned) kSwSlotsX) * kSwPlane; };
-    auto bslot = [&](int64_t p) { return (int) (((unsigned) (p - kc0 + 2) % (unsigned) kSwSlotsB) * kSwPlane); };
-
-    // one stencil update; returns the new value and the residual term
-    auto update = [&](const double *xm, const double *x0, const double *xp, int e, int bo, double &res2) {
+    const int tid = threadIdx.x;
+    // 32-bit indices: artss_ctx_create rejects levels of 2^31 cells or more
+    const int Nx = (int) L.Nx, Ny = (int) L.Ny, Nz = (int) L.Nz, nj = Nx, nk = (int) L.nxy();
+    const int bx0 = (int) box.x0, bx1 = (int) box.x1, by0 = (int) box.y0, by1 = (int) box.y1;
+    const int bz0 = (int) box.z0, bz1 = (int) box.z1;
+    auto update = [&](int e, double bv, double e_, double &res2) {
         double ax = c.ax, ay = c.ay, az = c.az, beta = c.beta, rb = c.rbeta;
         if (TURB) {
-            turb_alpha(c, E[bo + e], ax, ay, az, rb);
+            turb_alpha(c, e_, ax, ay, az, rb);
             beta = 1. / rb;
         }
-        const double old = x0[e];
-        const double out_h = beta * (c.dsign * B[bo + e] + ax * (x0[e + 1] + x0[e - 1]) +
-                                     ay * (x0[e + kSwWx] + x0[e - kSwWx]) + az * (xp[e] + xm[e]));
+        const double old = X[e];
+        const double out_h = beta * (c.dsign * bv + ax * (X[e + 1] + X[e - 1]) + ay * (X[e + kSbWx] + X[e - kSbWx]) +
+                                     az * (X[e + kSbWx * kSbWy] + X[e - kSbWx * kSbWy]));
         const double nw = c.omw * old + c.w * out_h;
         const double r = rb * (nw - old);
         res2 = r * r;
         return nw;
     };
-
-    for (int64_t p = kc0 - 2; p <= kc0 - 1 + kSwD; p++) stage(p);
     double acc = 0.0;
-    for (int64_t k = kc0 - 1; k <= kc1 + 1; k++) {
-        cp_async_wait<kSwD - 1>();  // planes up to k+1 have landed
-        __syncthreads();            // ... and step k-1 is done with the slots refilled next
-        stage(k + 1 + kSwD);
-        // red on plane k, tile + 1-cell ring
-        if (k >= box.z0 && k <= box.z1) {
-            const double *xm = xslot(k - 1), *xp = xslot(k + 1);
-            double *x0 = xslot(k);
-            const int bo = bslot(k);
-            for (int pr = tid; pr < kSwRedPairs; pr += kSwThreads) {
-                const int ry = 1 + pr / ((kSwTx + 2) / 2);
-                const int px = pr - (ry - 1) * ((kSwTx + 2) / 2);
-                const int64_t gj = wy0 + ry;
-                const int rx = 1 + 2 * px + (int) ((wx0 + 1 + gj + k) & 1);  // (i + j + k) even
-                const int64_t gi = wx0 + rx;
-                if (gi < box.x0 || gi > box.x1 || gj < box.y0 || gj > box.y1) continue;
-                if (!(__ldg(flags + gi + nj * gj + nk * k) & kInner)) continue;
-                const int e = rx + kSwWx * ry;
-                double r2;
-                const double nw = update(xm, x0, xp, e, bo, r2);
-                x0[e] = nw;
-                if (rx >= 2 && rx < kSwTx + 2 && ry >= 2 && ry < kSwTy + 2 && k >= kc0 && k <= kc1) acc += r2;
-            }
+    for (int tile = (int) blockIdx.x; tile < tiles; tile += (int) gridDim.x) {
+        // the window's first cell
+        const int wx = bx0 + tile % ntx * kSbX - 2, wy = by0 + tile / ntx % nty * kSbY - 2,
+                  wz = bz0 + tile / (ntx * nty) * kSbZ - 2;
+        for (int e = tid; e < kSbWx * kSbWy * kSbWz; e += kSbThreads) {
+            const int gi = wx + e % kSbWx, gj = wy + e / kSbWx % kSbWy, gk = wz + e / (kSbWx * kSbWy);
+            if (gi >= 0 && gi < Nx && gj >= 0 && gj < Ny && gk >= 0 && gk < Nz) cp_async8(X + e, in + gi + nj * gj + nk * gk);
         }
-        __syncthreads();
-        // black on plane k-1, tile only, and the tile's plane k-1 out
-        const int64_t kb = k - 1;
-        if (kb >= kc0 && kb <= kc1) {
-            const double *xm = xslot(kb - 1), *xp = xslot(kb + 1);
-            const double *x0 = xslot(kb);
-            const int bo = bslot(kb);
-            const int ty = threadIdx.y, tx = threadIdx.x;
-            const int64_t gj = wy0 + 2 + ty;
-            const int lx0 = 2 + 2 * tx;
-            const int par = (int) ((wx0 + lx0 + gj + kb + 1) & 1);  // (i + j + k) odd
-            const int e0 = lx0 + kSwWx * (2 + ty);
-            if (gj <= box.y1) {
+        // this thread's red and black cells: window offset (0: none), b and EV
+        int er[kSbRedU], eb[kSbBlackU];
+        double rb_[kSbRedU], re_[kSbRedU], bb_[kSbBlackU], be_[kSbBlackU];
+        unsigned tile_red = 0;
 #pragma unroll
-                for (int s = 0; s < 2; s++) {
-                    const int64_t gi = wx0 + lx0 + s;
-                    if (gi > box.x1) continue;
-                    const int64_t q = gi + nj * gj + nk * kb;
-                    double v = x0[e0 + s];
-                    if (s == par && (__ldg(flags + q) & kInner)) {
-                        double r2;
-                        v = update(xm, x0, xp, e0 + s, bo, r2);
-                        acc += r2;
-                    }
-                    out[q] = v;
-                }
+        for (int u = 0; u < kSbRedU; u++) {
+            const int n = tid + u * kSbThreads, row = n / kSbPairs, ry = 1 + row % (kSbY + 2), rz = 1 + row / (kSbY + 2);
+            const int gj = wy + ry, gk = wz + rz;
+            const int rx = 1 + 2 * (n % kSbPairs) + ((wx + 1 + gj + gk) & 1);  // (i + j + k) even
+            const int gi = wx + rx, q = gi + nj * gj + nk * gk;
+            er[u] = 0;
+            rb_[u] = re_[u] = 0.0;
+            if (n < kSbRed && gi >= bx0 && gi <= bx1 && gj >= by0 && gj <= by1 && gk >= bz0 && gk <= bz1 &&
+                (__ldg(flags + q) & kInner)) {
+                er[u] = rx + kSbWx * (ry + kSbWy * rz);
+                rb_[u] = b[q];
+                if (TURB) re_[u] = ev[q];
+                if (rx >= 2 && rx < kSbX + 2 && ry >= 2 && ry < kSbY + 2 && rz >= 2 && rz < kSbZ + 2) tile_red |= 1u << u;
             }
         }
+#pragma unroll
+        for (int u = 0; u < kSbBlackU; u++) {
+            const int n = tid + u * kSbThreads, row = n / (kSbX / 2), ty = 2 + row % kSbY, tz = 2 + row / kSbY;
+            const int gj = wy + ty, gk = wz + tz;
+            const int tx = 2 + 2 * (n % (kSbX / 2)) + ((wx + 3 + gj + gk) & 1);  // (i + j + k) odd
+            const int gi = wx + tx, q = gi + nj * gj + nk * gk;
+            eb[u] = 0;
+            bb_[u] = be_[u] = 0.0;
+            if (gi <= bx1 && gj <= by1 && gk <= bz1 && (__ldg(flags + q) & kInner)) {
+                eb[u] = tx + kSbWx * (ty + kSbWy * tz);
+                bb_[u] = b[q];
+                if (TURB) be_[u] = ev[q];
+            }
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kSbRedU; u++)
+            if (er[u]) {
+                double r2;
+                X[er[u]] = update(er[u], rb_[u], re_[u], r2);
+                if (tile_red >> u & 1) acc += r2;
+            }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kSbBlackU; u++)
+            if (eb[u]) {
+                double r2;
+                X[eb[u]] = update(eb[u], bb_[u], be_[u], r2);
+                acc += r2;
+            }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kSbX * kSbY * kSbZ / kSbThreads; u++) {
+            const int n = tid + u * kSbThreads, tx = n % kSbX, ty = n / kSbX % kSbY, tz = n / (kSbX * kSbY);
+            const int gi = wx + 2 + tx, gj = wy + 2 + ty, gk = wz + 2 + tz;
+            if (gi <= bx1 && gj <= by1 && gk <= bz1) out[gi + nj * gj + nk * gk] = X[tx + 2 + kSbWx * (ty + 2 + kSbWy * (tz + 2))];
+        }
+        if (tile + (int) gridDim.x < tiles) __syncthreads();  // the window is refilled
     }
-    cp_async_wait<0>();
     acc = artss_block_sum(acc, smem);
-    if (partials && tid == 0) partials[block_linear()] = acc;
+    if (partials && tid == 0) partials[blockIdx.x] = acc;
 }
 
-// ---- the same sweep with TMA plane staging -------------------------------
+// ---- the marching sweep with TMA plane staging -------------------------------
 //
 // One thread issues, per z-plane, one cp.async.bulk.tensor load of the
 // kTmaBoxX x kTmaBoxY window of x, b (and EV) into the plane's ring slot;
 // the loads complete on the slot's mbarrier.  The window starts at an even x
 // (a TMA box must start on a 16-byte boundary), so the tile sits ox = 0 or 1
-// cells further right in it than in the cp.async variant.  Red work is one
+// cells right of the ring's first column.  Red work is one
 // x-pair per thread (33 x 10 pairs: tile plus ring), black one x-pair per
 // thread of the first 256.  Waits on an mbarrier give up after a bounded
 // number of polls and raise the loop state's error flag instead of hanging.
@@ -1675,8 +1666,10 @@ namespace {
 // variant number of k_cgs_sweep3 with 64 x 8 tiles; + 1: 64 x 6 tiles; + 2: 64 x 16
 // tiles, one block per multiprocessor
 constexpr int kSweepRowPair = 6;
-constexpr int kSweepVariants = kSweepRowPair + 3;
+constexpr int kSweepBlock = kSweepRowPair + 3;  // k_cgs_sweep_block
+constexpr int kSweepVariants = kSweepBlock + 1;
 struct SweepMaps {
+    const double *px = nullptr, *pb = nullptr, *pe = nullptr;
     const CUtensorMap *x = nullptr, *b = nullptr, *e = nullptr;
     const CUtensorMap *x2 = nullptr, *b2 = nullptr, *e2 = nullptr;
     const CUtensorMap *x3 = nullptr, *b3 = nullptr, *e3 = nullptr;  // 72 x 10 and 66 x 8 windows
@@ -1752,13 +1745,26 @@ int launch_sweep3(artss_ctx *ctx, bool turb, int t, const Box3 &box, const CUten
 // Variants of the TMA sweep: v < 3 the kernel with two barriers per plane step
 // and z-depth kStDepths[v]; 3 <= v < 6 the one-phase kernel with
 // kStDepths[v - 3]; v = 6, 7 the row-pair kernel with 64 x 8 and 64 x 6 tiles; v >= 3 only
-// where the b / EV window starts at an even x.  Returns the number of blocks
-// (partials) in *nb.
-int launch_sweep_tma(artss_ctx *ctx, bool turb, int v, const Box3 &box, const SweepMaps &m, double *w,
+// where the b / EV window starts at an even x; v = kSweepBlock the block kernel, on
+// any level.  Returns the number of blocks (partials) in *nb.
+int launch_sweep(artss_ctx *ctx, bool turb, int v, const Box3 &box, const SweepMaps &m, double *w,
                      const Level &L, const DiffCoef &c, LoopState *pred, int *nb) {
     if (v == kSweepRowPair) return launch_sweep3<S3Tall>(ctx, turb, 0, box, m.x, m.b2, m.e2, w, L, c, pred, nb);
     if (v == kSweepRowPair + 1) return launch_sweep3<S3Flat>(ctx, turb, 1, box, m.x3, m.b3, m.e3, w, L, c, pred, nb);
     if (v == kSweepRowPair + 2) return launch_sweep3<S3Wide>(ctx, turb, 2, box, m.x4, m.b4, m.e4, w, L, c, pred, nb);
+    if (v == kSweepBlock) {
+        const int ntx = (int) ((box.nx() + kSbX - 1) / kSbX), nty = (int) ((box.ny() + kSbY - 1) / kSbY);
+        const int tiles = (int) sweep_block_tiles(box);
+        *nb = std::min(tiles, kSbMaxBlocks);
+        if (turb)
+            ARTSS_LAUNCH_PDL(ctx, FAM_CGS, k_cgs_sweep_block<true>, dim3((unsigned) *nb), kSbThreads, 0, w, m.px, m.pb, m.pe,
+                             (const uint8_t *) ctx->d_flags[0], L, box, c, ntx, nty, tiles, ctx->d_partials, pred);
+        else
+            ARTSS_LAUNCH_PDL(ctx, FAM_CGS, k_cgs_sweep_block<false>, dim3((unsigned) *nb), kSbThreads, 0, w, m.px, m.pb, m.pe,
+                             (const uint8_t *) ctx->d_flags[0], L, box, c, ntx, nty, tiles, ctx->d_partials, pred);
+        ARTSS_LAUNCH_CK(ctx);
+        return ARTSS_OK;
+    }
     const int zb = kStDepths[v % 3];
     const dim3 g = sweep_tma_grid(box, zb);
     *nb = nblocks(g);
@@ -1821,10 +1827,17 @@ int set_sweep_smem(bool turb) {
 // variant (kernel and z-depth) on that solve's first iteration (the sweep
 // reads `rd`, b, EV and writes only `w` and the partials, so repeating it
 // changes nothing) and keeps the fastest for the context.
-int tune_sweep(artss_ctx *ctx, bool turb, bool one_phase, const Box3 &box, const SweepMaps &m, double *w,
+// A call that may not tune takes the block kernel on levels whose marching kernels
+// would not fill the chip (they are level at 96^3 cells), else the row-pair one.
+constexpr int64_t kSweepBlockCells = 1000 * 1000;
+int tune_sweep(artss_ctx *ctx, bool turb, bool tma, bool one_phase, const Box3 &box, const SweepMaps &m, double *w,
                const Level &L, const DiffCoef &c, LoopState *pred, int *choice) {
+    if (!tma) {  // the marching kernels need TMA
+        *choice = kSweepBlock;
+        return ARTSS_OK;
+    }
     if (ctx->sweep_force >= 0) {
-        if (ctx->sweep_force >= 3 && !one_phase) {
+        if (ctx->sweep_force >= 3 && ctx->sweep_force != kSweepBlock && !one_phase) {
             set_error("sweep variant needs an inner box starting at an odd x");
             return ARTSS_ERR_ARG;
         }
@@ -1833,18 +1846,22 @@ int tune_sweep(artss_ctx *ctx, bool turb, bool one_phase, const Box3 &box, const
     }
     const TuneKey key{0, L.Nx, L.Ny, L.Nz, turb ? 1 : 0};
     auto it = ctx->tuned.find(key);
-    if (it != ctx->tuned.end() && (one_phase || it->second < 3)) { *choice = it->second; return ARTSS_OK; }
-    const int fallback = one_phase ? kSweepRowPair : 1;
+    if (it != ctx->tuned.end() && (one_phase || it->second < 3 || it->second == kSweepBlock)) {
+        *choice = it->second;
+        return ARTSS_OK;
+    }
+    const int fallback = box.nx() * box.ny() * box.nz() < kSweepBlockCells ? kSweepBlock : one_phase ? kSweepRowPair : 1;
     if (!ctx->autotune || ctx->capturing) { *choice = fallback; return ARTSS_OK; }
     cudaEvent_t e0, e1;
     ARTSS_CK(cudaEventCreate(&e0));
     ARTSS_CK(cudaEventCreate(&e1));
     int best = fallback, st = ARTSS_OK, nb = 0;
     float best_ms = 1e30f;
-    for (int v = 0; v < (one_phase ? kSweepVariants : 3) && !st; v++) {
-        if ((st = launch_sweep_tma(ctx, turb, v, box, m, w, L, c, pred, &nb))) break;  // warm
+    for (int v = 0; v < kSweepVariants && !st; v++) {
+        if (v >= 3 && v != kSweepBlock && !one_phase) continue;
+        if ((st = launch_sweep(ctx, turb, v, box, m, w, L, c, pred, &nb))) break;  // warm
         cudaEventRecord(e0, ctx->stream);
-        for (int r = 0; r < 3 && !st; r++) st = launch_sweep_tma(ctx, turb, v, box, m, w, L, c, pred, &nb);
+        for (int r = 0; r < 3 && !st; r++) st = launch_sweep(ctx, turb, v, box, m, w, L, c, pred, &nb);
         cudaEventRecord(e1, ctx->stream);
         if (cudaEventSynchronize(e1) != cudaSuccess) { st = cuda_fail(cudaGetLastError(), "autotune"); break; }
         float ms = 0;
@@ -1877,7 +1894,7 @@ int artss_ctx_pdl(artss_ctx *ctx, int enable) {
 
 int artss_ctx_sweep_variant(artss_ctx *ctx, int variant) {
     if (!ctx) { set_error("null argument"); return ARTSS_ERR_ARG; }
-    if (variant < -1 || variant >= kSweepVariants) { set_error("sweep variant is -1 .. 8"); return ARTSS_ERR_ARG; }
+    if (variant < -1 || variant >= kSweepVariants) { set_error("sweep variant is -1 .. 9"); return ARTSS_ERR_ARG; }
     ctx->sweep_force = variant;
     return ARTSS_OK;
 }
@@ -1906,18 +1923,12 @@ int artss_diffuse_cgs(artss_ctx *ctx, double *out, double *in, const double *b, 
     if (out == in || b == out || b == in) { set_error("out, in and b must be distinct arrays"); return ARTSS_ERR_ARG; }
     const Level &L = ctx->lvl[0];
     const Box3 box = inner_box(L);
-    const dim3 g = sweep_grid(box);
-    if ((st = check_reduce_blocks(g))) return st;
-    if ((st = check_reduce_blocks(sweep_tma_grid(box, kStDepths[0])))) return st;
-    int nb = nblocks(g);
-    // TMA plane staging where the row pitch allows it, cp.async otherwise
+    int nb = 0;
+    // the marching kernels stage planes by TMA where the row pitch allows it
     const bool tma = tma_level_ok(ctx, 0) && L.size() < ((int64_t) 1 << 31);
-    const size_t smem = tma ? sweep_tma_smem(ev != nullptr) : sweep_smem(ev != nullptr);
     if (tma) {
+        if ((st = check_reduce_blocks(sweep_tma_grid(box, kStDepths[0])))) return st;
         if ((st = set_sweep_smem(ev != nullptr))) return st;
-    } else {
-        if (ev) ARTSS_CK(cudaFuncSetAttribute(k_cgs_sweep<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-        else ARTSS_CK(cudaFuncSetAttribute(k_cgs_sweep<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
     }
     // one-phase kernel: its b / EV window starts at an even x when the inner box starts at an odd one
     const bool one_phase = tma && (box.x0 & 1) == 1;
@@ -1942,6 +1953,11 @@ int artss_diffuse_cgs(artss_ctx *ctx, double *out, double *in, const double *b, 
     // chosen so that a solve of the predicted length ends in out.
     double *buf[2] = {out, in};
     const int s0 = (int) (batch & 1);  // iteration n writes buf[(s0 + n) & 1]
+    for (int r = 0; r < 2; r++) {
+        maps[r].px = buf[r];
+        maps[r].pb = b;
+        maps[r].pe = ev;
+    }
     if (tma) {
         for (int r = 0; r < 2; r++) {
             SweepMaps &m = maps[r];
@@ -1965,10 +1981,10 @@ int artss_diffuse_cgs(artss_ctx *ctx, double *out, double *in, const double *b, 
             }
         }
     }
-    int depth = 1;  // the sweep variant (launch_sweep_tma)
-    if (tma && cond) {
+    int depth = 1;  // the sweep variant (launch_sweep)
+    if (cond) {
         const int n1 = (s0 + 1) & 1;
-        if ((st = tune_sweep(ctx, ev != nullptr, one_phase, box, maps[1 - n1], buf[n1], L, c, state(1), &depth)))
+        if ((st = tune_sweep(ctx, ev != nullptr, tma, one_phase, box, maps[1 - n1], buf[n1], L, c, state(1), &depth)))
             return st;
     }
     if (ctx->capturing) {
@@ -1979,18 +1995,8 @@ int artss_diffuse_cgs(artss_ctx *ctx, double *out, double *in, const double *b, 
             if ((st = gl.begin(ctx, 1))) return st;
             for (int n = 1; n <= 2; n++) {
                 double *w = buf[(s0 + n) & 1];
-                const double *rd = buf[(s0 + n + 1) & 1];
-                if (tma) {
-                    if ((st = launch_sweep_tma(ctx, ev != nullptr, depth, box, maps[(s0 + n + 1) & 1], w, L, c,
-                                               state(n), &nb)))
-                        return st;
-                } else if (ev)
-                    ARTSS_LAUNCH(ctx, FAM_CGS, k_cgs_sweep<true><<<g, dim3(kSwTx / 2, kSwTy), smem, ctx->stream>>>(
-                        w, rd, b, ev, ctx->d_flags[0], L, box, c, ctx->d_partials, state(n)));
-                else
-                    ARTSS_LAUNCH(ctx, FAM_CGS, k_cgs_sweep<false><<<g, dim3(kSwTx / 2, kSwTy), smem, ctx->stream>>>(
-                        w, rd, b, nullptr, ctx->d_flags[0], L, box, c, ctx->d_partials, state(n)));
-                if (!tma) ARTSS_LAUNCH_CK(ctx);
+                if ((st = launch_sweep(ctx, ev != nullptr, depth, box, maps[(s0 + n + 1) & 1], w, L, c, state(n), &nb)))
+                    return st;
                 if ((st = apply_bc_step(ctx, w, 0, field_type, slot, (n - 1) & 1, nb, cfg->tol_res, cfg->max_iter)))
                     return st;
             }
@@ -2008,18 +2014,7 @@ int artss_diffuse_cgs(artss_ctx *ctx, double *out, double *in, const double *b, 
         for (int64_t r = 0; r < batch; r++) {
             const long long n = it + 1 + r;
             double *w = buf[(s0 + n) & 1];
-            const double *rd = buf[(s0 + n + 1) & 1];
-            if (tma) {
-                if ((st = launch_sweep_tma(ctx, ev != nullptr, depth, box, maps[(s0 + n + 1) & 1], w, L, c, state(n),
-                                           &nb)))
-                    return st;
-            } else if (ev)
-                ARTSS_LAUNCH(ctx, FAM_CGS, k_cgs_sweep<true><<<g, dim3(kSwTx / 2, kSwTy), smem, ctx->stream>>>(
-                    w, rd, b, ev, ctx->d_flags[0], L, box, c, ctx->d_partials, state(n)));
-            else
-                ARTSS_LAUNCH(ctx, FAM_CGS, k_cgs_sweep<false><<<g, dim3(kSwTx / 2, kSwTy), smem, ctx->stream>>>(
-                    w, rd, b, nullptr, ctx->d_flags[0], L, box, c, ctx->d_partials, state(n)));
-            if (!tma) ARTSS_LAUNCH_CK(ctx);
+            if ((st = launch_sweep(ctx, ev != nullptr, depth, box, maps[(s0 + n + 1) & 1], w, L, c, state(n), &nb))) return st;
             if ((st = apply_bc_step(ctx, w, 0, field_type, slot, (int) ((n - 1) & 1), nb, cfg->tol_res, cfg->max_iter)))
                 return st;
         }

@@ -348,12 +348,13 @@ int artss_cgs_sweep_depth(artss_ctx *ctx, int turbulent);
 /* the tuned sweep variant of level 0 (0-2: two-phase kernel of z-depth 8,
  * 16, 32; 3-5: one-phase kernel; 6-8: row-pair kernel with persistent
  * blocks: 64 x 8 and 64 x 6 tiles two blocks per multiprocessor, 64 x 16
- * tiles one block), -1 before the first solve; artss_cgs_sweep_depth
- * returns -1 for variants 6-8 */
+ * tiles one block; 9: blocks of 32 x 8 x 4 cells), -1 before the first solve;
+ * artss_cgs_sweep_depth returns -1 for variants 6-9 */
 int artss_cgs_sweep_variant(artss_ctx *ctx, int turbulent);
-/* Pins the colored Gauss-Seidel sweep variant of artss_diffuse_cgs (0-8 as
- * above; 3-8 need an inner box that starts at an odd x), -1 (default): the
- * autotuner's choice.  No counterpart in the reference. */
+/* Pins the colored Gauss-Seidel sweep variant of artss_diffuse_cgs (0-9 as
+ * above; 3-8 need an inner box that starts at an odd x; a level whose row pitch
+ * is odd always takes 9), -1 (default): the autotuner's choice.  No counterpart
+ * in the reference. */
 int artss_ctx_sweep_variant(artss_ctx *ctx, int variant);
 /* IDiffusion::diffuse, ColoredGaussSeidelDiffuse with FP32 sweeps inside FP64
  * defect correction (no counterpart in the reference; mirrors
