@@ -114,7 +114,7 @@ struct LoopState {
     int cond;          // loop continues
     int pad;           // error flag: a bounded wait in a kernel of the loop gave up (2: a graph loop hit its cap)
     int guard;         // bodies run by a graph loop (conditional node) since the loop's init
-    int unused;
+    int blocks_done;   // blocks done, for a kernel whose last block does the loop step; 0 between launches
 };
 
 // Kernel families for launch counting and event timing (artss_ctx_profile).
@@ -415,7 +415,7 @@ inline dim3 col_grid(const Box3 &b, const ColShape &s) {
 enum ColKernel : int {
     kTuneAdvect1 = 101, kTuneAdvect3, kTuneSmagorinsky, kTuneDivergence, kTuneProjection, kTuneBuoyancy,
     kTuneMgJacobi, kTuneMgResiduum, kTuneMgRestrict, kTuneMgProlongate, kTuneMgJacobi0, kTuneMgDown,
-    kTuneMxJacobi0, kTuneMxJacobi, kTuneMxResiduum, kTuneMxRestrict
+    kTuneMxJacobi0, kTuneMxJacobi, kTuneMxResiduum, kTuneMxRestrict, kTuneMxDown
 };
 
 // Launches a column kernel, `launch(grid, block)` returning a status, with the
@@ -518,8 +518,6 @@ int tensor_map_3d(artss_ctx *ctx, const double *base, int level, const CUtensorM
 //   mode 0: residual = sqrt(sum); it += 1; cond = residual > tol && it < max_it
 int finalize_loop(artss_ctx *ctx, int slot, int nblocks, double tol, long long max_it);
 int init_loop(artss_ctx *ctx, int slot, double residual0, long long it0, int cond0);
-// loop step whose tolerance is rel_tol * sqrt(sum of loop slot ref_slot), on the device
-int finalize_loop_rel(artss_ctx *ctx, int slot, int nblocks, double rel_tol, int ref_slot, long long max_it);
 int read_loop(artss_ctx *ctx, int slot, LoopState *out);
 
 // A loop inside a whole-step capture: a WHILE conditional node whose body is

@@ -28,6 +28,7 @@
 #include "internal.cuh"
 
 #include <algorithm>
+#include <cstdlib>
 #include <unordered_map>
 
 struct artss_mixed {
@@ -41,12 +42,14 @@ struct artss_mixed {
     // the level's homogeneous pressure program applied by the writers of the
     // inner cells instead of by a launch after each sweep (levels 0 .. L-2, when
     // fold[l]): nbm[l][x] bit 0 = inner, bits 1..7 = index of the cell's push
-    // pattern in push[l]; bits 2d .. 2d + 1 of a pattern = what the boundary cell
-    // x + off[d] (d: -x, +x, -y, +y, -z, +z) takes from inner cell x with value v:
-    // 0 nothing, 1 +v, 2 -v
+    // pattern in push[l]; bits 2d .. 2d + 1 of a pattern = what the boundary cell one
+    // step (d % 3 - 1, d / 3 % 3 - 1, d / 9 - 1) away takes from inner cell x with
+    // value v: 0 nothing, 1 +v, 2 -v
     uint8_t *nbm[artss::kMaxLevel + 1]{};
-    uint16_t *push[artss::kMaxLevel + 1]{};  // 128 patterns per level (pattern 0: none)
+    uint64_t *push[artss::kMaxLevel + 1]{};  // 128 patterns per level (pattern 0: none)
     bool fold[artss::kMaxLevel + 1]{};
+    bool whole[artss::kMaxLevel + 1]{};      // the patterns hold the whole program, edges and corners too
+    bool q_bc_dead[artss::kMaxLevel + 1]{};  // the restriction of level l + 1 reads no boundary cell of level l
     uint64_t geom_version = ~0ull;       // ctx->geom_version the tables describe
     int64_t n_inner0 = 0;
     int64_t hint = 1;                    // outer iterations of the last solve
@@ -72,6 +75,10 @@ inline dim3 mx_grid(const Box3 &b) {
     const int j = (int) (box).y0 + (int) (blockIdx.y * blockDim.y + threadIdx.y); \
     const bool col = (i <= (int) (box).x1) && (j <= (int) (box).y1)
 
+// nbm of a boundary cell that takes +-the value of its inner partner in the pair of
+// cells 2 n, 2 n + 1 (kept out of the partner's pattern)
+constexpr unsigned kPartnerPlus = 2, kPartnerMinus = 4;
+
 struct CoefF {
     float ax, ay, az, beta, w, omw;
 };
@@ -79,28 +86,32 @@ struct CoefF {
 // weighted Jacobi sweep of the pressure operator (the multigrid variant of
 // JacobiDiffuse::JacobiStep, dsign = -1), FP32
 // store v at inner cell x and the boundary cells whose homogeneous program
-// value is +-x (push bits of the neighbour mask)
-__device__ __forceinline__ void mx_store(float *__restrict__ out, uint8_t mask, const uint16_t *__restrict__ push,
-                                         int x, float v, int nj, int nk) {
-    out[x] = v;
-    if (mask >> 1) {
-        const unsigned mm = __ldg(push + (mask >> 1));
-        const int off[6] = {-1, 1, -nj, nj, -nk, nk};
-#pragma unroll
-        for (int d = 0; d < 6; d++) {
-            const unsigned kind = (mm >> (2 * d)) & 3u;
-            if (kind) out[x + off[d]] = kind == 1u ? v : -v;
-        }
+// value is +-x (the cell's push pattern)
+template <class T>
+__device__ __forceinline__ void mx_push(T *__restrict__ out, unsigned mask, const uint64_t *__restrict__ push, int x, T v,
+                                        int nj, int nk) {
+    uint64_t mm = __ldg((const unsigned long long *) push + (mask >> 1));
+    while (mm) {
+        const int d = (__ffsll((long long) mm) - 1) >> 1;
+        out[x + (d % 3 - 1) + nj * (d / 3 % 3 - 1) + nk * (d / 9 - 1)] = (mm >> (2 * d)) & 1u ? v : -v;
+        mm &= ~(3ull << (2 * d));
     }
+}
+template <class T>
+__device__ __forceinline__ void mx_store(T *__restrict__ out, uint8_t mask, const uint64_t *__restrict__ push, int x, T v,
+                                         int nj, int nk) {
+    out[x] = v;
+    if (mask >> 1) mx_push(out, mask, push, x, v, nj, nk);
 }
 
 // CORRECT (the last sweep of level 0 in a V-cycle): instead of storing the
 // sweep's value v, add it to the FP64 iterate, p[x] += (double) v, which is
-// k_mx_correct's update of the same value (out and push unused)
+// k_mx_correct's update of the same value (out unused); push_p: p's boundary cells
+// with it, where p's program is homogeneous and wholly in the patterns
 template <bool CORRECT>
 __global__ void __launch_bounds__(256, 8) k_mx_jacobi(float *__restrict__ out, const float *__restrict__ in, const float *__restrict__ b,
-                            const uint8_t *__restrict__ nbm, const uint16_t *__restrict__ push, Level L, Box3 box,
-                            CoefF c, const LoopState *__restrict__ pred, double *__restrict__ p) {
+                            const uint8_t *__restrict__ nbm, const uint64_t *__restrict__ push, Level L, Box3 box,
+                            CoefF c, const LoopState *__restrict__ pred, double *__restrict__ p, int push_p) {
     pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
     pdl_trigger();
     if (pred && !pred->cond) return;
@@ -114,7 +125,7 @@ __global__ void __launch_bounds__(256, 8) k_mx_jacobi(float *__restrict__ out, c
             return c.omw * c0 + c.w * h;
         },
         [&](int x, int, float v, uint8_t fl) {
-            if (CORRECT) p[x] = p[x] + (double) v;
+            if (CORRECT) mx_store(p, push_p ? fl : (uint8_t) 0, push, x, p[x] + (double) v, nj, nk);
             else mx_store(out, fl, push, x, v, nj, nk);
         });
 }
@@ -183,10 +194,44 @@ __global__ void k_mx_restrict(float *__restrict__ out, const float *__restrict__
         [&](int x, int, float v, auto) { out[x] = v; });
 }
 
+// Residual and restriction in one pass: a coarse inner cell takes the mean of its
+// eight children's residuals, each with k_mx_residuum's expression, a child that is
+// not inner counting 0 as in the residual array (q_bc_dead).  Written and read back,
+// with its boundary program between, the residual cost 20 of 28 bytes a fine cell
+// and two more launches.
+__global__ void __launch_bounds__(256) k_mx_residuum_restrict(float *__restrict__ out, const float *__restrict__ e,
+                                                              const float *__restrict__ b,
+                                                              const uint8_t *__restrict__ cflags,
+                                                              const uint8_t *__restrict__ nbm, Level C, Level F, Box3 box,
+                                                              float rx, float ry, float rz,
+                                                              const LoopState *__restrict__ pred) {
+    pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
+    pdl_trigger();
+    if (pred && !pred->cond) return;
+    MX_COLUMN(box);
+    if (!col) return;
+    const int fx = (int) F.Nx, fxy = (int) F.nxy();
+    const int f0 = 2 * i - 1 + fx * (2 * j - 1);
+    for (int k = (int) box.z0 + (int) blockIdx.z; k <= (int) box.z1; k += (int) gridDim.z) {
+        const int q = i + (int) C.Nx * j + (int) C.nxy() * k;
+        if (!(cflags[q] & kInner)) continue;
+        float r[8];
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            const int x = f0 + (c & 1) + fx * ((c >> 1) & 1) + fxy * (2 * k - 1 + (c >> 2));
+            const float c2 = 2.f * e[x];
+            const float v = b[x] - (rx * (e[x - 1] - c2 + e[x + 1]) + ry * (e[x - fx] - c2 + e[x + fx]) +
+                                    rz * (e[x - fxy] - c2 + e[x + fxy]));
+            r[c] = (nbm[x] & kInner) ? v : 0.f;
+        }
+        out[q] = 0.125f * (r[0] + r[1] + r[2] + r[3] + r[4] + r[5] + r[6] + r[7]);
+    }
+}
+
 // first Jacobi sweep from a zero correction: every neighbour is zero, so
 // e = w * beta * (-b) on the inner cells
 __global__ void k_mx_jacobi0(float *__restrict__ out, const float *__restrict__ b, const uint8_t *__restrict__ flags,
-                             const uint16_t *__restrict__ push, Level L, Box3 box, CoefF c,
+                             const uint64_t *__restrict__ push, Level L, Box3 box, CoefF c,
                              const LoopState *__restrict__ pred) {
     pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
     pdl_trigger();
@@ -204,7 +249,7 @@ __global__ void k_mx_jacobi0(float *__restrict__ out, const float *__restrict__ 
 // children of each coarse inner cell, FP32
 __global__ void k_mx_prolong_add(float *__restrict__ fine, const float *__restrict__ in,
                                  const uint8_t *__restrict__ cflags, const uint8_t *__restrict__ fflags,
-                                 const uint16_t *__restrict__ push, Level C, Level F, Box3 fbox,
+                                 const uint64_t *__restrict__ push, Level C, Level F, Box3 fbox,
                                  const LoopState *__restrict__ pred) {
     pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
     pdl_trigger();
@@ -239,7 +284,7 @@ __global__ void k_mx_prolong_add(float *__restrict__ fine, const float *__restri
 __global__ void __launch_bounds__(256) k_mx_prolong_add8(float *__restrict__ fine, const float *__restrict__ in,
                                                          const uint8_t *__restrict__ cflags,
                                                          const uint8_t *__restrict__ fflags,
-                                                         const uint16_t *__restrict__ push, Level C, Level F,
+                                                         const uint64_t *__restrict__ push, Level C, Level F,
                                                          Box3 cbox, Box3 fbox, const LoopState *__restrict__ pred) {
     pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
     pdl_trigger();
@@ -306,16 +351,392 @@ __global__ void __launch_bounds__(256) k_mx_prolong_add8(float *__restrict__ fin
     }
 }
 
-// FP64 outer residual r = b - A p on level 0, stored as the FP32 right-hand
-// side of the correction equation; block partials of ||r||^2
-__global__ void __launch_bounds__(256, 8) k_mx_outer_residual(const double *__restrict__ p, const double *__restrict__ b,
-                                    float *__restrict__ r, const uint8_t *__restrict__ flags, Level L, Box3 box,
-                                    double rx, double ry, double rz, double *__restrict__ partials,
-                                    const LoopState *__restrict__ pred) {
+// Two neighbouring cells of x per thread, for rows of an even number of cells.  A plane
+// is walked as one array, so a warp's 64 cells run on over the ends of rows, whose
+// boundary cells are the 2 of Nx that are worked for nothing; the x neighbours come
+// from the lanes beside, the warp's outer two from memory.
+struct PairPos {
+    int x0, lane;  // first cell within the plane, lane
+    bool live;
+};
+__device__ __forceinline__ PairPos pair_pos(const Box3 &box, int nj) {
+    const int p0 = (int) box.y0 * nj / 2, p1 = ((int) box.y1 + 1) * nj / 2;
+    const int q = p0 + (int) (blockIdx.x * blockDim.x + threadIdx.x);
+    return {2 * min(q, p1 - 1), (int) threadIdx.x & 31, q < p1};
+}
+__device__ __forceinline__ float2 ld2(const float *p) { return *(const float2 *) p; }
+__device__ __forceinline__ double2 ld2(const double *p) { return *(const double2 *) p; }
+// the values left of a pair's first and right of its second cell; edge: the lane's
+// value from memory, for lanes 0 and 31
+template <class T, class T2>
+__device__ __forceinline__ void pair_sides(const T2 &c, T edge, int lane, T *l, T *r) {
+    *l = __shfl_up_sync(~0u, c.y, 1);
+    *r = __shfl_down_sync(~0u, c.x, 1);
+    if (lane == 0) *l = edge;
+    if (lane == 31) *r = edge;
+}
+// store a pair's inner cells, a boundary cell whose root is its partner in the pair
+// (kPartnerPlus, kPartnerMinus) with it, and what the push patterns name.  Half the
+// warps of a row hold one of its ends: by a pattern, those cost more instructions
+// than the sweep.
+template <class T, class T2>
+__device__ __forceinline__ void pair_store(T *__restrict__ out, unsigned fl, const uint64_t *__restrict__ push, int x, T2 v,
+                                           int nj, int nk) {
+    if (fl == 0x0101u) {
+        *(T2 *) (out + x) = v;
+        return;
+    }
+    const unsigned f0 = fl & 0xffu, f1 = fl >> 8;
+    const bool in0 = f0 & 1u, in1 = f1 & 1u;
+    if (!in0) v.x = f0 == kPartnerMinus ? -v.y : v.y;
+    if (!in1) v.y = f1 == kPartnerMinus ? -v.x : v.x;
+    if (f0 && f1) *(T2 *) (out + x) = v;
+    else if (f0) out[x] = v.x;
+    else if (f1) out[x + 1] = v.y;
+    if (in0 && f0 > 1u) mx_push(out, f0, push, x, v.x, nj, nk);
+    if (in1 && f1 > 1u) mx_push(out, f1, push, x + 1, v.y, nj, nk);
+}
+// a pair's flags as those of its inner cells alone: nothing but them is stored
+__device__ __forceinline__ unsigned pair_inner(unsigned fl) { return fl & 0x0101u; }
+
+// A sweep's thread holds kPairPlanes planes with all their loads in flight.  256^3, one
+// sweep / the two of kPairFromZero / the correcting one: 47 / 47 / 65 us here, 60 /
+// 44 + 60 / 95 us by k_mx_jacobi0 and k_mx_jacobi (floors by their bytes: 33 / 23 /
+// 63 us).  4 planes, 256 and 512 threads, a walk up the planes with the next one's
+// loads in flight (53 / 55 / 85 us: a last wave half empty) and 4 cells per thread
+// (61 us) were slower.  What bounds it now is the issue rate (87 % of the slots).
+constexpr int kPairThreads = 128, kPairPlanes = 2;
+
+enum PairMode : int { kPairSweep, kPairCorrect, kPairFromZero };
+
+// k_mx_jacobi on pairs of cells.  kPairFromZero: the first two sweeps from a zero
+// correction in one: the first one's result is e0 = w beta (-b) in inner cells and
+// the same of their roots' b in the boundary cells, which b carries (its writers
+// push it), so the second forms its neighbours from b alone (`in` = b).
+template <int MODE>
+__global__ void __launch_bounds__(kPairThreads) k_mx_jacobi2(float *__restrict__ out, const float *__restrict__ in,
+                                                    const float *__restrict__ b, const uint8_t *__restrict__ nbm,
+                                                    const uint64_t *__restrict__ push, Level L, Box3 box, CoefF c,
+                                                    const LoopState *__restrict__ pred, double *__restrict__ p, int push_p) {
+    pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
+    pdl_trigger();
+    if (pred && !pred->cond) return;
+    const int nj = (int) L.Nx, nk = (int) L.nxy(), z1 = (int) box.z1;
+    const PairPos t = pair_pos(box, nj);
+    constexpr int U = kPairPlanes;
+    const int k0 = (int) box.z0 + (int) blockIdx.y * U;
+    float2 cc[U + 2], ym[U], yp[U], bb[U];
+    float edge[U];
+    unsigned fl[U];
+    double2 pp[U];
+    const bool p2 = (uintptr_t) p % 16 == 0;
+#pragma unroll
+    for (int u = 0; u < U + 2; u++) cc[u] = ld2(in + t.x0 + nk * min(k0 - 1 + u, z1 + 1));
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int x = t.x0 + nk * min(k0 + u, z1);
+        fl[u] = *(const uint16_t *) (nbm + x);
+        ym[u] = ld2(in + x - nj);
+        yp[u] = ld2(in + x + nj);
+        if (MODE != kPairFromZero) bb[u] = ld2(b + x);
+        edge[u] = 0.f;
+        if (t.lane == 0 || t.lane == 31) edge[u] = in[x + (t.lane ? 2 : -1)];
+        if (MODE == kPairCorrect) pp[u] = p2 ? ld2(p + x) : make_double2(p[x], p[x + 1]);
+    }
+    asm volatile("" ::: "memory");  // every load issued before the arithmetic
+    const auto val = [&](float v) { return MODE == kPairFromZero ? c.w * (c.beta * -v) : v; };
+    if (MODE == kPairFromZero) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            bb[u] = cc[u + 1];
+            edge[u] = val(edge[u]);
+            ym[u] = make_float2(val(ym[u].x), val(ym[u].y));
+            yp[u] = make_float2(val(yp[u].x), val(yp[u].y));
+        }
+#pragma unroll
+        for (int u = 0; u < U + 2; u++) cc[u] = make_float2(val(cc[u].x), val(cc[u].y));
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        float l, r;
+        pair_sides(cc[u + 1], edge[u], t.lane, &l, &r);
+        const float c0 = cc[u + 1].x, c1 = cc[u + 1].y;
+        const float h0 = c.beta * (-bb[u].x + c.ax * (c1 + l) + c.ay * (yp[u].x + ym[u].x) + c.az * (cc[u + 2].x + cc[u].x));
+        const float h1 = c.beta * (-bb[u].y + c.ax * (r + c0) + c.ay * (yp[u].y + ym[u].y) + c.az * (cc[u + 2].y + cc[u].y));
+        const float v0 = c.omw * c0 + c.w * h0, v1 = c.omw * c1 + c.w * h1;
+        if (!t.live || k0 + u > z1) continue;
+        const int x = t.x0 + nk * (k0 + u);
+        if (MODE == kPairCorrect) {
+            if (p2) pair_store(p, push_p ? fl[u] : pair_inner(fl[u]), push, x, make_double2(pp[u].x + (double) v0, pp[u].y + (double) v1),
+                            nj, nk);
+            else {
+                if (fl[u] & 1u) p[x] = pp[u].x + (double) v0;
+                if (fl[u] & 0x100u) p[x + 1] = pp[u].y + (double) v1;
+            }
+        } else pair_store(out, fl[u], push, x, make_float2(v0, v1), nj, nk);
+    }
+}
+
+// k_mx_residuum_restrict, a warp on 31 coarse cells of a row: lane n forms the residuals
+// of fine cells 2 m and 2 m + 1 (m = its coarse cell) in the 4 rows of children and
+// takes those of 2 m - 1 from the lane before.  A thread walks up its run of coarse
+// planes with the next one's loads in flight.  256^3 to 128^3: 40 us (floor 24), 43
+// by k_mx_residuum_restrict, 52 with a thread per coarse cell; at 128^3 and below
+// 13 / 7 / 6 us.  push: the coarse cells' patterns,
+// where the coarse level's first sweeps read r in its boundary cells.
+__global__ void __launch_bounds__(256) k_mx_down2(float *__restrict__ out, const float *__restrict__ e,
+                                                  const float *__restrict__ b, const uint8_t *__restrict__ cflags,
+                                                  const uint8_t *__restrict__ nbm, const uint8_t *__restrict__ cnbm,
+                                                  const uint64_t *__restrict__ cpush, Level C, Level F, Box3 box, int planes, float rx,
+                                                  float ry, float rz, const LoopState *__restrict__ pred) {
+    pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
+    pdl_trigger();
+    if (pred && !pred->cond) return;
+    const int lane = (int) threadIdx.x;
+    const int m = (int) box.x0 - 1 + 31 * (int) blockIdx.x + lane, j = (int) box.y0 + (int) (blockIdx.y * 8 + threadIdx.y);
+    if (j > (int) box.y1) return;
+    const int ka = (int) box.z0 + (int) blockIdx.z * planes, ke = min(ka + planes - 1, (int) box.z1);
+    const int fx = (int) F.Nx, fxy = (int) F.nxy(), mc = min(m, (int) box.x1);
+    // rows 2 j - 2 .. 2 j + 1 of planes 2 k - 2 .. 2 k + 1, without the corners; a step up
+    // keeps the inner rows of the upper two planes
+    int x0 = 2 * mc + fx * (2 * j - 1) + fxy * (2 * ka - 1);
+    float2 v[4][4];
+#pragma unroll
+    for (int z = 0; z < 2; z++)
+#pragma unroll
+        for (int y = 1; y < 3; y++) v[z][y] = ld2(e + x0 + fx * (y - 1) + fxy * (z - 1));
+    struct In {
+        float2 lo0, lo3, up[4], top1, top2, b[4];
+        unsigned fl[4], cf, cm, side;
+    };
+    const auto load = [&](int x, int k) {
+        In n;
+        n.lo0 = ld2(e + x - fx);
+        n.lo3 = ld2(e + x + 2 * fx);
+#pragma unroll
+        for (int y = 0; y < 4; y++) n.up[y] = ld2(e + x + fx * (y - 1) + fxy);
+        n.top1 = ld2(e + x + 2 * fxy);
+        n.top2 = ld2(e + x + fx + 2 * fxy);
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            n.b[c] = ld2(b + x + fx * (c & 1) + fxy * (c >> 1));
+            n.fl[c] = *(const uint16_t *) (nbm + x + fx * (c & 1) + fxy * (c >> 1));
+        }
+        const int q = mc + (int) C.Nx * j + (int) C.nxy() * k;
+        n.cf = cflags[q];
+        n.cm = cnbm ? cnbm[q] : 0u;
+        n.side = cnbm ? cnbm[q ^ 1] : 0u;
+        return n;
+    };
+    In cur = load(x0, ka);
+    for (int k = ka; k <= ke; k++, x0 += 2 * fxy) {
+        v[1][0] = cur.lo0;
+        v[1][3] = cur.lo3;
+#pragma unroll
+        for (int y = 0; y < 4; y++) v[2][y] = cur.up[y];
+        v[3][1] = cur.top1;
+        v[3][2] = cur.top2;
+        In nxt = cur;
+        if (k < ke) nxt = load(x0 + 2 * fxy, k + 1);
+        float sum = 0.f;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int y = 1 + (c & 1), z = 1 + (c >> 1);
+            const float2 o = v[z][y];
+            float l, r;
+            pair_sides(o, 0.f, lane, &l, &r);  // lane 0's first and lane 31's second residual go unused
+            const float ax = 2.f * o.x, ay = 2.f * o.y;
+            float r0 = cur.b[c].x - (rx * (l - ax + o.y) + ry * (v[z][y - 1].x - ax + v[z][y + 1].x) +
+                                     rz * (v[z - 1][y].x - ax + v[z + 1][y].x));
+            float r1 = cur.b[c].y - (rx * (o.x - ay + r) + ry * (v[z][y - 1].y - ay + v[z][y + 1].y) +
+                                     rz * (v[z - 1][y].y - ay + v[z + 1][y].y));
+            if (!(cur.fl[c] & 1u)) r0 = 0.f;
+            if (!(cur.fl[c] & 0x100u)) r1 = 0.f;
+            const float left = __shfl_up_sync(~0u, r1, 1);
+            sum = c ? sum + left : left;
+            sum += r0;
+        }
+        if (lane && m <= (int) box.x1 && (cur.cf & kInner)) {
+            const int q = m + (int) C.Nx * j + (int) C.nxy() * k;
+            const float mean = 0.125f * sum;
+            mx_store(out, (uint8_t) cur.cm, cpush, q, mean, (int) C.Nx, (int) C.nxy());
+            if (cur.side == kPartnerPlus || cur.side == kPartnerMinus) out[q ^ 1] = cur.side == kPartnerPlus ? mean : -mean;
+        }
+#pragma unroll
+        for (int y = 1; y < 3; y++) {
+            v[0][y] = v[2][y];
+            v[1][y] = v[3][y];
+        }
+        cur = nxt;
+    }
+}
+
+// k_mx_prolong_add8's values, a warp on 31 fine pairs (2 m, 2 m + 1) of 2 rows and 2
+// planes: both cells' 8 coarse values lie in the columns m and m + 1, the lane's
+// own and the next lane's, and a pair is stored in one piece.  128^3 to 256^3: 49 us
+// (floor 24; instructions bound it), walking up the planes 52 to 58.
+__global__ void __launch_bounds__(256) k_mx_prolong_add2(float *__restrict__ fine, const float *__restrict__ in,
+                                                         const uint8_t *__restrict__ cflags,
+                                                         const uint8_t *__restrict__ nbm,
+                                                         const uint64_t *__restrict__ push, Level C, Level F,
+                                                         Box3 cbox, Box3 fbox, const LoopState *__restrict__ pred) {
+    pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
+    pdl_trigger();
+    if (pred && !pred->cond) return;
+    const int lane = (int) threadIdx.x;
+    const int cm = (int) cbox.x0 - 1 + 31 * (int) blockIdx.x + lane, j = (int) cbox.y0 + (int) (blockIdx.y * 8 + threadIdx.y),
+              k = (int) cbox.z0 + (int) blockIdx.z;
+    if (j > (int) cbox.y1) return;
+    const int m = min(cm, (int) cbox.x1 + 1);  // columns x0 - 1 .. x1 + 1, the last a right neighbour only
+    const int nj = (int) C.Nx, nk = (int) C.nxy(), fx = (int) F.Nx, fxy = (int) F.nxy();
+    const int x = m + nj * j + nk * k;
+    const int mf = min(m, (int) cbox.x1);
+    float w[3][3][2];
+    float2 fv[4];
+    unsigned fl[4];
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int b = 0; b < 3; b++) w[a][b][0] = in[x + nj * (b - 1) + nk * (a - 1)];
+    const unsigned own = cflags[x] & kInner;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const int f = 2 * mf + fx * (2 * j - 1 + (c & 1)) + fxy * (2 * k - 1 + (c >> 1));
+        fl[c] = *(const uint16_t *) (nbm + f);
+        fv[c] = ld2(fine + f);
+    }
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int b = 0; b < 3; b++) w[a][b][1] = __shfl_down_sync(~0u, w[a][b][0], 1);
+    const unsigned next = __shfl_down_sync(~0u, own, 1);
+    if (lane == 31 || cm > (int) cbox.x1) return;
+    const int i0 = 2 * m, i1 = 2 * m + 1;
+    const bool in0 = own && m >= (int) cbox.x0 && i0 >= (int) fbox.x0 && i0 <= (int) fbox.x1;
+    const bool in1 = next && m + 1 <= (int) cbox.x1 && i1 >= (int) fbox.x0 && i1 <= (int) fbox.x1;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const int fj = 2 * j - 1 + (c & 1), fk = 2 * k - 1 + (c >> 1);
+        if (fj < (int) fbox.y0 || fj > (int) fbox.y1 || fk < (int) fbox.z0 || fk > (int) fbox.z1) continue;
+        const int py = c & 1 ? 2 : 0, pz = c >> 1 ? 2 : 0;
+        float2 v;
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+            const int o = 1 - s;
+            const float g = 0.015625f * (27.f * w[1][1][s] + 9.f * w[1][1][o] + 9.f * w[1][py][s] + 9.f * w[pz][1][s] +
+                                         3.f * w[1][py][o] + 3.f * w[pz][1][o] + 3.f * w[pz][py][s] + w[pz][py][o]);
+            (s ? v.y : v.x) = (s ? fv[c].y : fv[c].x) + g;
+        }
+        unsigned f2 = fl[c];
+        // an inner cell outside the children stays as it is, with its boundary cells
+        if ((f2 & 1u) && !in0) f2 = f2 >> 8 & 1u ? f2 & 0xff00u : 0u;
+        if ((f2 & 0x100u) && !in1) f2 = f2 & 1u ? f2 & 0x00ffu : 0u;
+        pair_store(fine, f2, push, 2 * m + fx * fj + fxy * fk, v, fx, fxy);
+    }
+}
+
+// the loop step of a kernel that reduces: thread 0 of each block has stored the block's
+// partial sum; the last block to get here adds them in a fixed order
+__device__ __forceinline__ void last_block_loop_step(const double *partials, LoopState *st, const LoopState *ref, double tol,
+                                                     long long max_it, double *smem) {
+    __shared__ bool last;
+    const int blocks = (int) (gridDim.x * gridDim.y * gridDim.z), tid = (int) (threadIdx.x + blockDim.x * threadIdx.y);
+    if (tid == 0) {
+        __threadfence();
+        last = atomicAdd(&st->blocks_done, 1) == blocks - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double v = 0.0;
+    for (int n = tid; n < blocks; n += (int) (blockDim.x * blockDim.y)) v += __ldcg(partials + n);
+    v = artss_block_sum(v, smem);
+    if (tid == 0) {
+        if (ref) tol = tol * sqrt(ref->sum);
+        const double r = sqrt(v);
+        st->blocks_done = 0;
+        st->sum = v;
+        st->residual = r;
+        st->it += 1;
+        st->cond = (r > tol && st->it < max_it) ? 1 : 0;
+    }
+}
+
+// k_mx_outer_residual on pairs of cells, r's boundary cells with it (push); a thread walks
+// up its run of planes with the next one's loads in flight.  256^3: 79 us (floor 50),
+// 101 with two planes' loads at a time, 90 by k_mx_outer_residual and its finishing
+// launch.
+__global__ void __launch_bounds__(256) k_mx_outer_residual2(const double *__restrict__ p, const double *__restrict__ b,
+                                                            float *__restrict__ r, const uint8_t *__restrict__ nbm,
+                                                            const uint64_t *__restrict__ push, Level L, Box3 box, int planes,
+                                                            double rx, double ry, double rz, double *__restrict__ partials,
+                                                            LoopState *st, const LoopState *ref, double tol,
+                                                            long long max_it) {
     pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
     pdl_trigger();
     __shared__ double smem[32];
-    if (pred && !pred->cond) return;
+    if (!st->cond) return;  // nobody writes it before every block has passed here
+    const int nj = (int) L.Nx, nk = (int) L.nxy();
+    const PairPos t = pair_pos(box, nj);
+    const int ka = (int) box.z0 + (int) blockIdx.y * planes, ke = min(ka + planes - 1, (int) box.z1);
+    const bool p2 = ((uintptr_t) p | (uintptr_t) b) % 16 == 0;
+    const auto ldp = [&](const double *q) { return p2 ? ld2(q) : make_double2(q[0], q[1]); };
+    struct In {
+        double2 ym, yp, b, kp;
+        double edge;
+        unsigned fl;
+    };
+    const auto load = [&](int x) {
+        In v;
+        v.kp = ldp(p + x + nk);
+        v.ym = ldp(p + x - nj);
+        v.yp = ldp(p + x + nj);
+        v.b = ldp(b + x);
+        v.edge = 0.0;
+        if (t.lane == 0 || t.lane == 31) v.edge = p[x + (t.lane ? 2 : -1)];
+        v.fl = *(const uint16_t *) (nbm + x);
+        return v;
+    };
+    double acc = 0.0;
+    int x = t.x0 + nk * ka;
+    double2 km = ldp(p + x - nk), c0 = ldp(p + x);
+    In cur = load(x);
+#pragma unroll 2
+    for (int k = ka; k <= ke; k++, x += nk) {
+        In nxt = cur;
+        if (k < ke) nxt = load(x + nk);
+        double l, rr;
+        pair_sides(c0, cur.edge, t.lane, &l, &rr);
+        const double ax = 2 * c0.x, ay = 2 * c0.y;
+        const double v0 = cur.b.x - (rx * (l - ax + c0.y) + ry * (cur.ym.x - ax + cur.yp.x) + rz * (km.x - ax + cur.kp.x));
+        const double v1 = cur.b.y - (rx * (c0.x - ay + rr) + ry * (cur.ym.y - ay + cur.yp.y) + rz * (km.y - ay + cur.kp.y));
+        if (t.live) {
+            pair_store(r, cur.fl, push, x, make_float2((float) v0, (float) v1), nj, nk);
+            if (cur.fl & 1u) acc += v0 * v0;
+            if (cur.fl & 0x100u) acc += v1 * v1;
+        }
+        km = c0;
+        c0 = cur.kp;
+        cur = nxt;
+    }
+    acc = artss_block_sum(acc, smem);
+    if (threadIdx.x == 0) partials[blockIdx.x + gridDim.x * blockIdx.y] = acc;
+    __syncthreads();  // smem is rewritten
+    last_block_loop_step(partials, st, ref, tol, max_it, smem);
+}
+
+// FP64 outer residual r = b - A p on level 0, stored as the FP32 right-hand
+// side of the correction equation; the last block to finish adds the blocks' partial
+// sums of ||r||^2 in a fixed order and does the loop step (state `st`, tolerance tol,
+// times sqrt(ref->sum) with ref)
+__global__ void __launch_bounds__(256, 8) k_mx_outer_residual(const double *__restrict__ p, const double *__restrict__ b,
+                                    float *__restrict__ r, const uint8_t *__restrict__ flags, Level L, Box3 box,
+                                    double rx, double ry, double rz, double *__restrict__ partials, LoopState *st,
+                                    const LoopState *ref, double tol, long long max_it) {
+    pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
+    pdl_trigger();
+    __shared__ double smem[32];
+    if (!st->cond) return;  // nobody writes it before every block has passed here
     MX_COLUMN(box);
     const int nj = (int) L.Nx, nk = (int) L.nxy();
     double acc = 0.0;
@@ -334,6 +755,8 @@ __global__ void __launch_bounds__(256, 8) k_mx_outer_residual(const double *__re
     acc = artss_block_sum(acc, smem);
     if (threadIdx.x == 0 && threadIdx.y == 0)
         partials[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = acc;
+    __syncthreads();  // smem is rewritten
+    last_block_loop_step(partials, st, ref, tol, max_it, smem);
 }
 
 // p += e on the inner cells (FP64 += FP32)
@@ -436,22 +859,61 @@ int mx_smooth_rbgs(artss_mixed *m, int l, bool from_zero, const LoopState *pred)
     return ARTSS_OK;
 }
 
-// one weighted-Jacobi sweep m->t[l] <- m->e[l] (p: added to p instead, see
-// k_mx_jacobi), in the launch shape tuned for the level (the p form repeats
-// no launch, so it takes the shape the plain form was tuned to)
-int mx_jacobi(artss_mixed *m, int l, const CoefF &c, const LoopState *pred, double *p) {
+// rows of whole pairs of cells take the two-cell kernels, which need the pairs aligned
+// (256^3 pressure solve of 14 cycles: 7.2 ms by them, 9.5 by the one-cell kernels)
+bool mx_pairs(const artss_mixed *m, const Level &L) {
+    return L.Nx % 2 == 0 && m->cfg.n_relax > 1 && !(m->cfg.flags & (ARTSS_MIXED_BC_LAUNCH | ARTSS_MIXED_FINE_PROLONG));
+}
+// r carries its boundary cells, and the first two sweeps run as one
+bool mx_zero_pair(const artss_mixed *m, int l) {
+    return l + 1 < m->L && m->fold[l] && mx_pairs(m, m->ctx->lvl[l]);
+}
+inline dim3 pair_grid(const Level &L, const Box3 &b, int threads, int planes) {
+    return dim3((unsigned) ((b.ny() * L.Nx / 2 + threads - 1) / threads), (unsigned) ((b.nz() + planes - 1) / planes));
+}
+// planes per thread of the kernels that walk up the planes: 8 blocks per SM for the
+// latency of the loads, and no more, as each run reads the planes at its ends again
+inline int pair_planes(const artss_ctx *ctx, const Box3 &b, int64_t blocks_xy) {
+    return (int) std::max<int64_t>(1, std::min<int64_t>(32, blocks_xy * b.nz() / (8 * std::max(ctx->sm_count, 1))));
+}
+
+template <int MODE>
+int mx_jacobi2(artss_mixed *m, int l, const CoefF &c, const LoopState *pred, double *p = nullptr, int push_p = 0) {
     artss_ctx *ctx = m->ctx;
     const Level &L = ctx->lvl[l];
     const Box3 box = inner_box(L);
+    ARTSS_LAUNCH_PDL(ctx, FAM_MG_JACOBI, k_mx_jacobi2<MODE>, pair_grid(L, box, kPairThreads, kPairPlanes),
+                     dim3(kPairThreads), 0, MODE == kPairFromZero ? m->e[l] : m->t[l],
+                     MODE == kPairFromZero ? (const float *) m->r[l] : (const float *) m->e[l], (const float *) m->r[l],
+                     (const uint8_t *) m->nbm[l], (const uint64_t *) m->push[l], L, box, c, pred, p, push_p);
+    ARTSS_LAUNCH_CK(ctx);
+    return ARTSS_OK;
+}
+
+// the correcting sweep writes p's boundary cells too: its program is homogeneous and
+// wholly in level 0's patterns
+int mx_pushes_p(const artss_mixed *m, const double *p) {
+    return (uintptr_t) p % 16 == 0 && m->fold[0] && m->whole[0] && m->ctx->bc[0][ARTSS_FIELD_P].homogeneous;
+}
+
+// one weighted-Jacobi sweep m->t[l] <- m->e[l] (p: added to p instead, see
+// k_mx_jacobi), in the launch shape tuned for the level (the p form repeats
+// no launch, so it takes the shape the plain form was tuned to)
+int mx_jacobi(artss_mixed *m, int l, const CoefF &c, const LoopState *pred, double *p, int push_p = 0) {
+    artss_ctx *ctx = m->ctx;
+    const Level &L = ctx->lvl[l];
+    const Box3 box = inner_box(L);
+    if (mx_pairs(m, L))
+        return p ? mx_jacobi2<kPairCorrect>(m, l, c, pred, p, push_p) : mx_jacobi2<kPairSweep>(m, l, c, pred);
     return tuned_column_launch(ctx, kTuneMxJacobi, l, box, p == nullptr, [&](dim3 g, dim3 bl) -> int {
         if (p)
             ARTSS_LAUNCH_PDL(ctx, FAM_MG_JACOBI, k_mx_jacobi<true>, g, bl, 0, m->t[l], (const float *) m->e[l],
-                             (const float *) m->r[l], (const uint8_t *) m->nbm[l], (const uint16_t *) m->push[l], L,
-                             box, c, pred, p);
+                             (const float *) m->r[l], (const uint8_t *) m->nbm[l], (const uint64_t *) m->push[l], L,
+                             box, c, pred, p, push_p);
         else
             ARTSS_LAUNCH_PDL(ctx, FAM_MG_JACOBI, k_mx_jacobi<false>, g, bl, 0, m->t[l], (const float *) m->e[l],
-                             (const float *) m->r[l], (const uint8_t *) m->nbm[l], (const uint16_t *) m->push[l], L,
-                             box, c, pred, (double *) nullptr);
+                             (const float *) m->r[l], (const uint8_t *) m->nbm[l], (const uint64_t *) m->push[l], L,
+                             box, c, pred, (double *) nullptr, 0);
         ARTSS_LAUNCH_CK(ctx);
         return ARTSS_OK;
     }, 256);
@@ -465,16 +927,19 @@ int mx_smooth_from_zero(artss_mixed *m, int l, const LoopState *pred) {
     const Level &L = ctx->lvl[l];
     const Box3 box = inner_box(L);
     const CoefF c = coef_f(ctx, l, m->cfg.w);
-    int st;
-    if ((st = tuned_column_launch(ctx, kTuneMxJacobi0, l, box, true, [&](dim3 g, dim3 bl) -> int {
+    int st, first = 1;
+    if (mx_zero_pair(m, l)) {
+        if ((st = mx_jacobi2<kPairFromZero>(m, l, c, pred))) return st;
+        first = 2;
+    } else if ((st = tuned_column_launch(ctx, kTuneMxJacobi0, l, box, true, [&](dim3 g, dim3 bl) -> int {
              ARTSS_LAUNCH_PDL(ctx, FAM_MG_JACOBI, k_mx_jacobi0, g, bl, 0, m->e[l], (const float *) m->r[l],
-                              (const uint8_t *) m->nbm[l], (const uint16_t *) m->push[l], L, box, c, pred);
+                              (const uint8_t *) m->nbm[l], (const uint64_t *) m->push[l], L, box, c, pred);
              ARTSS_LAUNCH_CK(ctx);
              return ARTSS_OK;
          })))
         return st;
-    if ((st = mx_bc_sweep(m, m->e[l], l, pred))) return st;
-    for (int s = 1; s < m->cfg.n_relax; s++) {
+    if (first == 1 && (st = mx_bc_sweep(m, m->e[l], l, pred))) return st;
+    for (int s = first; s < m->cfg.n_relax; s++) {
         if ((st = mx_jacobi(m, l, c, pred, nullptr))) return st;
         std::swap(m->e[l], m->t[l]);
         if ((st = mx_bc_sweep(m, m->e[l], l, pred))) return st;
@@ -495,7 +960,7 @@ int mx_smooth(artss_mixed *m, int l, const LoopState *pred, double *p = nullptr,
     int st;
     for (int s = 0; s < m->cfg.n_relax; s++) {
         if (p && s + 1 == m->cfg.n_relax) {
-            if ((st = mx_jacobi(m, l, c, pred, p))) return st;
+            if ((st = mx_jacobi(m, l, c, pred, p, mx_pushes_p(m, p)))) return st;
             if (corrected) *corrected = true;
             break;
         }
@@ -506,34 +971,39 @@ int mx_smooth(artss_mixed *m, int l, const LoopState *pred, double *p = nullptr,
     return ARTSS_OK;
 }
 
-// Push masks of levels 0 .. L-2 from the inner bitmaps and the pressure
+// Push patterns of levels 0 .. L-2 from the inner cells and the pressure
 // boundary programs with every value zero (x_t = +-x_root after chain
 // folding).  Every boundary cell that a smoothing or residual stencil reads
-// (a face neighbour of an inner cell) must take its value from an inner face
-// neighbour, which then writes it with each of its own values.  A level where
-// that fails (a root that is not inner, not face-adjacent or itself written by
+// (a face neighbour of an inner cell) must take its value from an inner cell one
+// step away along an axis, which then writes it with each of its own values; where
+// every other boundary cell takes its value from an inner cell among its 26
+// neighbours too, the patterns hold the whole program.  A level where the former
+// fails (a root that is not inner, not face-adjacent or itself written by
 // the program, an inner target) or a solver with ARTSS_MIXED_RBGS /
 // ARTSS_MIXED_BC_LAUNCH launches the program after each sweep instead, with a
-// mask of inner bits only.
+// mask of inner bits only.  ARTSS_MIXED_BC_LAUNCH also keeps residual, its program
+// and restriction apart and takes the one-cell kernels.
 int mx_build_tables(artss_mixed *m) {
     artss_ctx *ctx = m->ctx;
     const bool allow = !(m->cfg.flags & (ARTSS_MIXED_RBGS | ARTSS_MIXED_BC_LAUNCH));
     for (int l = 0; l + 1 < m->L; l++) {
         const Level &L = ctx->lvl[l];
         const int64_t n = L.size();
-        std::vector<uint16_t> pat((size_t) n, 0);  // 2 bits per direction, as a push pattern
-        const std::vector<bool> &inner = ctx->h_inner[l];
-        const bool have_inner = (int64_t) inner.size() == n;
-        bool fold = allow && have_inner;
+        const CellBits &inner = ctx->inner_bits[l];
+        const bool have_inner = inner.n == n;
+        bool fold = allow && have_inner, whole = fold;
+        const bool pairs = mx_pairs(m, L);
+        std::vector<std::pair<int64_t, uint8_t>> partner;
+        std::vector<std::pair<int64_t, uint64_t>> pat, far_pat;  // (inner cell, its share of the pattern): read targets, others
         const BcProgram &p = ctx->bc[l][ARTSS_FIELD_P];
+        std::unordered_map<int64_t, std::pair<int64_t, int>> res;
         if (fold && p.present && p.n) {
             // final (root, sign) of every target, the program applied wave by wave
-            std::unordered_map<int64_t, std::pair<int64_t, int>> res;
             res.reserve((size_t) p.n * 2);
             for (int64_t a = 0; a < p.n; a++) {
                 int64_t r = p.h_root[(size_t) a];
                 int sg = p.h_sign[(size_t) a];
-                const auto it = res.find(r);
+                const auto it = p.waves > 1 ? res.find(r) : res.end();
                 if (it != res.end()) {
                     r = it->second.first;
                     sg *= it->second.second;
@@ -541,49 +1011,87 @@ int mx_build_tables(artss_mixed *m) {
                 res[p.h_target[(size_t) a]] = {r, sg};
             }
             const int64_t off[6] = {-1, 1, -L.Nx, L.Nx, -L.nxy(), L.nxy()};
+            pat.reserve(res.size());
             for (const auto &kv : res) {
                 const int64_t t = kv.first, r = kv.second.first;
-                const int sg = kv.second.second;
-                if (inner[(size_t) t]) { fold = false; break; }
+                if (inner.get(t)) { fold = false; break; }
                 bool read = false;  // t is a face neighbour of an inner cell
-                for (int d = 0; d < 6 && !read; d++) {
-                    const int64_t x = t - off[d];
-                    read = x >= 0 && x < n && inner[(size_t) x];
+                for (int64_t d : off) read = read || (t - d >= 0 && t - d < n && inner.get(t - d));
+                const int64_t tz = t / L.nxy(), ty = t / L.Nx % L.Ny, tx = t % L.Nx;
+                const int64_t dx = tx - r % L.Nx, dy = ty - r / L.Nx % L.Ny, dz = tz - r / L.nxy();
+                const int64_t far = std::max({std::abs(dx), std::abs(dy), std::abs(dz)});
+                const bool root_ok = far == 1 && inner.get(r) && !res.count(r);
+                if (read && !(root_ok && std::abs(dx) + std::abs(dy) + std::abs(dz) == 1)) { fold = false; break; }
+                if (!root_ok) {
+                    whole = false;
+                    continue;
                 }
-                if (!read) continue;
-                int dir = -1;  // t = r + off[dir]
-                for (int d = 0; d < 6; d++)
-                    if (r + off[d] == t) dir = d;
-                if (dir < 0 || r < 0 || r >= n || !inner[(size_t) r] || res.count(r)) { fold = false; break; }
-                pat[(size_t) r] = (uint16_t) (pat[(size_t) r] | ((sg > 0 ? 1u : 2u) << (2 * dir)));
+                if (pairs && dy == 0 && dz == 0 && (std::min(tx, tx - dx) % 2 == 0)) {
+                    partner.push_back({t, (uint8_t) (kv.second.second > 0 ? kPartnerPlus : kPartnerMinus)});
+                    continue;
+                }
+                const int dir = (int) ((dx + 1) + 3 * (dy + 1) + 9 * (dz + 1));
+                (read ? pat : far_pat).push_back({r, (kv.second.second > 0 ? 1ull : 2ull) << (2 * dir)});
             }
         }
-        // distinct patterns -> ids 1..127
         std::vector<uint8_t> nbm((size_t) n, 0);
-        std::vector<uint16_t> push(128, 0);
-        std::unordered_map<uint16_t, int> ids;
-        for (int64_t x = 0; x < n && fold; x++) {
-            const uint16_t pv = pat[(size_t) x];
-            if (!pv) continue;
-            auto it = ids.find(pv);
-            if (it == ids.end()) {
-                if (ids.size() >= 127) { fold = false; break; }
-                it = ids.emplace(pv, (int) ids.size() + 1).first;
-                push[(size_t) it->second] = pv;
-            }
-            nbm[(size_t) x] = (uint8_t) (it->second << 1);
-        }
-        if (!fold) {
-            std::fill(push.begin(), push.end(), (uint16_t) 0);
-            std::fill(nbm.begin(), nbm.end(), (uint8_t) 0);
-        }
         if (have_inner)
-            for (int64_t x = 0; x < n; x++)
-                if (inner[(size_t) x]) nbm[(size_t) x] = (uint8_t) (nbm[(size_t) x] | 1u);
+            for (int64_t i = 0; i < (int64_t) inner.w.size(); i++) {
+                const uint64_t w = inner.w[(size_t) i];
+                for (int64_t x = 64 * i; x < std::min(n, 64 * i + 64); x++) nbm[(size_t) x] = (uint8_t) (w >> (x & 63) & 1);
+            }
+        // distinct patterns -> ids 1..127, without the targets that no sweep reads
+        // where they make too many
+        std::vector<uint64_t> push(128, 0);
+        std::vector<std::pair<int64_t, int>> of;
+        const auto number = [&](std::vector<std::pair<int64_t, uint64_t>> v) {
+            std::unordered_map<uint64_t, int> ids;
+            std::sort(v.begin(), v.end());
+            of.clear();
+            std::fill(push.begin(), push.end(), (uint64_t) 0);
+            for (size_t a = 0; a < v.size();) {
+                const int64_t r = v[a].first;
+                uint64_t bits = 0;
+                for (; a < v.size() && v[a].first == r; a++) bits |= v[a].second;
+                auto it = ids.find(bits);
+                if (it == ids.end()) {
+                    if (ids.size() >= 127) return false;
+                    it = ids.emplace(bits, (int) ids.size() + 1).first;
+                    push[(size_t) it->second] = bits;
+                }
+                of.push_back({r, it->second});
+            }
+            return true;
+        };
+        if (fold && whole) {
+            far_pat.insert(far_pat.end(), pat.begin(), pat.end());
+            whole = number(std::move(far_pat));
+        }
+        if (fold && !whole) fold = number(pat);
+        if (fold)
+            for (const auto &a : partner) nbm[(size_t) a.first] = a.second;
+        if (fold)
+            for (const auto &a : of) nbm[(size_t) a.first] = (uint8_t) (nbm[(size_t) a.first] | a.second << 1);
+        else
+            std::fill(push.begin(), push.end(), (uint64_t) 0);
         m->fold[l] = fold;
+        m->whole[l] = fold && whole;
+        // the children of the coarse inner cells are inner or touched by nothing
+        const Level &C = ctx->lvl[l + 1];
+        const CellBits &cin = ctx->inner_bits[l + 1];
+        bool dead = have_inner && !(m->cfg.flags & ARTSS_MIXED_BC_LAUNCH) && cin.n == C.size() && C.i1 >= 1 && C.j1 >= 1 && C.k1 >= 1 &&
+                    2 * C.i2 + 1 < L.Nx && 2 * C.j2 + 1 < L.Ny && 2 * C.k2 + 1 < L.Nz;
+        for (int64_t t : p.h_target) {
+            if (!dead) break;
+            const int64_t ci = (t % L.Nx + 1) / 2, cj = (t / L.Nx % L.Ny + 1) / 2, ck = (t / L.nxy() + 1) / 2;
+            dead = ci >= C.Nx || cj >= C.Ny || ck >= C.Nz || !cin.get(ci + C.Nx * cj + C.nxy() * ck);
+        }
+        m->q_bc_dead[l] = dead;
+        // r's boundary cells are written from the patterns: none of an earlier geometry's
+        ARTSS_CK(cudaMemsetAsync(m->r[l], 0, (size_t) n * sizeof(float), ctx->stream));
         if (!m->nbm[l]) ARTSS_CK(cudaMalloc(&m->nbm[l], (size_t) n));
-        if (!m->push[l]) ARTSS_CK(cudaMalloc(&m->push[l], 128 * sizeof(uint16_t)));
-        ARTSS_CK(cudaMemcpyAsync(m->push[l], push.data(), 128 * sizeof(uint16_t), cudaMemcpyHostToDevice, ctx->stream));
+        if (!m->push[l]) ARTSS_CK(cudaMalloc(&m->push[l], 128 * sizeof(uint64_t)));
+        ARTSS_CK(cudaMemcpyAsync(m->push[l], push.data(), 128 * sizeof(uint64_t), cudaMemcpyHostToDevice, ctx->stream));
         ARTSS_CK(cudaMemcpyAsync(m->nbm[l], nbm.data(), (size_t) n, cudaMemcpyHostToDevice, ctx->stream));
         // the host vectors die with this iteration
         ARTSS_CK(cudaStreamSynchronize(ctx->stream));
@@ -603,6 +1111,34 @@ int mx_vcycle(artss_mixed *m, const LoopState *pred, double *p = nullptr, bool *
         if ((st = mx_smooth_from_zero(m, l, pred))) return st;
         const Level &L = ctx->lvl[l];
         const Box3 box = inner_box(L);
+        if (m->q_bc_dead[l]) {
+            const Level &C = ctx->lvl[l + 1];
+            const Box3 cbox = inner_box(C);
+            if (mx_pairs(m, L)) {
+                const bool push = mx_zero_pair(m, l + 1);
+                dim3 gr((unsigned) ((cbox.nx() + 30) / 31), (unsigned) ((cbox.ny() + 7) / 8));
+                const int planes = pair_planes(ctx, cbox, (int64_t) gr.x * gr.y);
+                gr.z = (unsigned) ((cbox.nz() + planes - 1) / planes);
+                ARTSS_LAUNCH_PDL(ctx, FAM_MG_RESIDUUM, k_mx_down2, gr, dim3(32, 8), 0, m->r[l + 1],
+                                 (const float *) m->e[l], (const float *) m->r[l], (const uint8_t *) ctx->d_flags[l + 1],
+                                 (const uint8_t *) m->nbm[l], (const uint8_t *) (push ? m->nbm[l + 1] : nullptr),
+                                 (const uint64_t *) m->push[l + 1], C, L, cbox, planes, (float) (1. / (g.dx[l] * g.dx[l])),
+                                 (float) (1. / (g.dy[l] * g.dy[l])), (float) (1. / (g.dz[l] * g.dz[l])), pred);
+                ARTSS_LAUNCH_CK(ctx);
+            } else if ((st = tuned_column_launch(ctx, kTuneMxDown, l + 1, cbox, true, [&](dim3 gr, dim3 bl) -> int {
+                     ARTSS_LAUNCH_PDL(ctx, FAM_MG_RESIDUUM, k_mx_residuum_restrict, gr, bl, 0, m->r[l + 1],
+                                      (const float *) m->e[l], (const float *) m->r[l],
+                                      (const uint8_t *) ctx->d_flags[l + 1], (const uint8_t *) m->nbm[l], C, L, cbox,
+                                      (float) (1. / (g.dx[l] * g.dx[l])), (float) (1. / (g.dy[l] * g.dy[l])),
+                                      (float) (1. / (g.dz[l] * g.dz[l])), pred);
+                     ARTSS_LAUNCH_CK(ctx);
+                     return ARTSS_OK;
+                 }, 256)))
+                return st;
+            else if (mx_zero_pair(m, l + 1) && (st = mx_bc(m, m->r[l + 1], l + 1, pred)))
+                return st;
+            continue;
+        }
         if ((st = tuned_column_launch(ctx, kTuneMxResiduum, l, box, true, [&](dim3 gr, dim3 bl) -> int {
                  ARTSS_LAUNCH_PDL(ctx, FAM_MG_RESIDUUM, k_mx_residuum, gr, bl, 0, m->q[l], (const float *) m->e[l],
                                   (const float *) m->r[l], (const uint8_t *) m->nbm[l], L, box,
@@ -622,6 +1158,7 @@ int mx_vcycle(artss_mixed *m, const LoopState *pred, double *p = nullptr, bool *
                  return ARTSS_OK;
              })))
             return st;
+        if (mx_zero_pair(m, l + 1) && (st = mx_bc(m, m->r[l + 1], l + 1, pred))) return st;
     }
     // coarsest level: FP64 solve from zero
     {
@@ -639,8 +1176,9 @@ int mx_vcycle(artss_mixed *m, const LoopState *pred, double *p = nullptr, bool *
     }
     for (int l = Lc - 1; l >= 0; l--) {
         // the prolongation reads the coarse correction's boundary cells (edges
-        // and corners too): the level's program once, where the sweeps skipped it
-        if (l + 1 < Lc && m->fold[l + 1] && (st = mx_bc(m, m->e[l + 1], l + 1, pred))) return st;
+        // and corners too): the level's program once, where the sweeps skipped it and
+        // did not write them all
+        if (l + 1 < Lc && m->fold[l + 1] && !m->whole[l + 1] && (st = mx_bc(m, m->e[l + 1], l + 1, pred))) return st;
         const Level &C = ctx->lvl[l + 1], &F = ctx->lvl[l];
         // the fine children 2c - 1, 2c of the coarse inner box, within the fine inner box
         const Box3 fbox{std::max(F.i1, 2 * C.i1 - 1), std::min(F.i2, 2 * C.i2), std::max(F.j1, 2 * C.j1 - 1),
@@ -649,11 +1187,16 @@ int mx_vcycle(artss_mixed *m, const LoopState *pred, double *p = nullptr, bool *
         if (m->cfg.flags & ARTSS_MIXED_FINE_PROLONG) {
             ARTSS_LAUNCH_PDL(ctx, FAM_MG_PROLONGATE, k_mx_prolong_add, mx_grid(fbox), box_block(), 0,
                              m->e[l], (const float *) m->e[l + 1], (const uint8_t *) ctx->d_flags[l + 1],
-                             (const uint8_t *) m->nbm[l], (const uint16_t *) m->push[l], C, F, fbox, pred);
+                             (const uint8_t *) m->nbm[l], (const uint64_t *) m->push[l], C, F, fbox, pred);
+        } else if (mx_pairs(m, F)) {
+            const dim3 gr((unsigned) ((cbox.nx() + 31) / 31), (unsigned) ((cbox.ny() + 7) / 8), (unsigned) cbox.nz());
+            ARTSS_LAUNCH_PDL(ctx, FAM_MG_PROLONGATE, k_mx_prolong_add2, gr, dim3(32, 8), 0, m->e[l],
+                             (const float *) m->e[l + 1], (const uint8_t *) ctx->d_flags[l + 1],
+                             (const uint8_t *) m->nbm[l], (const uint64_t *) m->push[l], C, F, cbox, fbox, pred);
         } else {
             ARTSS_LAUNCH_PDL(ctx, FAM_MG_PROLONGATE, k_mx_prolong_add8, mx_grid(cbox), box_block(), 0,
                              m->e[l], (const float *) m->e[l + 1], (const uint8_t *) ctx->d_flags[l + 1],
-                             (const uint8_t *) m->nbm[l], (const uint16_t *) m->push[l], C, F, cbox, fbox, pred);
+                             (const uint8_t *) m->nbm[l], (const uint64_t *) m->push[l], C, F, cbox, fbox, pred);
         }
         ARTSS_LAUNCH_CK(ctx);
         if ((st = mx_bc_sweep(m, m->e[l], l, pred))) return st;
@@ -772,6 +1315,11 @@ int artss_mixed_solve(artss_mixed *m, double *p, const double *b, artss_solve_st
     int st;
     const dim3 grid = mx_grid(box);
     if ((st = check_reduce_blocks(grid))) return st;
+    // at most 4096 partial sums for the last block to add, where planes allow it
+    const int64_t pair_blocks = (box.ny() * L.Nx / 2 + 255) / 256;
+    const int planes = (int) std::max<int64_t>(pair_planes(ctx, box, pair_blocks), pair_blocks * box.nz() / 4096);
+    const dim3 pgrid = pair_grid(L, box, 256, planes);
+    if ((st = check_reduce_blocks(pgrid))) return st;
     if (m->geom_version != ctx->geom_version) {
         // cell lists or boundary programs changed since the tables were built
         if (ctx->capturing) { set_error("the mixed solver's boundary tables are stale; solve once before capturing"); return ARTSS_ERR_ARG; }
@@ -812,13 +1360,18 @@ int artss_mixed_solve(artss_mixed *m, double *p, const double *b, artss_solve_st
     }
     while (cond) {
         for (int64_t r = 0; r < batch; r++) {
-            ARTSS_LAUNCH_PDL(ctx, FAM_MG_RESNORM, k_mx_outer_residual, grid, box_block(), 0, 
-                                                  p, b, m->r[0], ctx->d_flags[0], L, box, rx, ry, rz,
-                                                  ctx->d_partials, pred);
+            const LoopState *ref = ctx->capturing ? ctx->d_loop + kSlotSum : nullptr;
+            const double eps = ctx->capturing ? m->cfg.rel_tol : tol;
+            if (mx_pairs(m, L))
+                ARTSS_LAUNCH_PDL(ctx, FAM_MG_RESNORM, k_mx_outer_residual2, pgrid, dim3(256), 0, (const double *) p, b,
+                                 m->r[0], (const uint8_t *) m->nbm[0], (const uint64_t *) m->push[0], L, box, planes,
+                                 rx, ry, rz,
+                                 ctx->d_partials, ctx->d_loop + kSlotOuter, ref, eps, max_eval);
+            else
+                ARTSS_LAUNCH_PDL(ctx, FAM_MG_RESNORM, k_mx_outer_residual, grid, box_block(), 0, (const double *) p, b,
+                                 m->r[0], (const uint8_t *) ctx->d_flags[0], L, box, rx, ry, rz,
+                                 ctx->d_partials, ctx->d_loop + kSlotOuter, ref, eps, max_eval);
             ARTSS_LAUNCH_CK(ctx);
-            if (ctx->capturing) st = finalize_loop_rel(ctx, kSlotOuter, nb, m->cfg.rel_tol, kSlotSum, max_eval);
-            else st = finalize_loop(ctx, kSlotOuter, nb, tol, max_eval);
-            if (st) return st;
             bool corrected = false;
             if ((st = mx_vcycle(m, pred, p, &corrected))) return st;
             if (!corrected) {
@@ -826,7 +1379,7 @@ int artss_mixed_solve(artss_mixed *m, double *p, const double *b, artss_solve_st
                                                     p, m->e[0], ctx->d_flags[0], L, box, pred);
                 ARTSS_LAUNCH_CK(ctx);
             }
-            if ((st = apply_bc(ctx, p, 0, ARTSS_FIELD_P, pred))) return st;
+            if (!(corrected && mx_pushes_p(m, p)) && (st = apply_bc(ctx, p, 0, ARTSS_FIELD_P, pred))) return st;
         }
         if (ctx->capturing) {
             if ((st = gl.end(kSlotOuter, max_eval + 2))) return st;

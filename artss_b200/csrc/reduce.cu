@@ -10,17 +10,12 @@
 
 namespace artss {
 
-// mode 0: loop step with tolerance tol; 3: the same with tol * sqrt(ref->sum);
-// 1: plain sum; 2: sum and its square root
+// mode 0: loop step with tolerance tol; 1: plain sum; 2: sum and its square root
 __global__ void k_finalize_loop(const double *__restrict__ partials, int nblocks, LoopState *__restrict__ st,
-                                double tol, long long max_it, int mode, const LoopState *__restrict__ ref) {
+                                double tol, long long max_it, int mode) {
     pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
     pdl_trigger();
     __shared__ double smem[32];
-    if (mode == 3) {
-        tol = tol * sqrt(ref->sum);
-        mode = 0;
-    }
     // a predicated iteration enqueued after the loop ended changes nothing
     if (mode == 0 && !st->cond) return;
     double v = 0.0;
@@ -71,7 +66,7 @@ __global__ void k_loop_continue(LoopState *st, cudaGraphConditionalHandle h, lon
 }
 
 int finalize_loop(artss_ctx *ctx, int slot, int nblocks, double tol, long long max_it) {
-    ARTSS_LAUNCH_PDL(ctx, FAM_REDUCE, k_finalize_loop, 1, kReduceThreads, 0, ctx->d_partials, nblocks, ctx->d_loop + slot, tol, max_it, 0, nullptr);
+    ARTSS_LAUNCH_PDL(ctx, FAM_REDUCE, k_finalize_loop, 1, kReduceThreads, 0, ctx->d_partials, nblocks, ctx->d_loop + slot, tol, max_it, 0);
     ARTSS_LAUNCH_CK(ctx);
     return ARTSS_OK;
 }
@@ -83,22 +78,14 @@ int finalize_loop_pair(artss_ctx *ctx, int slot, int parity, int nblocks, double
     return ARTSS_OK;
 }
 
-int finalize_loop_rel(artss_ctx *ctx, int slot, int nblocks, double rel_tol, int ref_slot, long long max_it) {
-    ARTSS_LAUNCH_PDL(ctx, FAM_REDUCE, k_finalize_loop, 1, kReduceThreads, 0, 
-                                      ctx->d_partials, nblocks, ctx->d_loop + slot, rel_tol, max_it, 3,
-                                      ctx->d_loop + ref_slot);
-    ARTSS_LAUNCH_CK(ctx);
-    return ARTSS_OK;
-}
-
 int finalize_sum(artss_ctx *ctx, int slot, int nblocks) {
-    ARTSS_LAUNCH_PDL(ctx, FAM_REDUCE, k_finalize_loop, 1, kReduceThreads, 0, ctx->d_partials, nblocks, ctx->d_loop + slot, 0.0, 0, 1, nullptr);
+    ARTSS_LAUNCH_PDL(ctx, FAM_REDUCE, k_finalize_loop, 1, kReduceThreads, 0, ctx->d_partials, nblocks, ctx->d_loop + slot, 0.0, 0, 1);
     ARTSS_LAUNCH_CK(ctx);
     return ARTSS_OK;
 }
 
 int finalize_residual(artss_ctx *ctx, int slot, int nblocks) {
-    ARTSS_LAUNCH_PDL(ctx, FAM_REDUCE, k_finalize_loop, 1, kReduceThreads, 0, ctx->d_partials, nblocks, ctx->d_loop + slot, 0.0, 0, 2, nullptr);
+    ARTSS_LAUNCH_PDL(ctx, FAM_REDUCE, k_finalize_loop, 1, kReduceThreads, 0, ctx->d_partials, nblocks, ctx->d_loop + slot, 0.0, 0, 2);
     ARTSS_LAUNCH_CK(ctx);
     return ARTSS_OK;
 }
