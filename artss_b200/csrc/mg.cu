@@ -1327,6 +1327,181 @@ k_mg_coarse_jacobi_pipe(TS *__restrict__ out, TS *__restrict__ tmp, const TS *__
     cl.sync();
 }
 
+// ---------------------------------------------------------------- one-block Jacobi coarse solve
+//
+// k_mg_coarse_jacobi_pipe on one block, for levels of a few thousand cells at most: a
+// sweep there is a chain of latencies (the halo copies and the cluster barrier, 1.8 us
+// for 8^3 cells), here two block barriers: one before the boundary program, whose
+// assignments the threads hold in registers, and one after it.  (Targets written by their
+// root's thread, without the first barrier, were slower: a corner's 7 in a row.)
+//  * the residual of iterate k-1 comes out of the pass that computes iterate k, beside
+//    the boundary program, and a warp of its own adds its parts while the others are at
+//    iterate k+1: the decision on iterate k-1 arrives two sweeps late, and four buffers
+//    keep what it may want.
+// Values and iteration count are those of the pipelined form; the residual's sum is
+// taken in another order.
+constexpr int kJbThreads = 992;  // at most, and a warp for the residual
+constexpr int kJbTargets = 2;    // boundary assignments per thread
+// Where the cluster form takes the level too: two solves of 100 sweeps, with the level
+// passes around them, 483 us by the cluster against 332 by the block at 8^3 cells (coarse
+// solve 176 against 101 us), 588 against 500 at 10^3, 621 against 630 at 12^3.  Planes of
+// an odd number of cells have no cluster form: 907 against 449 at 9^3.
+constexpr int kJbPipeCells = 1536;
+
+// S cells per thread
+template <int S>
+__global__ void __launch_bounds__(kJbThreads + 32, 1)
+k_mg_coarse_jacobi_block(double *__restrict__ out, double *__restrict__ tmp, const double *__restrict__ b,
+                         const uint8_t *__restrict__ flags, Level L, Box3 box, MgCoef c, double rx, double ry, double rz,
+                         const __grid_constant__ BcView bc, double tol, long long max_it, LoopState *__restrict__ st) {
+    pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
+    pdl_trigger();
+    extern __shared__ __align__(16) double sm[];
+    __shared__ int s_stop[2];
+    __shared__ double s_sum;
+    const int tid = (int) threadIdx.x, nt = (int) blockDim.x - 32, all = (int) blockDim.x, lane = tid & 31;
+    const int nj = (int) L.Nx, nk = (int) L.nxy(), ntot = (int) L.size();
+    const int n = bc.waves > 0 ? (int) bc.begin[1] : 0;
+    double *X = sm;                           // iterate k in buffer k % 4
+    double *red = X + 4 * ntot;               // [2][256]: the residual's parts
+    if (tid == 0) s_stop[0] = s_stop[1] = 0;
+    for (int q = tid; q < ntot; q += all) X[q] = out[q];
+    __syncthreads();
+    const auto chain = [&](double x, uint32_t d, uint32_t mneg, int q) {
+#pragma unroll
+        for (int e = 0; e < kBcMaxDepth; e++)
+            if (e < (int) d) x = ((mneg >> e) & 1 ? -x : x) + (bc.value ? __ldg(bc.value + e * bc.n + q) : 0.0);
+        return x;
+    };
+    // this thread's assignments: target, root | lagged << 31, depth | neg << 8 | 1 << 31; those of
+    // constant roots are done here
+    constexpr int T = kJbTargets;
+    int bt[T];
+    uint32_t br[T], bd[T];
+#pragma unroll
+    for (int u = 0; u < T; u++) {
+        const int q = tid + u * nt;
+        bt[u] = 0;
+        br[u] = 0;
+        bd[u] = 0;
+        if (tid >= nt || q >= n) continue;
+        const int t = (int) __ldg(bc.target + q), r = (int) __ldg(bc.root + q);
+        const uint32_t db = __ldg(bc.depth + q), d = db & ~(uint32_t) kBcLagged, mneg = __ldg(bc.neg + q);
+        X[t] = chain(out[r], d, mneg, q);  // from before the program, also where X holds a target of it
+        if (!(db & kBcLagged) && !(__ldg(flags + r) & kInner)) continue;
+        bt[u] = t;
+        br[u] = (uint32_t) r | (db & kBcLagged ? 1u << 31 : 0u);
+        bd[u] = d | mneg << 8 | 1u << 31;
+    }
+    __syncthreads();
+    int ca[S];
+    double cb[S];
+    unsigned m0 = 0;
+    const int nx = (int) box.nx(), nxy = (int) (box.nx() * box.ny()), ncell = nxy * (int) box.nz();
+#pragma unroll
+    for (int m = 0; m < S; m++) {
+        const int lin = tid + m * nt;
+        ca[m] = nk;
+        cb[m] = 0.0;
+        if (tid < nt && lin < ncell) {
+            const int r = lin % nxy;
+            const int q = (int) box.x0 + r % nx + nj * ((int) box.y0 + r / nx) + nk * ((int) box.z0 + lin / nxy);
+            if (__ldg(flags + q) & kInner) {
+                ca[m] = q;
+                cb[m] = b[q];
+                m0 |= 1u << m;
+            }
+        }
+    }
+    for (int q = tid; q < ntot; q += all) X[ntot + q] = X[2 * ntot + q] = X[3 * ntot + q] = X[q];
+    __syncthreads();
+
+    double res = 10000.;
+    long long it = 0;
+    if (res > tol && max_it > 0) {
+        const double tol2 = tol * tol;
+        const bool fast = tol2 > 1e-280 && tol2 < 1e280;
+        for (long long k = 1;; k++) {
+            // phase k - 1 has decided on iterate k - 3
+            if (k >= 4 && s_stop[(k - 1) & 1]) {
+                it = k - 3;
+                break;
+            }
+            const double *P = X + (int) ((k - 1) & 3) * ntot, *Q = X + (int) ((k + 2) & 3) * ntot;
+            double *N = X + (int) (k & 3) * ntot;
+            const bool sweep = k <= max_it, resid = k >= 2 && k - 1 <= max_it;
+            double rr[S];
+            if (tid < nt) {
+#pragma unroll
+                for (int m = 0; m < S; m++) {
+                    rr[m] = 0.0;
+                    if (!(m0 >> m & 1)) continue;
+                    const int a = ca[m];
+                    const double c0 = P[a], xm = P[a - 1], xp = P[a + 1], ym = P[a - nj], yp = P[a + nj], zm = P[a - nk],
+                                 zp = P[a + nk];
+                    if (sweep) {
+                        const double out_h =
+                            c.beta * (c.dsign * cb[m] + c.ax * (xp + xm) + c.ay * (yp + ym) + c.az * (zp + zm));
+                        N[a] = c.omw * c0 + c.w * out_h;
+                    }
+                    if (resid) rr[m] = cb[m] - (rx * (xm - 2 * c0 + xp) + ry * (ym - 2 * c0 + yp) + rz * (zm - 2 * c0 + zp));
+                }
+            }
+            if (sweep) __syncthreads();  // the roots' new values are in N
+            if (tid < nt) {
+                if (sweep) {
+#pragma unroll
+                    for (int u = 0; u < T; u++)
+                        if (bd[u])
+                            N[bt[u]] = chain((br[u] >> 31 ? Q : N)[br[u] & 0x7fffffffu], bd[u] & 0xffu, bd[u] >> 8 & 0xffu,
+                                             tid + u * nt);
+                }
+                double acc = 0.0;
+#pragma unroll
+                for (int m = 0; m < S; m++) acc += rr[m] * rr[m];
+                if (resid) {
+                    acc += __shfl_xor_sync(~0u, acc, 1);
+                    acc += __shfl_xor_sync(~0u, acc, 2);
+                    if (!(lane & 3)) red[(int) (k & 1) * 256 + (tid >> 2)] = acc;
+                }
+            } else if (k >= 3 && k - 2 <= max_it) {
+                const double *r = red + (int) ((k - 1) & 1) * 256;
+                double v = 0.0;
+                for (int q = lane; q < nt / 4; q += 32) v += r[q];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(~0u, v, o);
+                // res > tol on the squared sum where that is exact, as the pipelined form
+                bool above;
+                if (fast && v > tol2 * (1.0 + 0x1p-49)) above = true;
+                else if (fast && v < tol2 * (1.0 - 0x1p-49)) above = false;
+                else above = sqrt(v) > tol;
+                if (lane == 0) {
+                    s_sum = v;
+                    s_stop[k & 1] = !(above && k - 2 < max_it);
+                }
+            }
+            __syncthreads();
+        }
+        res = sqrt(s_sum);
+    }
+    // after `it` swaps out holds iterate it when it is odd and it-1 when it is even
+    const double *Xo = X + (int) (it & 3) * ntot, *Xt = Xo;
+    if (it >= 1) {
+        const double *prev = X + (int) ((it - 1) & 3) * ntot;
+        if (it % 2 == 0) Xo = prev;
+        else Xt = prev;
+    }
+    for (int q = tid; q < ntot; q += all) {
+        out[q] = Xo[q];
+        if (tmp) tmp[q] = Xt[q];
+    }
+    if (tid == 0 && st) {
+        st->it = it;
+        st->residual = res;
+        st->cond = 0;
+    }
+}
+
 // Launch shape of the cluster coarse solve, or false when the level does not fit it.
 // ranks of the cluster for a level: one per z-plane up to kClusterSize
 inline int cluster_ranks(const Level &L) { return (int) std::min<int64_t>(kClusterSize, L.Nz); }
@@ -1577,6 +1752,43 @@ BcView pipe_view(const artss_ctx *ctx, int level) {
     return v;
 }
 
+// cells per thread of k_mg_coarse_jacobi_block for a level, 0 where it is not taken
+int coarse_block_slots(const artss_ctx *ctx, int level, int64_t *smem) {
+    const Level &L = ctx->lvl[level];
+    const BcProgram &p = ctx->bc[level][ARTSS_FIELD_P];
+    if (p.present && p.waves > 1 && !p.flat.n) return 0;
+    const BcView v = pipe_view(ctx, level);
+    const Box3 box = inner_box(L);
+    const int64_t cells = box.nx() * box.ny() * box.nz();
+    *smem = (4 * L.size() + 512) * (int64_t) sizeof(double);
+    if (*smem > kCoarseSmemBytes) return 0;
+    for (int s : {1, 2})
+        if (cells <= (int64_t) s * kJbThreads && v.n <= kJbTargets * (((cells + s - 1) / s + 31) / 32 * 32)) return s;
+    return 0;
+}
+
+template <int S>
+int launch_coarse_jacobi_block(artss_ctx *ctx, double *out, double *tmp, const double *b, int level, const MgCoef &c,
+                               double rx, double ry, double rz, double tol, long long mi, int64_t smem, LoopState *st) {
+    static bool attr_set = false;
+    if (!attr_set) {
+        ARTSS_CK(cudaFuncSetAttribute(k_mg_coarse_jacobi_block<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int) kCoarseSmemBytes));
+        attr_set = true;
+    }
+    const Level &L = ctx->lvl[level];
+    const Box3 box = inner_box(L);
+    const BcProgram &prog = ctx->bc[level][ARTSS_FIELD_P];
+    BcView v = pipe_view(ctx, level);
+    if (prog.present && prog.zero_values) v.value = nullptr;
+    const int64_t per = (box.nx() * box.ny() * box.nz() + S - 1) / S;
+    ARTSS_LAUNCH_PDL(ctx, FAM_MG_COARSE, k_mg_coarse_jacobi_block<S>, 1, (unsigned) ((per + 31) / 32 * 32 + 32), smem, out,
+                     tmp, b, (const uint8_t *) ctx->d_flags[level], L, box, c, rx, ry, rz, v, tol, mi,
+                     st);
+    ARTSS_LAUNCH_CK(ctx);
+    return ARTSS_OK;
+}
+
 // out = 0 (the coarse solve's start on the cluster path)
 __global__ void k_fill_f32(float *__restrict__ f, int64_t n, const LoopState *__restrict__ pred) {
     pdl_wait();  // launched by launch_pdl: the predecessor's writes are visible after this
@@ -1706,9 +1918,17 @@ int mg_coarse_solve(artss_mg *mg, double *out, double *tmp, const double *b, int
     int cap = 0;
     int64_t csmem = 0;
     PipeLaunch pl{};
-    if (mg->cluster_coarse && !cgs && mg->pipelined_coarse && coarse_pipe_plan(ctx, level, &pl))
-        return launch_coarse_pipe<double>(ctx, out, tmp, b, level, c, rx, ry, rz, pipe_view(ctx, level), tol, 0, mi, pl,
-                                          ctx->d_loop + 1, nullptr);
+    if (mg->cluster_coarse && !cgs && mg->pipelined_coarse) {
+        int64_t bsmem = 0;
+        const int slots = coarse_block_slots(ctx, level, &bsmem);
+        const auto go = slots == 1 ? launch_coarse_jacobi_block<1> : launch_coarse_jacobi_block<2>;
+        const bool pipe = coarse_pipe_plan(ctx, level, &pl);
+        if (slots && (!pipe || box.nx() * box.ny() * box.nz() <= kJbPipeCells))
+            return go(ctx, out, tmp, b, level, c, rx, ry, rz, tol, mi, bsmem, ctx->d_loop + 1);
+        if (pipe)
+            return launch_coarse_pipe<double>(ctx, out, tmp, b, level, c, rx, ry, rz, pipe_view(ctx, level), tol, 0, mi,
+                                              pl, ctx->d_loop + 1, nullptr);
+    }
     if (mg->cluster_coarse && cluster_fits(ctx, level, cgs ? 1 : 2, &cap, &csmem)) {
         if (cgs)
             return launch_coarse_cluster<true, double>(ctx, out, tmp, b, level, c, rx, ry, rz, v, tol, 0, mi, cap, csmem,
