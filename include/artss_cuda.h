@@ -264,10 +264,11 @@ int artss_get_cell_flags(artss_ctx *ctx, int level, uint8_t *host_out, int64_t n
 /* Replaces Multigrid::apply_boundary_condition's per-patch loops
  * (src/domain/Multigrid.cpp:555-572): the ordered assignments for one field
  * type on one level (obstacles in id order, then domain patches
- * left..back).  The library compiles them into dependency-free waves. */
+ * left..back).  The library compiles them into dependency-free waves, and
+ * several waves into a flat form that runs as one launch. */
 int artss_set_boundary_program(artss_ctx *ctx, int level, int field_type,
                                const artss_bc_assign *ops, int64_t n_ops);
-/* Number of kernel waves the compiled program of (level, field_type) needs. */
+/* Number of dependency-free waves in the compiled program of (level, field_type). */
 int artss_boundary_program_waves(artss_ctx *ctx, int level, int field_type);
 
 /* DomainController::apply_boundary (src/domain/DomainController.cpp:145-147). */
@@ -315,7 +316,7 @@ int artss_turb_const_smagorinsky(artss_ctx *ctx, double *nu_t,
  * reference's filters, its in-place 27-cell averaging of the coefficient in
  * list order and ev = 0 where ev + nu < 0; no boundary program (the reference
  * applies none).  The first call (or the first after the cell lists or
- * boundary programs changed) sets up 40 level-0 work arrays and must not be
+ * boundary programs changed) sets up 11 level-0 work arrays and must not be
  * inside a stream capture. */
 int artss_turb_dynamic_smagorinsky(artss_ctx *ctx, double *nu_t, const double *u, const double *v,
                                    const double *w, double nu);
