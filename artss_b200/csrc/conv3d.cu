@@ -9,30 +9,40 @@
 //
 // GEMM view of the forward pass: M = 128 output voxels (8 in x, 16 in y), a
 // block owns `zb` such planes above one another and `nt` output channels, K = 27
-// taps x C_in.  Per 16 input channels the block's input planes with their halo
-// (10 x 18 x (zb + 2) voxels) and the weights are brought into shared memory
-// ONCE, as 16-byte pieces [z][channel / 8][y][x][8 channels] by cp.async (zero
-// filled outside the grid, which is the padding).  In that no-swizzle layout the
-// 8 rows of a core matrix are 8 neighbours in x and the 16 groups lie one y row
-// apart, so every tap is the same tile at another start address: the tap needs no
-// copy of its own.  The three taps of a (dy, dx) pair that differ in dz read the
-// same input plane and write three neighbouring output planes, whose accumulators
-// lie side by side in tensor memory: one MMA with N = 3 nt does all three, so the
-// A tile, whose reading bounds these narrow layers (4 KB per MMA, 32 cycles, more
-// than the arithmetic for N < 128), is read 9 instead of 27 times per plane.
+// taps x C_in.  Input planes with their halo (10 x 18 voxels, all C_in channels)
+// arrive in shared memory ONCE, `pz` planes to a step, as 16-byte pieces
+// [z][channel / 8][y][x][8 channels] by cp.async (zero filled outside the grid, which
+// is the padding).  In that no-swizzle layout the 8 rows of a core matrix are 8
+// neighbours in x and the 16 groups lie one y row apart, so every tap is the same
+// tile at another start address: the tap needs no copy of its own.  The three taps of
+// a (dy, dx) pair that differ in dz read the same input plane and write three
+// neighbouring output planes, whose accumulators lie side by side in tensor memory:
+// one MMA with N = 3 nt does all three, so the A tile, whose reading bounds these
+// narrow layers (4 KB per MMA, 32 cycles, more than the arithmetic for N < 128), is
+// read 9 instead of 27 times per plane.
 //
-// The accumulators start from zero (tcgen05.st); the epilogue adds the bias,
-// clamps and stores.  Several blocks share a multiprocessor, so that one block's
-// loads and epilogue run under another's MMAs; zb, nt and the number of stages
-// follow from a cost model of the two (conv_plan).  Measured at 64 x 64 x 128, 16 ->
-// 16 channels: 25 us (293 TFLOP/s), 48 -> 16: 56 us (390); with one TMA copy of the
-// tile per tap, 256 rows of 16 bytes at some four cycles each, the ten layers of the
-// network took 3008 us, now 260.
+// The order of the sum is part of the result: FP32 accumulation rounds after each
+// MMA, the next layer rounds to BF16, and ten layers and a training step magnify the
+// last bit (to 0.8 % of an output after two steps on 21 networks, 9.6 % at worst seen).  An output adds its products tap by
+// tap, t = 0 .. 26, and within a tap 16 input channels at a time: planes in the order
+// of z, for each its 9 taps, for each all its channels.  So the channels of a plane
+// have to be in shared memory together.
+//
+// The weights stay for all of a block's planes where they fit beside them; else a block
+// owns one output plane and the weights of a dz arrive with its input plane.  Several
+// blocks share a multiprocessor, so that one block's loads and epilogue run under
+// another's MMAs (a ring of stages within a block took the room of a second block and
+// was slower).  The accumulators start from zero (tcgen05.st); the epilogue adds the
+// bias, clamps and stores.  zb, nt and pz follow from a cost model (conv_plan).
+// Measured at 64 x 64 x 128, 16 -> 16 channels: 27 us (272 TFLOP/s), 48 -> 16: 58 us
+// (377); 32 x 32 x 64, 96 -> 32: 33 us.  With all taps of 16 channels before the next 16,
+// in another order then, 25, 57 and 34 us.
 //
 // Every wait is bounded and raises an error flag.
 #include "internal.cuh"
 #include "tc.cuh"
 
+#include <cmath>
 #include <cuda_bf16.h>
 
 namespace artss {
@@ -42,6 +52,7 @@ namespace {
 constexpr int kConvPolls = 1 << 20;
 constexpr int kConvThreads = 256;
 constexpr size_t kConvSmemMax = 227 * 1024 - 1024;  // dynamic limit minus the kernels' static shared memory
+constexpr int64_t kConvSmemSm = 228 * 1024;         // of a multiprocessor
 constexpr int kTx = 8, kTy = 16;                    // output voxels of one MMA (M = 128)
 constexpr int kHx = kTx + 2, kHy = kTy + 2;         // with halo
 constexpr unsigned kRowB = kHx * 16;                // bytes between y rows of a channel group
@@ -84,18 +95,17 @@ __device__ __forceinline__ void load_halo(uint32_t dst, const __nv_bfloat16 *__r
     }
 }
 
-struct ConvPlan {
-    int zb, nt, stages, tiles_z, cols;
-    unsigned a_bytes, b_bytes;
-    size_t smem;
-};
-
+// KK: C_in / 16 where it is known when compiled (0: any).  One thread issues the MMAs, a
+// tap and 16 channels each some 40 cycles of the tensor core: with the channel loop
+// unrolled the operands' descriptors are one addition each (64 x 64 x 128, 16 -> 16
+// channels: 25 us, 33 with a loop and its products).
+template <int KK>
 __global__ void __launch_bounds__(kConvThreads)
 k_conv3d_fwd(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ wp,
              const float *__restrict__ bias, __nv_bfloat16 *__restrict__ y, ConvShape s, ConvPlan p, int relu,
              int *__restrict__ err) {
     extern __shared__ __align__(128) uint8_t cv_sm[];
-    __shared__ __align__(8) uint64_t done[2];  // the MMAs of the stage's last use have completed
+    __shared__ __align__(8) uint64_t done;  // the step's MMAs have completed
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tile = (int) blockIdx.x;
@@ -103,27 +113,31 @@ k_conv3d_fwd(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restric
               z0 = (tile / (s.tiles_x * s.tiles_y)) * p.zb;
     const int n0 = (int) blockIdx.y * p.nt;
     const int zb = min(p.zb, s.D - z0);  // output planes of this block
-    const int nt = p.nt, chunks = s.cin / 16;
+    const int nt = p.nt, groups = KK ? 2 * KK : s.cin / 8;
+    const int steps = (zb + 2 + p.pz - 1) / p.pz;
+    const int wrows = p.resident ? 3 * nt : nt;  // rows of the B operand of a tap's dz
+    const unsigned tap_bytes = (unsigned) (groups * wrows * 16), plane_bytes = (unsigned) groups * kGroupB;
     const uint32_t base = tc::smem_addr(cv_sm);
-    const unsigned stage_bytes = p.a_bytes + p.b_bytes;
 
-    // input planes z0 - 1 .. z0 + zb and the weights of input channels 16 c ..: the
-    // weights as [dy dx][channel / 8][dz][nt][8], dz descending, so that any run of
-    // dz is one operand of neighbouring rows
-    auto load = [&](int c) {
-        const uint32_t a = base + (uint32_t) (c % p.stages) * stage_bytes, b = a + p.a_bytes;
-        load_halo(a, x, s, x0, y0, z0, zb + 2, 2 * c, 2, tid);
-        for (int e = tid; e < 54 * nt; e += kConvThreads) {
-            const int n = e % nt, kc = (e / nt) & 1, tap = e / (2 * nt);
-            const int dz = tap / 9, t9 = tap % 9;
-            cp_async16(b + (uint32_t) ((t9 * 2 + kc) * 3 * nt + (2 - dz) * nt + n) * 16,
-                       wp + (((size_t) tap * (s.cin / 8) + 2 * c + kc) * s.cout + n0 + n) * 8, true);
+    // input planes z0 - 1 + q, q = pz step ..; and the weights of dz = q - 1 for q < 3 as
+    // [dy dx][channel / 8][dz][nt][8], dz descending, so that any run of dz is one operand
+    // of neighbouring rows (an output plane has dz = q - 1 of step q's planes or an earlier one's)
+    auto load = [&](int step) {
+        const uint32_t a = base + p.w_bytes;
+        const int q0 = step * p.pz, q1 = min(q0 + p.pz, zb + 2);
+        load_halo(a, x, s, x0, y0, z0 + q0, q1 - q0, 0, groups, tid);
+        for (int dz = q0; dz < min(q1, 3); dz++) {
+            const uint32_t b = p.resident ? base + (uint32_t) ((2 - dz) * nt * 16) : a + p.a_bytes;
+            for (int e = tid; e < 9 * groups * nt; e += kConvThreads) {
+                const int n = e % nt, kc = (e / nt) % groups, t9 = e / (nt * groups);
+                cp_async16(b + (uint32_t) t9 * tap_bytes + (uint32_t) (kc * wrows + n) * 16,
+                           wp + (((size_t) (9 * dz + t9) * groups + kc) * s.cout + n0 + n) * 8, true);
+            }
         }
     };
     load(0);
     if (tid == 0) {
-        tc::mbar_init(&done[0], 1);
-        tc::mbar_init(&done[1], 1);
+        tc::mbar_init(&done, 1);
         tc::fence_barrier_init();
     }
     if (warp == 0) {
@@ -140,39 +154,44 @@ k_conv3d_fwd(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restric
     tc::tc_fence_before();
 
     bool ok = true;
-    for (int c = 0; c < chunks && ok; c++) {
+    for (int c = 0; c < steps && ok; c++) {
+        if (c > 0) {
+            ok = tc::mbar_wait(&done, (unsigned) ((c - 1) & 1), kConvPolls);
+            if (ok) load(c);
+            // no thread leaves the loop before the others have seen the same
+            ok = !__syncthreads_or(!ok);
+            if (!ok) break;
+        }
         cp_async_done();
         tc::fence_proxy_async();  // this thread's pieces, before the tensor core reads them
         __syncthreads();
         if (tid == 0) {
             tc::tc_fence_after();
-            const uint8_t *a = cv_sm + (size_t) (c % p.stages) * stage_bytes, *b = a + p.a_bytes;
-            for (int q = 0; q < zb + 2; q++) {
+            const uint8_t *a = cv_sm + p.w_bytes;
+            const uint8_t *b = p.resident ? cv_sm : a + p.a_bytes;
+            for (int q = c * p.pz; q < min((c + 1) * p.pz, zb + 2); q++) {
                 // input plane q feeds output planes q - 2 (dz = +1), q - 1, q (dz = -1)
                 const int lo = max(0, q - 2), hi = min(zb - 1, q), nz = hi - lo + 1;
                 const int gz = z0 - 1 + q;
                 if (gz < 0 || gz >= s.D) continue;  // padding adds nothing
                 const uint32_t idesc = tc::idesc_bf16(128, nz * nt, 0, 0);
-                const uint8_t *aq = a + (size_t) q * 2 * kGroupB, *bq = b + (size_t) (lo - q + 2) * nt * 16;
+                // descriptors count 16 bytes
+                const uint64_t a0 = tc::smem_desc(a + (size_t) (q - c * p.pz) * plane_bytes, kGroupB, kRowB);
+                const uint64_t b0 = tc::smem_desc(b + (p.resident ? (size_t) (lo - q + 2) * nt * 16 : 0),
+                                                  (unsigned) (wrows * 16), 128);
+                uint64_t db = b0;
 #pragma unroll
-                for (int t = 0; t < 9; t++)
-                    tc::mma_bf16(tmem + (uint32_t) (lo * nt),
-                                 tc::smem_desc(aq + (t / 3) * kRowB + (t % 3) * 16, kGroupB, kRowB),
-                                 tc::smem_desc(bq + (size_t) t * 6 * nt * 16, (unsigned) (3 * nt * 16), 128), idesc, 1);
+                for (int t = 0; t < 9; t++) {
+                    const uint64_t da = a0 + ((t / 3) * kRowB + (t % 3) * 16) / 16;
+#pragma unroll
+                    for (int kk = 0; kk < groups / 2; kk++, db += 2 * (unsigned) wrows)  // a tap's channel groups follow the last one's
+                        tc::mma_bf16(tmem + (uint32_t) (lo * nt), da + (uint64_t) (kk * (2 * kGroupB / 16)), db, idesc, 1);
+                }
             }
-            tc::mma_commit(&done[c % p.stages]);
-        }
-        const int n = c + 1;
-        if (n < chunks) {
-            // the stage of chunk n was last read by the MMAs of chunk n - stages
-            const int u = n - p.stages;
-            if (u >= 0) ok = tc::mbar_wait(&done[u % p.stages], (unsigned) ((u / p.stages) & 1), kConvPolls);
-            if (ok) load(n);
-            // no thread leaves the loop before the others have seen the same
-            ok = !__syncthreads_or(!ok);
+            tc::mma_commit(&done);
         }
     }
-    if (ok) ok = tc::mbar_wait(&done[(chunks - 1) % p.stages], (unsigned) (((chunks - 1) / p.stages) & 1), kConvPolls);
+    if (ok) ok = tc::mbar_wait(&done, (unsigned) ((steps - 1) & 1), kConvPolls);
     if (__syncthreads_or(!ok)) {
         if (tid == 0 && err) atomicExch(err, 1);
         cp_async_done();
@@ -351,37 +370,47 @@ int conv_shape(const artss_conv_desc *d, ConvShape *s) {
     return ARTSS_OK;
 }
 
-// zb and nt of the forward kernel: the pair with the least
-//     waves x (shared-memory cycles of its MMAs + cycles of its loads)
-// where one MMA reads 4 KB of A and 96 nt bytes of B at 128 bytes a cycle and
-// loads arrive at some 48 bytes a cycle and multiprocessor.  At 64 x 64 x 128
-// this takes 8 planes for the 16-channel layers (512 blocks, 3 a multiprocessor)
-// and 1 plane with 32 of the 64 channels on 16 x 16 x 32 (128 blocks: 64 with all
-// channels would leave half of the chip idle).
+// The forward kernel's plan: the one with the least time by a model of its parts, whose
+// weights (microseconds) were fitted to the times of up to 90 plans for each of 15 layers
+// from 8 x 8 x 16 to 64 x 64 x 128 voxels, 16 to 96 channels.  Rounds: of blocks that
+// run side by side; a step is a wait for loads and two barriers, an MMA its issue and its
+// operands.  A plan that leaves a multiprocessor to one block counts 1.3 times, and
+// shared memory counts a little, as blocks of other streams run beside these: over the
+// 15 layers the choice is 2.5 % (at most 9 %) off the fastest plan on one stream and 5 %
+// on three, without these two 1 % and 20 %.
 ConvPlan conv_plan(const ConvShape &s, int sms) {
     ConvPlan best{};
     double least = 0;
-    for (int zb = 8; zb >= 1; zb /= 2)
-        for (int nt = channel_tile(s.cout, 64); nt >= 16; nt = nt > 16 ? channel_tile(s.cout, nt - 16) : 0) {
-            ConvPlan p{};
-            p.zb = zb;
-            p.nt = nt;
-            p.tiles_z = (s.D + zb - 1) / zb;
-            p.cols = tmem_cols(zb * nt);
-            p.a_bytes = (unsigned) (zb + 2) * 2 * kGroupB;
-            p.b_bytes = (unsigned) (54 * nt * 16);
-            const size_t stage = p.a_bytes + p.b_bytes;
-            if (p.cols > 256 || stage > kConvSmemMax / 2) continue;  // two blocks a multiprocessor
-            p.stages = s.cin > 16 && 2 * stage <= kConvSmemMax / 2 ? 2 : 1;
-            p.smem = p.stages * stage;
-            const int64_t blocks = (int64_t) s.tiles_x * s.tiles_y * p.tiles_z * (s.cout / nt);
-            const double cost = (double) ((blocks + sms - 1) / sms) *
-                                ((zb + 2) * 9. * (32. + 0.75 * nt) + (double) stage / 48.);
-            if (least == 0 || cost < least) {
-                least = cost;
-                best = p;
-            }
-        }
+    const unsigned plane = (unsigned) s.cin / 8 * kGroupB;
+    for (int resident = 1; resident >= 0; resident--)
+        for (int zb = resident ? 8 : 1; zb >= 1; zb /= 2)
+            for (int nt = channel_tile(s.cout, 64); nt >= 16; nt = nt > 16 ? channel_tile(s.cout, nt - 16) : 0)
+                for (int pz = resident ? zb + 2 : 1; pz >= 1; pz--) {
+                    ConvPlan p{};
+                    p.zb = zb;
+                    p.nt = nt;
+                    p.pz = pz;
+                    p.resident = resident;
+                    p.tiles_z = (s.D + zb - 1) / zb;
+                    p.cols = tmem_cols(zb * nt);
+                    const unsigned dz = (unsigned) (9 * s.cin * nt * 2);  // the weights of one dz
+                    p.w_bytes = resident ? 3 * dz : 0;
+                    p.a_bytes = (unsigned) pz * plane;
+                    p.smem = (size_t) p.w_bytes + p.a_bytes + (resident ? 0 : dz);
+                    if (p.cols > 256 || p.smem > kConvSmemMax) continue;
+                    const int64_t blocks = (int64_t) s.tiles_x * s.tiles_y * p.tiles_z * (s.cout / nt);
+                    const int64_t share = std::min<int64_t>(kConvSmemSm / (int64_t) (p.smem + 1024), 512 / p.cols);
+                    const double waves = (double) ((blocks + sms - 1) / sms);
+                    const double rounds = std::max(1., (double) blocks / (double) (sms * share));
+                    const double mmas = (zb + 2) * 9. * (s.cin / 16), rows = (resident ? 3. : 1.) * nt;
+                    const double steps = (zb + 2 + pz - 1) / pz, bytes = (zb + 2) * (double) plane + 3. * dz;
+                    const double us = rounds * (1.9 * steps + 0.026 * mmas) + waves * (1.2e-4 * mmas * rows + 4.7e-5 * bytes);
+                    const double cost = us * (share > 1 ? 1. : 1.3) * std::pow((double) p.smem, 0.12);
+                    if (least == 0 || cost < least) {
+                        least = cost;
+                        best = p;
+                    }
+                }
     return best;
 }
 
@@ -423,10 +452,19 @@ int conv3d_fwd(artss_ctx *ctx, const artss_conv_desc *d, const void *x, const vo
     if (((uintptr_t) x & 15) || ((uintptr_t) wp & 15) || ((uintptr_t) y & 15)) {
         set_error("conv3d: arrays must be 16-byte aligned"); return ARTSS_ERR_ARG;
     }
-    const ConvPlan p = conv_plan(s, std::max(ctx->sm_count, 1));
-    ARTSS_CK(cudaFuncSetAttribute(k_conv3d_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kConvSmemMax));
+    // the search takes some microseconds: a context keeps the plans of its layers
+    const std::array<int, 5> key{s.D, s.H, s.W, s.cin, s.cout};
+    auto known = ctx->conv_plans.find(key);
+    if (known == ctx->conv_plans.end()) {
+        if (ctx->conv_plans.size() >= 256) ctx->conv_plans.clear();
+        known = ctx->conv_plans.emplace(key, conv_plan(s, std::max(ctx->sm_count, 1))).first;
+    }
+    const ConvPlan p = known->second;
+    const auto kernel = s.cin == 16 ? k_conv3d_fwd<1> : s.cin == 32 ? k_conv3d_fwd<2> : s.cin == 48 ? k_conv3d_fwd<3>
+                      : s.cin == 64 ? k_conv3d_fwd<4> : s.cin == 96 ? k_conv3d_fwd<6> : k_conv3d_fwd<0>;
+    ARTSS_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kConvSmemMax));
     const dim3 grid((unsigned) (s.tiles_x * s.tiles_y * p.tiles_z), (unsigned) (s.cout / p.nt));
-    ARTSS_LAUNCH(ctx, FAM_CONV, k_conv3d_fwd<<<grid, kConvThreads, p.smem, ctx->stream>>>(
+    ARTSS_LAUNCH(ctx, FAM_CONV, kernel<<<grid, kConvThreads, p.smem, ctx->stream>>>(
                                     (const __nv_bfloat16 *) x, (const __nv_bfloat16 *) wp, bias, (__nv_bfloat16 *) y, s,
                                     p, d->relu, &ctx->d_loop[kNnErrSlot].pad));
     ARTSS_LAUNCH_CK(ctx);

@@ -6,6 +6,7 @@
 
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <array>
 #include <cstdint>
 #include <condition_variable>
 #include <map>
@@ -117,6 +118,17 @@ struct LoopState {
     int blocks_done;   // blocks done, for a kernel whose last block does the loop step; 0 between launches
 };
 
+// How a forward convolution is cut into blocks and steps (conv3d.cu).
+struct ConvPlan {
+    int zb, nt;       // output planes and channels of a block
+    int pz;           // input planes of a step
+    int resident;     // the weights of all taps stay in shared memory
+    int tiles_z, cols;
+    unsigned w_bytes;  // resident weights, then
+    unsigned a_bytes;  // the step's input planes, then (not resident) the weights of its dz
+    size_t smem;
+};
+
 // Kernel families for launch counting and event timing (artss_ctx_profile).
 enum Family : int {
     FAM_ADVECT = 0, FAM_SMAGORINSKY, FAM_DIVERGENCE, FAM_PROJECTION, FAM_BUOYANCY, FAM_ADD_SOURCE,
@@ -190,6 +202,7 @@ struct artss_ctx {
     float *cgsm_w = nullptr;                                     // FP32 defect / correction of artss_diffuse_cgs_mixed
     int64_t cgsm_n = 0;
     std::map<artss::TuneKey, int> tuned;                         // autotuned variant per kernel and shape
+    std::map<std::array<int, 5>, artss::ConvPlan> conv_plans;    // per D, H, W, C_in, C_out
     // host transfers overlapped with the step: a second stream, completion
     // events of its uploads by slot, a mark of the main stream, its tail
     // whole-step capture (artss_graph_begin .. artss_graph_end): loops become
