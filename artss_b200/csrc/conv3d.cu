@@ -234,11 +234,17 @@ k_conv3d_fwd(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restric
 // (SBO); the channel groups of planes z - 1, z, z + 1 follow one another at the
 // same distance, so the three dz taps are one operand of N = 3 ct columns and an
 // x tile is loaded once for all its taps (before: one 256-row copy per tap).
-// A block accumulates `tg` (dy, dx) pairs for `ct` input channels over all its
-// voxel tiles in tensor memory and adds them to dW once, with FP32 atomics (dW
-// must be zeroed by the caller).
+// A block accumulates `tg` (dy, dx) pairs for `ct` input channels over `chain` of its
+// voxel tiles in tensor memory and adds them to dW with FP32 atomics (dW must be
+// zeroed by the caller), then starts the next ones from zero.  FP32 accumulation in
+// tensor memory rounds towards zero, so a sum's error grows with the length of the
+// chain and not with its root: at 56 x 64 x 128, 48 -> 16 channels, 592 MMAs in a row
+// were off by 8.9e-6, 200 are by 2.5e-6.  The chains' sums are added up in shared memory
+// where that has room, else every one goes to dW.
 struct WgradPlan {
-    int ct, tg, groups, tiles_z, cols;  // groups of (dy, dx) pairs
+    int ct, tg, groups, cols;  // groups of (dy, dx) pairs
+    int chain;                 // voxel tiles summed in tensor memory at a time
+    unsigned sums;             // where the chains' sums lie in shared memory [column][C_out], 0: nowhere
     unsigned a_bytes, b_bytes;
     size_t smem;
 };
@@ -286,6 +292,30 @@ k_conv3d_wgrad(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restr
     tc::tc_fence_after();
     const uint32_t tmem = tmem_base;
     const uint32_t idesc = tc::idesc_bf16(128, 3 * p.ct, 1, 1);
+    // lane = output channel co, columns = (pair, dz, input channel); a column of a lane
+    // is always the same thread's
+    auto drain = [&](bool first, bool last) {
+        tc::tc_fence_after();
+        const int co = 32 * (warp & 3) + lane;
+        const uint32_t src = tmem + ((uint32_t) (32 * (warp & 3)) << 16);
+        float *sums = (float *) (cv_sm + p.sums);
+        const int nc = nt * 3 * p.ct / 16;
+        if (32 * (warp & 3) < s.cout)
+            for (int q = warp >> 2; q < nc; q += 2) {
+                const int c = 16 * q, pair = t0 + c / (3 * p.ct), dz = c / p.ct % 3, ci = ci0 + c % p.ct;
+                float v[16];
+                tc::tmem_ld16(src + (uint32_t) c, v);
+                if (co >= s.cout) continue;
+                float *d = dw + ((size_t) (9 * dz + pair) * s.cout + co) * s.cin + ci, *m = sums + c * s.cout + co;
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    if (p.sums && !first) v[i] += m[i * s.cout];
+                    if (p.sums && !last) m[i * s.cout] = v[i];
+                    else atomicAdd(d + i, v[i]);
+                }
+            }
+        tc::tc_fence_before();
+    };
     bool ok = true;
     for (int it = 0; it < my_tiles && ok; it++) {
         cp_async_done();
@@ -300,7 +330,7 @@ k_conv3d_wgrad(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restr
                 for (int kk = 0; kk < kTy / 2; kk++)  // 16 voxels (two y rows) per MMA
                     tc::mma_bf16(tmem + (uint32_t) (t * 3 * p.ct),
                                  tc::smem_desc(a + kk * 2 * kTx * 16, kTx * 16, kTx * kTy * 16),
-                                 tc::smem_desc(bt + kk * 2 * kRowB, kRowB, kGroupB), idesc, (it | kk) != 0);
+                                 tc::smem_desc(bt + kk * 2 * kRowB, kRowB, kGroupB), idesc, (it % p.chain | kk) != 0);
             }
             tc::mma_commit(&done[it & 1]);
         }
@@ -310,29 +340,15 @@ k_conv3d_wgrad(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restr
             if (ok) load(n);
             ok = !__syncthreads_or(!ok);
         }
+        if (ok && (n == my_tiles || n % p.chain == 0)) {
+            ok = tc::mbar_wait(&done[it & 1], (unsigned) ((it >> 1) & 1), kConvPolls);
+            ok = !__syncthreads_or(!ok);
+            if (ok) drain(it < p.chain, n == my_tiles);  // before the next chain's MMAs: the barrier above them
+        }
     }
-    if (ok) ok = tc::mbar_wait(&done[(my_tiles - 1) & 1], (unsigned) (((my_tiles - 1) >> 1) & 1), kConvPolls);
-    if (__syncthreads_or(!ok)) {
+    if (!ok) {
         if (tid == 0 && err) atomicExch(err, 1);
         cp_async_done();
-    } else {
-        tc::tc_fence_after();
-        // lane = output channel co, columns = (pair, dz, input channel)
-        const int co = 32 * (warp & 3) + lane;
-        const uint32_t src = tmem + ((uint32_t) (32 * (warp & 3)) << 16);
-        const int nc = nt * 3 * p.ct / 16;
-        if (32 * (warp & 3) < s.cout)
-            for (int q = warp >> 2; q < nc; q += 2) {
-                const int c = 16 * q, pair = t0 + c / (3 * p.ct), dz = c / p.ct % 3, ci = ci0 + c % p.ct;
-                float v[16];
-                tc::tmem_ld16(src + (uint32_t) c, v);
-                if (co < s.cout) {
-                    float *d = dw + ((size_t) (9 * dz + pair) * s.cout + co) * s.cin + ci;
-#pragma unroll
-                    for (int i = 0; i < 16; i++) atomicAdd(d + i, v[i]);
-                }
-            }
-        tc::tc_fence_before();
     }
     __syncthreads();
     tc::tc_fence_after();
@@ -437,7 +453,14 @@ int conv3d_wgrad(artss_ctx *ctx, const artss_conv_desc *d, const void *x, const 
     ARTSS_CK(cudaFuncSetAttribute(k_conv3d_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kConvSmemMax));
     const int tiles = s.tiles_x * s.tiles_y * s.D, yb = p.groups * (s.cin / p.ct);
     // one block a multiprocessor (tensor memory), the parts of dW side by side
-    const int gx = std::max(1, std::min(tiles, std::max(ctx->sm_count, 1) / yb));
+    const int sms = std::max(ctx->sm_count, 1), gx = std::max(1, std::min(tiles, sms / yb));
+    // as many tiles as a block would have if every one had all of dW
+    p.chain = (tiles + sms - 1) / sms;
+    const size_t sums = (size_t) p.tg * 3 * p.ct * s.cout * sizeof(float);
+    if ((tiles + gx - 1) / gx > p.chain && p.smem + sums <= kConvSmemMax) {
+        p.sums = (unsigned) p.smem;
+        p.smem += sums;
+    }
     ARTSS_LAUNCH(ctx, FAM_CONV, k_conv3d_wgrad<<<dim3((unsigned) gx, (unsigned) yb), kConvThreads, p.smem, ctx->stream>>>(
                                     (const __nv_bfloat16 *) x, (const __nv_bfloat16 *) dy, dw, s, p,
                                     &ctx->d_loop[kNnErrSlot].pad));
