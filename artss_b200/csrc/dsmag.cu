@@ -269,6 +269,7 @@ __device__ __forceinline__ double div27(double x) {
 constexpr int kAvG = 8, kAvRing = 32, kAvPitch = 33;  // an odd pitch spreads the rows over the banks
 constexpr int kAvRows = 512, kAvLoaders = 128;        // rows (threads) of a block at most; loading threads
 constexpr int kAvPolls = 1 << 20;
+constexpr size_t kAvSmemMax = 225 * 1024;             // of a block at most
 
 inline size_t av_smem(int ny, int kn) { return (size_t) (kn + 2) * (ny + 2) * kAvPitch * sizeof(double); }
 
@@ -508,7 +509,7 @@ int ds_average_planes(const Box3 &box, int sms) {
     const int64_t ny = box.ny(), nz = box.nz();
     if (ny > kAvRows) return 0;
     int64_t K = std::min<int64_t>(nz, kAvRows / ny);
-    while (K > 0 && av_smem((int) ny, (int) K) > 225 * 1024) K--;
+    while (K > 0 && av_smem((int) ny, (int) K) > kAvSmemMax) K--;
     if (K == 0) return 0;
     const int64_t blocks = (nz + K - 1) / K;
     if (blocks > sms || blocks >= kDsProgress) return 0;
@@ -569,7 +570,9 @@ int artss_turb_dynamic_smagorinsky(artss_ctx *ctx, double *ev, const double *u, 
     if (K > 0) {
         const int ny = (int) box.ny(), blocks = (int) ((box.nz() + K - 1) / K);
         const size_t smem = av_smem(ny, K);
-        ARTSS_CK(cudaFuncSetAttribute(k_ds_average_wave, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+        // one limit for every grid: the attribute is the function's, which contexts of other
+        // sizes launch from other threads
+        ARTSS_CK(cudaFuncSetAttribute(k_ds_average_wave, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kAvSmemMax));
         void *wargs[] = {&Cs, (void *) &flags, &Lc, &bc, &K, &progress};
         cudaError_t err;
         ARTSS_LAUNCH(ctx, FAM_SMAGORINSKY,
