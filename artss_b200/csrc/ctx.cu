@@ -251,13 +251,13 @@ int artss_ctx_create(const artss_grid_desc *grid, int device, artss_ctx **out) {
     if ((e = cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess)
         return fail(e, "multiprocessor count");
     if ((e = cudaMalloc(&ctx->d_partials, kMaxPartials * sizeof(double))) != cudaSuccess) return fail(e, "partials");
-    if ((e = cudaMalloc(&ctx->d_loop, 16 * sizeof(LoopState))) != cudaSuccess) return fail(e, "loop state");
+    if ((e = cudaMalloc(&ctx->d_loop, kLoopSlots * sizeof(LoopState))) != cudaSuccess) return fail(e, "loop state");
     if ((e = cudaMalloc(&ctx->d_param, kParams * sizeof(double))) != cudaSuccess) return fail(e, "parameters");
     if ((e = cudaMemset(ctx->d_param, 0, kParams * sizeof(double))) != cudaSuccess) return fail(e, "parameters");
     if ((e = cudaStreamCreateWithFlags(&ctx->body_stream, cudaStreamNonBlocking)) != cudaSuccess)
         return fail(e, "capture stream");
-    if ((e = cudaMemset(ctx->d_loop, 0, 16 * sizeof(LoopState))) != cudaSuccess) return fail(e, "loop state");
-    if ((e = cudaMallocHost(&ctx->h_loop, 16 * sizeof(LoopState))) != cudaSuccess) return fail(e, "pinned loop state");
+    if ((e = cudaMemset(ctx->d_loop, 0, kLoopSlots * sizeof(LoopState))) != cudaSuccess) return fail(e, "loop state");
+    if ((e = cudaMallocHost(&ctx->h_loop, kLoopSlots * sizeof(LoopState))) != cudaSuccess) return fail(e, "pinned loop state");
     for (int l = 0; l <= grid->n_levels; l++) {
         const int64_t n = ctx->lvl[l].size();
         if ((e = cudaMalloc(&ctx->d_flags[l], n)) != cudaSuccess) return fail(e, "cell flags");
@@ -334,7 +334,12 @@ void *artss_ctx_stream(artss_ctx *ctx) { return ctx ? (void *) ctx->stream : nul
 
 int artss_ctx_sync(artss_ctx *ctx) {
     if (!ctx) { set_error("null context"); return ARTSS_ERR_ARG; }
-    ARTSS_CK(cudaStreamSynchronize(ctx->stream));
+    return sync_and_report(ctx);
+}
+
+int artss_ctx_wait_limit(artss_ctx *ctx, int polls) {
+    if (!ctx) { set_error("null context"); return ARTSS_ERR_ARG; }
+    ctx->wait_polls = polls < 0 ? 1 << 20 : polls;
     return ARTSS_OK;
 }
 
@@ -379,8 +384,7 @@ int artss_upload(artss_ctx *ctx, double *dst, const double *host, int64_t n) {
 int artss_download(artss_ctx *ctx, double *host, const double *src, int64_t n) {
     if (!ctx || !src || !host || n < 0) { set_error("bad download arguments"); return ARTSS_ERR_ARG; }
     ARTSS_CK(cudaMemcpyAsync(host, src, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    ARTSS_CK(cudaStreamSynchronize(ctx->stream));
-    return ARTSS_OK;
+    return sync_and_report(ctx);
 }
 
 int artss_upload_async(artss_ctx *ctx, double *dst, const double *host, int64_t n) {

@@ -261,21 +261,20 @@ __device__ __forceinline__ double div27(double x) {
 // before; several calls in flight overlap, since a call uses 20 multiprocessors.
 // Loader warps fill the ring kAvG steps ahead.  Rows of the plane before the
 // block's first are read once the block that owns it has published that it has
-// updated them (the wait is bounded; a block that gives up raises the error flag
-// and ends, and k_ds_ev then writes NaN); every other row is read as the
+// updated them (the wait is bounded; a block that gives up raises two flags and
+// ends: k_ds_ev then writes NaN, and the context's next wait reports the error); every other row is read as the
 // reference reads it, before its update: its columns are loaded at least one
 // column before their own block, or the next one, gets to them.
 // Blocks wait on the block before them, so all are resident (cooperative launch).
 constexpr int kAvG = 8, kAvRing = 32, kAvPitch = 33;  // an odd pitch spreads the rows over the banks
 constexpr int kAvRows = 512, kAvLoaders = 128;        // rows (threads) of a block at most; loading threads
-constexpr int kAvPolls = 1 << 20;
 constexpr size_t kAvSmemMax = 225 * 1024;             // of a block at most
 
 inline size_t av_smem(int ny, int kn) { return (size_t) (kn + 2) * (ny + 2) * kAvPitch * sizeof(double); }
 
 __global__ void __launch_bounds__(kAvRows + kAvLoaders, 1)
 k_ds_average_wave(double *__restrict__ Cs, const uint8_t *__restrict__ flags, Level L, Box3 box, int K,
-                  int *__restrict__ progress) {
+                  int *__restrict__ progress, int polls, int *__restrict__ err) {
     extern __shared__ double ring[];
     const int nj = (int) L.Nx, nk = (int) L.nxy();
     const int x0 = (int) box.x0, x1 = (int) box.x1, y0 = (int) box.y0;
@@ -351,7 +350,7 @@ k_ds_average_wave(double *__restrict__ Cs, const uint8_t *__restrict__ flags, Le
             if (lt == 0) {
                 const int need = min(prev_steps, kAvG * (S + 1) + 4 * K - 1);
                 bool ok = false;
-                for (int n = 0; n < kAvPolls && !ok; n++) {
+                for (int n = 0; n < polls && !ok; n++) {
                     int v;
                     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(progress + prev) : "memory");
                     ok = v >= need;
@@ -381,7 +380,10 @@ k_ds_average_wave(double *__restrict__ Cs, const uint8_t *__restrict__ flags, Le
         }
         if (lt == 0) {
             __threadfence();
-            if (stop) atomicExch(progress + kDsProgress - 1, 1);
+            if (stop) {
+                atomicExch(progress + kDsProgress - 1, 1);
+                atomicExch(err, 1);
+            }
             else asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(progress + blockIdx.x), "r"(1 << 30) : "memory");
         }
         return;
@@ -573,7 +575,8 @@ int artss_turb_dynamic_smagorinsky(artss_ctx *ctx, double *ev, const double *u, 
         // one limit for every grid: the attribute is the function's, which contexts of other
         // sizes launch from other threads
         ARTSS_CK(cudaFuncSetAttribute(k_ds_average_wave, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kAvSmemMax));
-        void *wargs[] = {&Cs, (void *) &flags, &Lc, &bc, &K, &progress};
+        int polls = ctx->wait_polls, *err_flag = &ctx->d_loop[kDsErrSlot].pad;
+        void *wargs[] = {&Cs, (void *) &flags, &Lc, &bc, &K, &progress, &polls, &err_flag};
         cudaError_t err;
         ARTSS_LAUNCH(ctx, FAM_SMAGORINSKY,
                      err = cudaLaunchCooperativeKernel((const void *) k_ds_average_wave, dim3((unsigned) blocks),

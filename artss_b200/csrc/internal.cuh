@@ -30,6 +30,8 @@ constexpr uint8_t kBcLagged = 0x80;     // flat program: the root is itself a ta
 constexpr int kReduceThreads = 256;
 constexpr int kMaxPartials = 1 << 16;   // per-block partial sums of up to two reduction passes
 constexpr int kDiffuseSlot = 8;         // loop states of the diffusion solvers, a pair (8, 9)
+constexpr int kDsErrSlot = 14;          // loop slot whose error flag the dynamic Smagorinsky averaging raises
+constexpr int kLoopSlots = 16;
 constexpr int kNnErrSlot = 15;          // loop slot whose error flag the network kernels raise
 constexpr int kTmaBoxX = 72, kTmaBoxY = 12;  // TMA plane window (cells): a 64 x 8 tile, a 2-cell ring, x aligned to 2
 
@@ -199,6 +201,7 @@ struct artss_ctx {
     int sweep3_obst_state[3] = {0, 0, 0};                        // 0 not built, 1 built, 2 every box cell inner
     double *dsmag = nullptr;                                     // work arrays of artss_turb_dynamic_smagorinsky
     uint64_t dsmag_version = 0;                                  // geom_version they were zeroed for
+    int wait_polls = 1 << 20;                                    // of a block that waits for the one before it (dsmag.cu)
     float *cgsm_w = nullptr;                                     // FP32 defect / correction of artss_diffuse_cgs_mixed
     int64_t cgsm_n = 0;
     std::map<artss::TuneKey, int> tuned;                         // autotuned variant per kernel and shape
@@ -532,6 +535,9 @@ int tensor_map_3d(artss_ctx *ctx, const double *base, int level, const CUtensorM
 int finalize_loop(artss_ctx *ctx, int slot, int nblocks, double tol, long long max_it);
 int init_loop(artss_ctx *ctx, int slot, double residual0, long long it0, int cond0);
 int read_loop(artss_ctx *ctx, int slot, LoopState *out);
+// Waits for the stream and reports an error flag raised since the last report by
+// launches that no call of their own reads back (dynamic Smagorinsky).
+int sync_and_report(artss_ctx *ctx);
 
 // A loop inside a whole-step capture: a WHILE conditional node whose body is
 // everything enqueued on the context between begin and end (the context's

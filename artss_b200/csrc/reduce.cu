@@ -134,8 +134,22 @@ int GraphLoop::end(int slot, long long cap) {
 int read_loop(artss_ctx *ctx, int slot, LoopState *out) {
     ARTSS_CK(cudaMemcpyAsync(ctx->h_loop + slot, ctx->d_loop + slot, sizeof(LoopState), cudaMemcpyDeviceToHost,
                              ctx->stream));
-    ARTSS_CK(cudaStreamSynchronize(ctx->stream));
+    int st = sync_and_report(ctx);
+    if (st) return st;
     *out = ctx->h_loop[slot];
+    return ARTSS_OK;
+}
+
+int sync_and_report(artss_ctx *ctx) {
+    LoopState *h = ctx->h_loop + kDsErrSlot, *d = ctx->d_loop + kDsErrSlot;
+    if (ctx->dsmag) ARTSS_CK(cudaMemcpyAsync(h, d, sizeof(LoopState), cudaMemcpyDeviceToHost, ctx->stream));
+    ARTSS_CK(cudaStreamSynchronize(ctx->stream));
+    if (ctx->dsmag && h->pad) {
+        ARTSS_CK(cudaMemsetAsync(&d->pad, 0, sizeof(int), ctx->stream));
+        ARTSS_CK(cudaStreamSynchronize(ctx->stream));
+        set_error("dynamic Smagorinsky: a block of the averaging gave up waiting for the one before it");
+        return ARTSS_ERR_CUDA;
+    }
     return ARTSS_OK;
 }
 

@@ -135,6 +135,12 @@ int artss_ctx_destroy(artss_ctx *ctx);
 /* cudaStream_t of the context (all work of the context runs on it). */
 void *artss_ctx_stream(artss_ctx *ctx);
 int artss_ctx_sync(artss_ctx *ctx);
+/* Polls after which a block of artss_turb_dynamic_smagorinsky's averaging that waits
+ * for another one gives up (default, and for polls < 0: 2^20).  The result is then
+ * NaN, and the next call that waits for the stream (artss_ctx_sync, artss_download,
+ * a solve that reads its loop's state) returns ARTSS_ERR_CUDA.  No counterpart in the
+ * reference. */
+int artss_ctx_wait_limit(artss_ctx *ctx, int polls);
 const char *artss_last_error(void);
 /* Number of kernels this context has launched so far. */
 int64_t artss_ctx_kernel_launches(artss_ctx *ctx);

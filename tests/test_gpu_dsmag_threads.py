@@ -76,3 +76,22 @@ def test_small_call_between_capture_and_instantiation(pair):
     for m in pair:
         assert np.array_equal(m.result(), m.want)
     lib.artss_graph_destroy(graph)
+
+
+def test_a_wait_that_runs_out_is_reported(pair):
+    """two blocks of five planes; the second one's wait for the first runs out at once"""
+    large, small = pair
+    lib, h = large.ctx.lib, large.ctx.h
+    A.cuda_check(lib.artss_ctx_wait_limit(h, 0), "limit")
+    large.call()
+    small.call()
+    assert not large.bad and lib.artss_ctx_sync(h) == -2  # ARTSS_ERR_CUDA
+    assert "averaging" in lib.artss_last_error().decode()
+    assert np.isnan(large.result()).any()  # reported once
+    large.call()
+    with pytest.raises(RuntimeError):
+        large.result()
+    A.cuda_check(lib.artss_ctx_wait_limit(h, -1), "limit")
+    for m in pair:
+        m.call()
+        assert lib.artss_ctx_sync(m.ctx.h) == 0 and np.array_equal(m.result(), m.want)
