@@ -751,8 +751,7 @@ int artss_io_sync(artss_ctx *ctx) {
         ARTSS_CK(cudaStreamSynchronize(ctx->io_up));
         ARTSS_CK(cudaStreamSynchronize(ctx->io_down));
     }
-    ARTSS_CK(cudaStreamSynchronize(ctx->stream));
-    return ARTSS_OK;
+    return sync_and_report(ctx);
 }
 
 int artss_set_cell_lists(artss_ctx *ctx, int level, const int64_t *inner, int64_t n_inner,
