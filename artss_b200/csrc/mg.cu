@@ -34,7 +34,9 @@ struct artss_mg {
         int64_t launches, fam[artss::FAM_COUNT];
     };
     std::vector<Graph> graphs;
+    uint64_t graphs_version = ~0ull;  // ctx->geom_version whose programs they were captured with
     bool use_graphs = true;
+    uint64_t geom_version = ~0ull;    // ctx->geom_version that the two tables below describe (mg_tables)
     // the restriction of level l+1's inner cells reads no target of level l's
     // boundary program: the program on residuum0[l] has no reader
     bool r0_bc_dead[artss::kMaxLevel + 1]{};
@@ -2106,6 +2108,79 @@ int mg_prolongate_add(artss_mg *mg, double *fine, const double *coarse, int coar
     return ARTSS_OK;
 }
 
+// r0_bc_dead and closed of the present cell lists and boundary programs.  They decide
+// which launches and copies a V-cycle leaves out, so every entry point that runs one
+// comes by here first.  Where they changed, cells of the residual and prolongated arrays
+// that only the old ones wrote are zeroed, as in a new solver (the other arrays are
+// filled or copied before they are read).  Inside a capture the zeroing becomes part of
+// the graph and the next eager call does it once more.
+int mg_tables(artss_mg *mg) {
+    artss_ctx *ctx = mg->ctx;
+    if (mg->geom_version == ctx->geom_version) return ARTSS_OK;
+    int st;
+    if (mg->geom_version != ~0ull)
+        for (int l = 0; l < mg->L; l++) {
+            if ((st = artss_fill(ctx, mg->r0[l], l, 0.0))) return st;
+            if ((st = artss_fill(ctx, mg->e0[l], l, 0.0))) return st;
+        }
+    // residuum0[l] is read only by the restriction to level l+1, at the 8 fine
+    // cells of each coarse inner cell
+    for (int l = 0; l < mg->L; l++) {
+        const BcProgram &p = ctx->bc[l][ARTSS_FIELD_P];
+        const Level &F = ctx->lvl[l], &Cl = ctx->lvl[l + 1];
+        const CellBits &cin = ctx->inner_bits[l + 1];
+        mg->r0_bc_dead[l] = false;
+        if (!p.present || cin.n != Cl.size()) continue;
+        std::vector<bool> is_target((size_t) F.size(), false);
+        for (int64_t t : p.h_target) is_target[(size_t) t] = true;
+        bool read = false;
+        for (int64_t k = 0; k < Cl.Nz && !read; k++)
+            for (int64_t j = 0; j < Cl.Ny && !read; j++)
+                for (int64_t i = 0; i < Cl.Nx && !read; i++) {
+                    if (!cin.get(i + Cl.Nx * j + Cl.nxy() * k)) continue;
+                    for (int c = 0; c < 8 && !read; c++) {
+                        const int64_t fi = 2 * i - 1 + (c & 1), fj = 2 * j - 1 + (c >> 1 & 1), fk = 2 * k - 1 + (c >> 2);
+                        if (fi < 0 || fj < 0 || fk < 0 || fi >= F.Nx || fj >= F.Ny || fk >= F.Nz) read = true;
+                        else read = is_target[(size_t) (fi + F.Nx * fj + F.nxy() * fk)];
+                    }
+                }
+        mg->r0_bc_dead[l] = !read;
+    }
+    for (int l = 0; l < mg->L; l++) {
+        const BcProgram &p = ctx->bc[l][ARTSS_FIELD_P];
+        const Level &F = ctx->lvl[l];
+        const CellBits &in = ctx->inner_bits[l], &cin = ctx->inner_bits[l + 1];
+        const Level &Cl = ctx->lvl[l + 1];
+        mg->closed[l] = false;
+        if (!p.present || p.waves > 1 || in.n != F.size() || cin.n != Cl.size()) continue;
+        CellBits known = in;
+        bool ok = true;
+        for (int64_t t : p.h_target) known.set(t);
+        for (int64_t r : p.h_root) ok = ok && in.get(r);
+        // smoothing and residual read the 6 face neighbours, the prolongation from a
+        // coarse level all 26
+        for (int c = -1; c <= 1; c++)
+            for (int b = -1; b <= 1; b++)
+                for (int a = -1; a <= 1; a++)
+                    if (l > 0 || abs(a) + abs(b) + abs(c) == 1)
+                        ok = ok && in.neighbours_in(known, a + F.Nx * b + F.nxy() * c);
+        // ... and the prolongation to this level, cells 2 c - 1 and 2 c of an inner
+        // coarse cell c, writes known cells only
+        ok = ok && 2 * Cl.i2 < F.Nx && 2 * Cl.j2 < F.Ny && 2 * Cl.k2 < F.Nz;
+        for (int64_t i = 0; i < (int64_t) known.w.size() && ok; i++)
+            for (uint64_t rest = ~known.w[(size_t) i]; rest && ok; rest &= rest - 1) {
+                const int64_t q = 64 * i + __builtin_ctzll(rest);
+                if (q >= F.size()) break;
+                const int64_t z = q / F.nxy(), y = q / F.Nx % F.Ny, x = q % F.Nx;
+                const int64_t ci = (x + 1) / 2, cj = (y + 1) / 2, ck = (z + 1) / 2;
+                ok = ci >= Cl.Nx || cj >= Cl.Ny || ck >= Cl.Nz || !cin.get(ci + Cl.Nx * cj + Cl.nxy() * ck);
+            }
+        mg->closed[l] = ok;
+    }
+    if (!ctx->capturing) mg->geom_version = ctx->geom_version;
+    return ARTSS_OK;
+}
+
 // VCycleMG::VCycleMultigrid (VCycleMG.cpp:215-288).  The reference copies out
 // into error1[0], works on error1[0] and copies it back; nothing reads out in
 // between, so level 0's error1 is out itself here.  b0: the level-0 right-hand
@@ -2222,59 +2297,8 @@ int artss_mg_create(artss_ctx *ctx, const artss_mg_cfg *cfg, artss_mg **out) {
         st = st ? st : artss_field_alloc(ctx, l + 1, &mg->e1[l + 1]);
         st = st ? st : artss_field_alloc(ctx, l + 1, &mg->tmp[l + 1]);
     }
+    if (!st) st = mg_tables(mg);
     if (st) { artss_mg_destroy(mg); return st; }
-    // residuum0[l] is read only by the restriction to level l+1, at the 8 fine
-    // cells of each coarse inner cell
-    for (int l = 0; l < mg->L; l++) {
-        const BcProgram &p = ctx->bc[l][ARTSS_FIELD_P];
-        const Level &F = ctx->lvl[l], &Cl = ctx->lvl[l + 1];
-        const std::vector<bool> &cin = ctx->h_inner[l + 1];
-        if (!p.present || (int64_t) cin.size() != Cl.size()) continue;
-        std::vector<bool> is_target((size_t) F.size(), false);
-        for (int64_t t : p.h_target) is_target[(size_t) t] = true;
-        bool read = false;
-        for (int64_t k = 0; k < Cl.Nz && !read; k++)
-            for (int64_t j = 0; j < Cl.Ny && !read; j++)
-                for (int64_t i = 0; i < Cl.Nx && !read; i++) {
-                    if (!cin[(size_t) (i + Cl.Nx * j + Cl.nxy() * k)]) continue;
-                    for (int c = 0; c < 8 && !read; c++) {
-                        const int64_t fi = 2 * i - 1 + (c & 1), fj = 2 * j - 1 + (c >> 1 & 1), fk = 2 * k - 1 + (c >> 2);
-                        if (fi < 0 || fj < 0 || fk < 0 || fi >= F.Nx || fj >= F.Ny || fk >= F.Nz) read = true;
-                        else read = is_target[(size_t) (fi + F.Nx * fj + F.nxy() * fk)];
-                    }
-                }
-        mg->r0_bc_dead[l] = !read;
-    }
-    for (int l = 0; l < mg->L; l++) {
-        const BcProgram &p = ctx->bc[l][ARTSS_FIELD_P];
-        const Level &F = ctx->lvl[l];
-        const CellBits &in = ctx->inner_bits[l], &cin = ctx->inner_bits[l + 1];
-        const Level &Cl = ctx->lvl[l + 1];
-        if (!p.present || p.waves > 1 || in.n != F.size() || cin.n != Cl.size()) continue;
-        CellBits known = in;
-        bool ok = true;
-        for (int64_t t : p.h_target) known.set(t);
-        for (int64_t r : p.h_root) ok = ok && in.get(r);
-        // smoothing and residual read the 6 face neighbours, the prolongation from a
-        // coarse level all 26
-        for (int c = -1; c <= 1; c++)
-            for (int b = -1; b <= 1; b++)
-                for (int a = -1; a <= 1; a++)
-                    if (l > 0 || abs(a) + abs(b) + abs(c) == 1)
-                        ok = ok && in.neighbours_in(known, a + F.Nx * b + F.nxy() * c);
-        // ... and the prolongation to this level, cells 2 c - 1 and 2 c of an inner
-        // coarse cell c, writes known cells only
-        ok = ok && 2 * Cl.i2 < F.Nx && 2 * Cl.j2 < F.Ny && 2 * Cl.k2 < F.Nz;
-        for (int64_t i = 0; i < (int64_t) known.w.size() && ok; i++)
-            for (uint64_t rest = ~known.w[(size_t) i]; rest && ok; rest &= rest - 1) {
-                const int64_t q = 64 * i + __builtin_ctzll(rest);
-                if (q >= F.size()) break;
-                const int64_t z = q / F.nxy(), y = q / F.Nx % F.Ny, x = q % F.Nx;
-                const int64_t ci = (x + 1) / 2, cj = (y + 1) / 2, ck = (z + 1) / 2;
-                ok = ci >= Cl.Nx || cj >= Cl.Ny || ck >= Cl.Nz || !cin.get(ci + Cl.Nx * cj + Cl.nxy() * ck);
-            }
-        mg->closed[l] = ok;
-    }
     *out = mg;
     return ARTSS_OK;
 }
@@ -2301,7 +2325,8 @@ int artss_mg_set_rhs(artss_mg *mg, const double *p, const double *rhs) {
 
 int artss_mg_vcycle(artss_mg *mg, double *p) {
     if (!mg || !p) { set_error("null argument"); return ARTSS_ERR_ARG; }
-    return mg_vcycle(mg, p, nullptr);
+    int st = mg_tables(mg);
+    return st ? st : mg_vcycle(mg, p, nullptr);
 }
 
 // kernel families a V-cycle launches: event profiling of any of them needs eager launches
@@ -2353,7 +2378,8 @@ int artss_mg_pressure(artss_mg *mg, double *p, const double *rhs, int first_step
         return ARTSS_ERR_ARG;
     }
     if (!mg || !p || !rhs) { set_error("null argument"); return ARTSS_ERR_ARG; }
-    int st;
+    int st = mg_tables(mg);
+    if (st) return st;
     int64_t cycles = 0, coarse = 0;
     double residual = -1.0;
     if (first_step) {
@@ -2381,6 +2407,11 @@ int artss_mg_pressure(artss_mg *mg, double *p, const double *rhs, int first_step
         // the later-step call is a fixed launch sequence: replay it as one graph
         artss_ctx *ctx = mg->ctx;
         artss_mg::Graph *g = nullptr;
+        if (mg->graphs_version != ctx->geom_version) {  // captured with other programs, whose tables are gone
+            for (auto &e : mg->graphs) cudaGraphExecDestroy(e.exec);
+            mg->graphs.clear();
+            mg->graphs_version = ctx->geom_version;
+        }
         for (auto &e : mg->graphs)
             if (e.p == p && e.rhs == rhs) g = &e;
         if (!g) {
@@ -2441,7 +2472,8 @@ int artss_mg_solve_rel(artss_mg *mg, double *p, const double *rhs, double rel_to
                        artss_solve_stats *stats) {
     if (!mg || !p || !rhs) { set_error("null argument"); return ARTSS_ERR_ARG; }
     if (max_cycles < 0 || !(rel_tol >= 0)) { set_error("invalid tolerance or cycle limit"); return ARTSS_ERR_ARG; }
-    int st;
+    int st = mg_tables(mg);
+    if (st) return st;
     if ((st = artss_mg_set_rhs(mg, p, rhs))) return st;
     double res = 0, b_norm = 0;
     if ((st = artss_residual_norm(mg->ctx, p, rhs, &res, &b_norm))) return st;
