@@ -501,7 +501,7 @@ int artss_set_boundary_program(artss_ctx *ctx, int level, int field_type, const 
 int artss_boundary_program_waves(artss_ctx *ctx, int level, int field_type) {
     if (check_level(ctx, level) || check_field_type(field_type)) return -1;
     const BcProgram &p = ctx->bc[level][field_type];
-    return !p.present ? 0 : p.flat.n ? 1 : p.waves;
+    return p.present ? p.waves : 0;
 }
 
 int artss_apply_boundary(artss_ctx *ctx, double *field, int level, int field_type) {

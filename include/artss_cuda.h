@@ -274,7 +274,8 @@ int artss_get_cell_flags(artss_ctx *ctx, int level, uint8_t *host_out, int64_t n
  * several waves into a flat form that runs as one launch. */
 int artss_set_boundary_program(artss_ctx *ctx, int level, int field_type,
                                const artss_bc_assign *ops, int64_t n_ops);
-/* Number of dependency-free waves in the compiled program of (level, field_type). */
+/* Number of dependency-free waves in the compiled program of (level, field_type); one of
+ * several waves takes a launch for each only where it has no flat form. */
 int artss_boundary_program_waves(artss_ctx *ctx, int level, int field_type);
 
 /* DomainController::apply_boundary (src/domain/DomainController.cpp:145-147). */

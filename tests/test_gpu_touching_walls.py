@@ -26,6 +26,8 @@ def room(request, tmp_path_factory):
 
 def test_programs(room):
     geom, ctx, osc = room
+    waves = [ctx.lib.artss_boundary_program_waves(ctx.h, 0, ft) for ft in range(1, 7)]
+    assert max(waves) > 1  # the walls touch
     for level in range(geom.levels + 1):
         for ft in range(1, 7):
             if geom.boundary_program(level, ft).size == 0:
@@ -35,7 +37,9 @@ def test_programs(room):
             x[::11] = -0.0
             d = ctx.field(x, level)
             for _ in range(2):
+                launches = ctx.lib.artss_ctx_kernel_launches(ctx.h)
                 A.cuda_check(ctx.lib.artss_apply_boundary(ctx.h, d, level, ft), "bc")
+                assert ctx.lib.artss_ctx_kernel_launches(ctx.h) == launches + 1  # the flat form
                 oracle.lib().oracle_apply_bc(osc.ptr, P(x), level, ft)
                 got = ctx.download(d, level)
                 assert np.array_equal(got, x) and np.array_equal(np.signbit(got), np.signbit(x)), (level, ft)
