@@ -1759,6 +1759,12 @@ int coarse_block_slots(const artss_ctx *ctx, int level, int64_t *smem) {
     const Level &L = ctx->lvl[level];
     const BcProgram &p = ctx->bc[level][ARTSS_FIELD_P];
     if (p.present && p.waves > 1 && !p.flat.n) return 0;
+    // a target that is swept needs its assignment after every sweep, also from a constant
+    // root, and a root that is one has its swept value before the program
+    const CellBits &in = ctx->inner_bits[level];
+    if (in.n != L.size()) return 0;
+    for (int64_t t : p.h_target)
+        if (in.get(t)) return 0;
     const BcView v = pipe_view(ctx, level);
     const Box3 box = inner_box(L);
     const int64_t cells = box.nx() * box.ny() * box.nz();

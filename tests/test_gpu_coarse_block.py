@@ -2,6 +2,8 @@
 one-block forms: the same pressures bit for bit, stopped after one to all sweeps and by
 the tolerance, for programs of one wave, flat ones, valued ones and levels of one and of
 two cells per thread."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -44,5 +46,39 @@ def test_forms(name, tmp_path):
             for flags in (2, 4):
                 for a, b in zip(pressures(ctx, p0, rhs, sweeps, tol, flags), got):
                     assert np.array_equal(a, b), (sweeps, tol, flags)
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("chain", [False, True])
+def test_assigned_inner_cells(tmp_path, chain):
+    """A program that also assigns inner cells of the coarse solve's level, from a cell that
+    nothing writes and (chain: a flat program) from one another: the other forms' bits."""
+    geom = A.Geometry(scenes.write(SCENES["cube8"](), str(tmp_path / "s.xml")))
+    ctx = cabi.Context(geom)
+    try:
+        prog = geom.boundary_program(1, 4)
+        prog = np.ascontiguousarray(prog[(prog["target"] != 0) & (prog["source"] != 0)])  # nothing writes the array's first cell
+        nx, nxy = ctx.grid.Nx[1], ctx.grid.Nx[1] * ctx.grid.Ny[1]
+        at = lambda i, j, k: i + nx * j + nxy * k  # noqa: E731
+        # (target, source): inner from a constant cell, inner from inner
+        more = [(at(4, 4, 4), at(0, 0, 0)), (at(5, 2, 6), at(3, 3, 3))]
+        if chain:  # a cell that is read before it is written: several waves
+            more = [(at(6, 6, 6), at(4, 4, 4))] + more
+        arr = (A.BcAssign * (prog.size + len(more)))()
+        C.memmove(arr, prog.ctypes.data, prog.nbytes)
+        for n, (t, s) in enumerate(more):
+            arr[prog.size + n] = A.BcAssign(target=t, source=s, sign=1, value=0.25)
+        A.cuda_check(ctx.lib.artss_set_boundary_program(ctx.h, 1, 4, arr, prog.size + len(more)), "bc")
+        assert (ctx.lib.artss_boundary_program_waves(ctx.h, 1, 4) > 1) == chain
+        inner = geom.list("inner", 0)
+        for sweeps in (1, 2, 3, 20):
+            rng = np.random.default_rng(sweeps)
+            p0, rhs = rng.uniform(-1, 1, ctx.size()), np.zeros(ctx.size())
+            rhs[inner] = rng.uniform(-1, 1, inner.size)
+            got = pressures(ctx, p0, rhs, sweeps, 1e-300, 0)
+            for flags in (2, 4):
+                for a, b in zip(pressures(ctx, p0, rhs, sweeps, 1e-300, flags), got):
+                    assert np.array_equal(a, b), (sweeps, flags)
     finally:
         ctx.close()
