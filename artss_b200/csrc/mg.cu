@@ -2146,7 +2146,9 @@ int mg_tables(artss_mg *mg) {
                     if (!cin.get(i + Cl.Nx * j + Cl.nxy() * k)) continue;
                     for (int c = 0; c < 8 && !read; c++) {
                         const int64_t fi = 2 * i - 1 + (c & 1), fj = 2 * j - 1 + (c >> 1 & 1), fk = 2 * k - 1 + (c >> 2);
-                        if (fi < 0 || fj < 0 || fk < 0 || fi >= F.Nx || fj >= F.Ny || fk >= F.Nz) read = true;
+                        // the fused pass reads a child's neighbours: children on the array's
+                        // faces, which grids of odd inner sizes have, take the general way
+                        if (fi < 1 || fj < 1 || fk < 1 || fi > F.Nx - 2 || fj > F.Ny - 2 || fk > F.Nz - 2) read = true;
                         else read = is_target[(size_t) (fi + F.Nx * fj + F.nxy() * fk)];
                     }
                 }
