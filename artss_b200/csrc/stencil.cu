@@ -1827,9 +1827,12 @@ int set_sweep_smem(bool turb) {
 // variant (kernel and z-depth) on that solve's first iteration (the sweep
 // reads `rd`, b, EV and writes only `w` and the partials, so repeating it
 // changes nothing) and keeps the fastest for the context.
-// A call that may not tune takes the block kernel on levels whose marching kernels
-// would not fill the chip (they are level at 96^3 cells), else the row-pair one.
-constexpr int64_t kSweepBlockCells = 1000 * 1000;
+// Levels whose marching kernels would not fill the chip take the block kernel without
+// a trial: it is the fastest on all of 32^3 to 88^3 (681 k cells: 20.8 against 22.2 us,
+// turbulent), 128 x 64 x 64, 160 x 64 x 64 and 96 x 48 x 96, and from 786 k cells (64 x 128
+// x 96) on others are.  With its trials the first solve of a level took 1.9 ms, a later
+// one 0.2.  A call on a larger level that may not tune takes the row-pair kernel.
+constexpr int64_t kSweepBlockCells = 700 * 1000;
 int tune_sweep(artss_ctx *ctx, bool turb, bool tma, bool one_phase, const Box3 &box, const SweepMaps &m, double *w,
                const Level &L, const DiffCoef &c, LoopState *pred, int *choice) {
     if (!tma) {  // the marching kernels need TMA
@@ -1850,8 +1853,13 @@ int tune_sweep(artss_ctx *ctx, bool turb, bool tma, bool one_phase, const Box3 &
         *choice = it->second;
         return ARTSS_OK;
     }
-    const int fallback = box.nx() * box.ny() * box.nz() < kSweepBlockCells ? kSweepBlock : one_phase ? kSweepRowPair : 1;
+    const bool small = box.nx() * box.ny() * box.nz() < kSweepBlockCells;
+    const int fallback = small ? kSweepBlock : one_phase ? kSweepRowPair : 1;
     if (!ctx->autotune || ctx->capturing) { *choice = fallback; return ARTSS_OK; }
+    if (small) {
+        *choice = ctx->tuned[key] = kSweepBlock;
+        return ARTSS_OK;
+    }
     cudaEvent_t e0, e1;
     ARTSS_CK(cudaEventCreate(&e0));
     ARTSS_CK(cudaEventCreate(&e1));
@@ -1861,7 +1869,7 @@ int tune_sweep(artss_ctx *ctx, bool turb, bool tma, bool one_phase, const Box3 &
         if (v >= 3 && v != kSweepBlock && !one_phase) continue;
         if ((st = launch_sweep(ctx, turb, v, box, m, w, L, c, pred, &nb))) break;  // warm
         cudaEventRecord(e0, ctx->stream);
-        for (int r = 0; r < 3 && !st; r++) st = launch_sweep(ctx, turb, v, box, m, w, L, c, pred, &nb);
+        for (int r = 0; r < 2 && !st; r++) st = launch_sweep(ctx, turb, v, box, m, w, L, c, pred, &nb);
         cudaEventRecord(e1, ctx->stream);
         if (cudaEventSynchronize(e1) != cudaSuccess) { st = cuda_fail(cudaGetLastError(), "autotune"); break; }
         float ms = 0;
