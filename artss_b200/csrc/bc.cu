@@ -370,6 +370,26 @@ void free_flat(BcProgram::Flat &x) {
     x = BcProgram::Flat{};
 }
 
+// JacobiDiffuse copies in = out over the domain list after every iteration
+// (JacobiDiffuse.cpp:85-89).  The two arrays may take turns instead where that copy
+// gives the next iteration exactly what the array just written holds: every face
+// neighbour of an inner cell is on the domain list (obstacles that leave cells off
+// it keep their old values in `in`), the cells on it are the inner ones and the
+// program's targets, and the program reads nothing that it writes (one wave).
+// Decided when lists and programs are set: at 128^3 the check took 0.8 ms of a first solve.
+void update_alternates(artss_ctx *ctx, int field_type) {
+    const BcProgram &p = ctx->bc[0][field_type];
+    const CellBits &in = ctx->inner_bits[0], &dom = ctx->domain_bits;
+    bool ok = ctx->faces_in_domain && (!p.present || p.waves <= 1);
+    if (ok) {
+        CellBits set = in;
+        for (int64_t t : p.h_target) set.set(t);
+        for (int64_t r : p.h_root) ok = ok && dom.get(r);
+        ok = ok && set.w == dom.w;
+    }
+    ctx->alternates[field_type] = ok;
+}
+
 // the flat form of a program of several waves, on the device
 int build_flat(artss_ctx *ctx, BcProgram &p, const artss_bc_assign *ops, int64_t n_ops) {
     std::vector<Folded> f;
@@ -467,6 +487,7 @@ int artss_set_boundary_program(artss_ctx *ctx, int level, int field_type, const 
     p.h_root = root;
     p.h_sign = sign;
     ctx->geom_version++;
+    if (level == 0) update_alternates(ctx, field_type);
     p.zero_values = true;
     for (double v : val) {
         uint64_t bits;

@@ -796,6 +796,11 @@ int artss_set_cell_lists(artss_ctx *ctx, int level, const int64_t *inner, int64_
     if (level == 0) {
         ctx->domain_bits.reset(L.size());
         for (int64_t q = 0; q < n_domain; q++) ctx->domain_bits.set(domain[q]);
+        bool ok = true;
+        for (int64_t d : {(int64_t) -1, (int64_t) 1, -L.Nx, L.Nx, -L.nxy(), L.nxy()})
+            ok = ok && ctx->inner_bits[0].neighbours_in(ctx->domain_bits, d);
+        ctx->faces_in_domain = ok;
+        for (int ft = 0; ft < kFieldTypes; ft++) update_alternates(ctx, ft);
     }
     for (auto &prog : ctx->bc[level]) prog.pipe_state = -2;
     int64_t *d_list = nullptr;

@@ -177,10 +177,8 @@ struct artss_ctx {
     uint8_t *d_flags[artss::kMaxLevel + 1]{};
     std::vector<bool> h_inner[artss::kMaxLevel + 1];  // inner-cell bitmap per level, host copy
     artss::CellBits inner_bits[artss::kMaxLevel + 1], domain_bits;  // inner cells; domain list of level 0
-    // per field type: the Jacobi diffusion may alternate between its two arrays
-    // (jacobi_alternates), decided for geometry alternates_version
-    int8_t alternates[artss::kFieldTypes] = {};
-    uint64_t alternates_version[artss::kFieldTypes] = {};
+    bool faces_in_domain = false;                                   // every face neighbour of an inner cell is on the domain list
+    bool alternates[artss::kFieldTypes] = {};                       // the Jacobi diffusion's arrays may take turns (update_alternates)
     int64_t n_inner[artss::kMaxLevel + 1]{};  // inner cells per level (artss_set_cell_lists)
     double *proj[artss::kMaxLevel + 1]{};     // scratch of artss_coarse_project (lazily, freed with fields)
     artss::BcProgram bc[artss::kMaxLevel + 1][artss::kFieldTypes];
@@ -503,6 +501,8 @@ inline int check_reduce_blocks(const dim3 &g) {
 // Boundary program execution (bc.cu).
 // pred != NULL: every launch returns at once when pred->cond == 0 (predicated loop body)
 int apply_bc(artss_ctx *ctx, double *f, int level, int field_type, const LoopState *pred = nullptr);
+// ctx->alternates of a field type, after a change of level 0's cell lists or of its program
+void update_alternates(artss_ctx *ctx, int field_type);
 
 // The end of a predicated loop iteration: the boundary program on f and the loop
 // step (the sum of the sweep's `nblocks` partials, the residual, the decision) in one

@@ -2111,36 +2111,6 @@ int artss_diffuse_cgs_mixed(artss_ctx *ctx, double *out, double *in, const doubl
     return ARTSS_OK;
 }
 
-}  // extern "C"
-
-namespace {
-// JacobiDiffuse copies in = out over the domain list after every iteration
-// (JacobiDiffuse.cpp:85-89).  The two arrays may take turns instead where that copy
-// gives the next iteration exactly what the array just written holds: every face
-// neighbour of an inner cell is on the domain list (obstacles that leave cells off
-// it keep their old values in `in`), the cells on it are the inner ones and the
-// program's targets, and the program reads nothing that it writes (one wave).
-bool jacobi_alternates(artss_ctx *ctx, int ft) {
-    if (ctx->alternates[ft] && ctx->alternates_version[ft] == ctx->geom_version) return ctx->alternates[ft] > 0;
-    const Level &L = ctx->lvl[0];
-    const CellBits &in = ctx->inner_bits[0], &dom = ctx->domain_bits;
-    const BcProgram &p = ctx->bc[0][ft];
-    bool ok = in.n == L.size() && dom.n == L.size() && (!p.present || p.waves <= 1);
-    if (ok) {
-        CellBits set = in;
-        for (int64_t t : p.h_target) set.set(t);
-        for (int64_t r : p.h_root) ok = ok && dom.get(r);
-        ok = ok && set.w == dom.w;
-        for (int64_t d : {(int64_t) -1, (int64_t) 1, -L.Nx, L.Nx, -L.nxy(), L.nxy()}) ok = ok && in.neighbours_in(dom, d);
-    }
-    ctx->alternates[ft] = ok ? 1 : -1;
-    ctx->alternates_version[ft] = ctx->geom_version;
-    return ok;
-}
-}  // namespace
-
-extern "C" {
-
 int artss_diffuse_jacobi(artss_ctx *ctx, double *out, double *in, const double *b, double D, const double *ev,
                          double dt, int field_type, const artss_iter_cfg *cfg, artss_iter_stats *stats) {
     int st = check_field_args(ctx, {out, in, b, cfg});
@@ -2163,7 +2133,7 @@ int artss_diffuse_jacobi(artss_ctx *ctx, double *out, double *in, const double *
     LoopState ls{};
     int64_t batch = std::max<int64_t>(1, std::min<int64_t>(loop_hint(ctx, 1, field_type), cfg->max_iter));
     // the arrays take turns (iteration n odd: in -> out), or `in` follows `out` by a copy
-    const bool turns = out != in && b != in && b != out && ev != in && ev != out && jacobi_alternates(ctx, field_type);
+    const bool turns = out != in && b != in && b != out && ev != in && ev != out && ctx->alternates[field_type];
     auto iteration = [&](long long n) -> int {
         double *w = turns && !(n & 1) ? in : out;
         const double *rd = turns && !(n & 1) ? out : in;
