@@ -789,8 +789,6 @@ int artss_set_cell_lists(artss_ctx *ctx, int level, const int64_t *inner, int64_
         return true;
     };
     if (!check(inner, n_inner, 0, "inner") || !check(domain, n_domain, 1, "domain")) return ARTSS_ERR_ARG;
-    ctx->h_inner[level].assign((size_t) L.size(), false);
-    for (int64_t q = 0; q < n_inner; q++) ctx->h_inner[level][(size_t) inner[q]] = true;
     ctx->inner_bits[level].reset(L.size());
     for (int64_t q = 0; q < n_inner; q++) ctx->inner_bits[level].set(inner[q]);
     if (level == 0) {

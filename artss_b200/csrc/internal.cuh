@@ -175,7 +175,6 @@ struct artss_ctx {
     artss_grid_desc grid{};
     artss::Level lvl[artss::kMaxLevel + 1]{};
     uint8_t *d_flags[artss::kMaxLevel + 1]{};
-    std::vector<bool> h_inner[artss::kMaxLevel + 1];  // inner-cell bitmap per level, host copy
     artss::CellBits inner_bits[artss::kMaxLevel + 1], domain_bits;  // inner cells; domain list of level 0
     bool faces_in_domain = false;                                   // every face neighbour of an inner cell is on the domain list
     bool alternates[artss::kFieldTypes] = {};                       // the Jacobi diffusion's arrays may take turns (update_alternates)

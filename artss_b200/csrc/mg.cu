@@ -1571,9 +1571,9 @@ bool coarse_pipe_plan(artss_ctx *ctx, int level, PipeLaunch *pl) {
 bool coarse_pipe_plan_new(artss_ctx *ctx, int level, PipeLaunch *pl) {
     BcProgram &p = ctx->bc[level][ARTSS_FIELD_P];
     const Level &L = ctx->lvl[level];
-    const std::vector<bool> &in = ctx->h_inner[level];
+    const CellBits &in = ctx->inner_bits[level];
     const int nz = (int) L.Nz;
-    if (cluster_ranks(L) < 2 || L.nxy() % 2 || in.empty() || (int64_t) in.size() != L.size()) return false;
+    if (cluster_ranks(L) < 2 || L.nxy() % 2 || in.n != L.size()) return false;
     const bool flat = p.flat.n > 0;
     if (p.present && p.waves > 1 && !flat) return false;
     const std::vector<int64_t> &ht = flat ? p.flat.h_target : p.h_target, &hr = flat ? p.flat.h_root : p.h_root;
@@ -1585,7 +1585,7 @@ bool coarse_pipe_plan_new(artss_ctx *ctx, int level, PipeLaunch *pl) {
     for (int64_t q = 0; q < n; q++) {
         const int64_t t = ht[q], r = hr[q];
         const int kt = (int) (t / L.nxy()), kr = (int) (r / L.nxy());
-        if (in[(size_t) t]) return false;
+        if (in.get(t)) return false;
         // a chain that spans more than neighbouring planes stays within one rank
         if (kr < kt - 1 || kr > kt + 1)
             for (int c = std::min(kr, kt) + 1; c <= std::max(kr, kt); c++) forbidden[c] = 1;
@@ -1627,7 +1627,7 @@ bool coarse_pipe_plan_new(artss_ctx *ctx, int level, PipeLaunch *pl) {
             int nt = 0, nf = 0;
             for (int64_t q = 0; q < n; q++) {
                 const bool lagged = flat && (p.flat.h_depth[(size_t) q] & kBcLagged);
-                if (!in[(size_t) hr[q]] && !lagged) continue;
+                if (!in.get(hr[q]) && !lagged) continue;
                 const int kt = (int) (ht[q] / L.nxy()), kr = (int) (hr[q] / L.nxy());
                 const bool own_t = kt >= a && kt < e, own_r = kr >= a && kr < e;
                 if (lagged) {

@@ -1685,17 +1685,17 @@ struct SweepMaps {
 int sweep3_obst(artss_ctx *ctx, const Box3 &box, int t, int ty_rows, int ncx, int ncy, const uint8_t **out) {
     if (ctx->sweep3_obst_state[t] == 0) {
         const Level &L = ctx->lvl[0];
-        const std::vector<bool> &in = ctx->h_inner[0];
-        if (!in.empty() && ctx->n_inner[0] == box.nx() * box.ny() * box.nz()) {
+        const CellBits &in = ctx->inner_bits[0];
+        if (in.n && ctx->n_inner[0] == box.nx() * box.ny() * box.nz()) {
             ctx->sweep3_obst_state[t] = 2;
         } else {
             // no lists uploaded: every cell goes through its flag
-            std::vector<uint8_t> tab((size_t) ncx * ncy * L.Nz, in.empty() ? 1 : 0);
-            if (!in.empty()) {
+            std::vector<uint8_t> tab((size_t) ncx * ncy * L.Nz, in.n ? 0 : 1);
+            if (in.n) {
                 for (int64_t k = box.z0; k <= box.z1; k++)
                     for (int64_t y = box.y0; y <= box.y1; y++)
                         for (int64_t x = box.x0; x <= box.x1; x++) {
-                            if (in[(size_t) (x + L.Nx * y + L.nxy() * k)]) continue;
+                            if (in.get(x + L.Nx * y + L.nxy() * k)) continue;
                             const int64_t cx = (x - box.x0) / 64, cy = (y - box.y0) / ty_rows;
                             for (int64_t ty = std::max<int64_t>(0, cy - 1); ty <= std::min<int64_t>(ncy - 1, cy + 1); ty++)
                                 for (int64_t tx = std::max<int64_t>(0, cx - 1); tx <= std::min<int64_t>(ncx - 1, cx + 1);
