@@ -46,7 +46,7 @@ CASES = {
 }
 
 
-@pytest.mark.parametrize("relax", [1, 3])
+@pytest.mark.parametrize("relax", [1, 2, 3])
 @pytest.mark.parametrize("case", list(CASES))
 def test_forms_agree(case, relax, tmp_path):
     sc = CASES[case]()

@@ -1,6 +1,6 @@
 """The colored Gauss-Seidel sweep on blocks of 32 x 8 x 4 cells: edges of blocks,
-one cell past them, grids smaller than one, both parities of the pitch, obstacles,
-bit for bit against the oracle."""
+one cell past them, grids smaller than one, both parities of the pitch, obstacles, more
+tiles (8400) than a launch has blocks (8192), bit for bit against the oracle."""
 import ctypes as C
 
 import numpy as np
@@ -15,7 +15,7 @@ P = oracle.p
 
 
 @pytest.mark.parametrize("turbulent", [False, True])
-@pytest.mark.parametrize("dims", [(32, 8, 4), (33, 9, 5), (64, 16, 8), (3, 3, 3), (31, 7, 13), (95, 41, 22)])
+@pytest.mark.parametrize("dims", [(32, 8, 4), (33, 9, 5), (64, 16, 8), (3, 3, 3), (31, 7, 13), (95, 41, 22), (33, 9, 8400)])
 def test_blocks(tmp_path, dims, turbulent):
     nx, ny, nz = dims
     sc = scenes.Scene(nx=nx, ny=ny, nz=nz, X=(0.0, 0.1 * nx), Y=(0.0, 0.1 * ny), Z=(0.0, 0.1 * nz), steps=1, n_level=0,
