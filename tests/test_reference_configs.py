@@ -32,8 +32,8 @@ def _names(g):
 
 
 def test_reference_tree_holds_configs():
-    if not os.path.isdir(REFERENCE):
-        pytest.skip("reference source tree not present")
+    if not os.path.isdir(os.path.join(REFERENCE, "src")):
+        pytest.skip("reference source tree not present")  # the directory may be there, empty
     assert len(_configs()) >= 20
 
 
